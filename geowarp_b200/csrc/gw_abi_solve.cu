@@ -8,6 +8,7 @@
 #include "gw_host.cuh"
 #include "gw_mg.cuh"
 #include "gw_mg_tail.cuh"
+#include "gw_sell.cuh"
 
 using namespace gw;
 using namespace gwh;
@@ -293,6 +294,9 @@ struct MgLevel {
     int *parent;            // levels with a coarser one: coarse rows of the 2^D parents of each row
     void *pvals;            // level 0: BF16 copy of the fine Jacobian read by the V-cycle (mixed)
     uint8_t *flags;
+    // 2D: the sliced layout (gw_sell.cuh) of this level's matrix
+    int *scols, *strips;
+    void *svals;
 };
 struct MgHier {
     int nl = 0;             // levels holding a matrix; the last one is solved with a dense inverse
@@ -328,6 +332,12 @@ struct FlexVecs {
     double *V, *Z, *w, *partials;
     GScalars *sc;
 };
+void mg_carve_sell(Bump &bp, MgLevel &v, int64_t n_rows, int nf) {
+    const int64_t e = sell_elems(n_rows);
+    v.scols = (int *)bp.take(4 * e);
+    v.strips = (int *)bp.take(4 * (n_rows / 8 + 1));  // chunks of at least 8 rows
+    v.svals = bp.take(8 * e * nf * nf);
+}
 void mg_carve_hier(Bump &bp, MgHier &h, const gw_grid_t &g0, int64_t n_rows0, int nf) {
     const int64_t n0 = n_rows0 * nf;
     const int D = g0.dim, mw = D == 2 ? 1 : 4, S = D == 2 ? 25 : 125;
@@ -341,7 +351,8 @@ void mg_carve_hier(Bump &bp, MgHier &h, const gw_grid_t &g0, int64_t n_rows0, in
     l0.fixed = (uint8_t *)bp.take(n_rows0);
     const int CN = D == 2 ? 9 : 27, PN = D == 2 ? 4 : 8;
     l0.parent = (int *)bp.take(4 * n_rows0 * PN);
-    l0.pvals = bp.take(2 * n_rows0 * S * nf * nf);
+    l0.pvals = bp.take(2 * (D == 2 ? sell_elems(n_rows0) : n_rows0 * S) * nf * nf);
+    if (D == 2) mg_carve_sell(bp, l0, n_rows0, nf);
     gw_grid_t g = g0;
     int64_t nodes = g0.n_nodes;
     int l = 0;
@@ -369,6 +380,7 @@ void mg_carve_hier(Bump &bp, MgHier &h, const gw_grid_t &g0, int64_t n_rows0, in
         c.fixed = (uint8_t *)bp.take(nodes);
         c.child = (int *)bp.take(4 * nodes * CN);
         c.parent = (int *)bp.take(4 * nodes * PN);
+        if (D == 2) mg_carve_sell(bp, c, nodes, nf);
     }
     h.nl = l + 1;  // upper bound; the plan may stop earlier
     h.dM = (double *)bp.take(8 * (int64_t)kMgCoarseMax * kMgCoarseMax);
@@ -462,6 +474,14 @@ int mg_pattern(MgHier &h, const gw_bsr_t *A0, gw_mg_plan_t *plan, cudaStream_t s
     }
     h.nl = l + 1;
     h.dn = h.lv[l].A.n_rows * NF;
+    if (D == 2)
+        for (int q = 0; q < (h.nl > 1 ? h.nl - 1 : 1); ++q) {
+            MgLevel &v = h.lv[q];
+            const int lpr = sell_lpr(v.A.n_rows);
+            k_sell_pattern<<<gw_count_launch(nblk((int64_t)sell_chunks(v.A.n_rows, lpr) * 32, kThreads)), kThreads, 0, s>>>(
+                make_ptrs(v.A), lpr, v.strips, v.scols);
+            GW_LAUNCHED();
+        }
     memset(plan, 0, sizeof(*plan));
     plan->levels = h.nl;
     plan->dense_n = h.dn;
@@ -534,6 +554,164 @@ int mg_numeric(MgHier &h, cudaStream_t s) {
     k_mg_dense_invert<<<gw_count_launch(1), 1024, smem, s>>>(h.dM, h.dInv, n);
     GW_LAUNCHED();
     return GW_OK;
+}
+
+// -------------------------------------------------------------- 2D: sliced rows
+// Launches one kernel of the Arnoldi step with programmatic dependent launch.
+template <typename... KA, typename... A>
+void launch_pdl(void (*k)(KA...), int grid, int block, size_t smem, cudaStream_t s, A... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(gw_count_launch(grid));
+    cfg.blockDim = dim3(block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute at;
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    (void)cudaLaunchKernelEx(&cfg, k, KA(args)...);  // checked by the caller's GW_LAUNCHED / end of capture
+}
+
+SellA sell_of(const MgLevel &v, bool bf16) {
+    SellA a;
+    a.n_rows = v.A.n_rows;
+    a.n_chunks = sell_chunks(v.A.n_rows, sell_lpr(v.A.n_rows));
+    a.cols = v.scols;
+    a.trips = v.strips;
+    a.vals = bf16 ? v.pvals : v.svals;
+    return a;
+}
+
+// warps per CTA of the sliced row kernels: at most 8 (their register bound)
+int sell_block() { return 32 * std::min(g_tune[GW_TUNE_ROW_WARPS], 8); }
+int sell_grid(const SellA &a) {
+    const int b = nblk(a.n_chunks, sell_block() / 32);
+    return b < 1 ? 1 : b;
+}
+
+// Values of the sliced layout: the finest level on every solve (fresh = false),
+// and after a numeric phase the smoothed coarse levels too, in one launch.
+template <int NF, typename VT>
+int sell_values(const MgHier &h, bool fresh, cudaStream_t s) {
+    SellJobs js;
+    js.n = 0;
+    js.warps = 0;
+    const int last = fresh ? std::max(h.nl - 1, 1) : 1;
+    auto add = [&](const MgLevel &v, void *out) {
+        SellJob &j = js.j[js.n++];
+        j.A = make_ptrs(v.A);
+        j.lpr = sell_lpr(v.A.n_rows);
+        j.first_warp = js.warps;
+        j.trips = v.strips;
+        j.cols = v.scols;
+        j.vals = out;
+        js.warps += sell_chunks(v.A.n_rows, j.lpr);
+    };
+    for (int l = 0; l < last; ++l) add(h.lv[l], h.lv[l].svals);
+    k_sell_values<NF, VT, VT><<<gw_count_launch(nblk((int64_t)js.warps * 32, kThreads)), kThreads, 0, s>>>(js);
+    if constexpr (std::is_same<VT, float>::value) {
+        if (mg_bf16_fine<VT>()) {
+            js.n = js.warps = 0;
+            add(h.lv[0], h.lv[0].pvals);
+            k_sell_values<NF, float, __nv_bfloat16><<<gw_count_launch(nblk((int64_t)js.warps * 32, kThreads)), kThreads, 0, s>>>(js);
+        }
+    }
+    GW_LAUNCHED();
+    return GW_OK;
+}
+
+template <int NF, typename VT>
+void sell_jacobi(const MgHier &h, int l, VecRef b, const double *xin, VecRef xout, const GScalars *sc, cudaStream_t s) {
+    const MgLevel &v = h.lv[l];
+    const bool bf = l == 0 && mg_bf16_fine<VT>();
+    const SellA a = sell_of(v, bf);
+    const double vs = 8.0 * v.A.n_rows * NF, mat = (double)v.A.nnzb * (NF * NF * (bf ? 2 : sizeof(VT)) + 4);
+    ProfScope ps(l == 0 ? PC_MG_JACOBI : PC_MG_JACOBI_COARSE, s, 3 * vs + 8.0 * v.A.n_rows * NF * NF + mat);
+    const bool one = sell_lpr(v.A.n_rows) == 1;
+    void (*k)(SellA, const double *, VecRef, const double *, VecRef, double, const GScalars *);
+    if (bf) k = one ? k_sell_jacobi<NF, __nv_bfloat16, 1> : k_sell_jacobi<NF, __nv_bfloat16, 4>;
+    else k = one ? k_sell_jacobi<NF, VT, 1> : k_sell_jacobi<NF, VT, 4>;
+    launch_pdl(k, sell_grid(a), sell_block(), 0, s, a, (const double *)v.Minv, b, xin, xout, mg_omega(), sc);
+}
+
+template <int NF, typename VT>
+void sell_residual(const MgHier &h, int l, VecRef b, const double *x, const GScalars *sc, cudaStream_t s) {
+    const MgLevel &v = h.lv[l];
+    const bool bf = l == 0 && mg_bf16_fine<VT>();
+    const SellA a = sell_of(v, bf);
+    ProfScope ps(PC_MG_RESID, s, 3 * 8.0 * v.A.n_rows * NF + (double)v.A.nnzb * (NF * NF * (bf ? 2 : sizeof(VT)) + 4));
+    const bool one = sell_lpr(v.A.n_rows) == 1;
+    void (*k)(SellA, VecRef, const double *, double *, const GScalars *);
+    if (bf) k = one ? k_sell_residual<NF, __nv_bfloat16, 1> : k_sell_residual<NF, __nv_bfloat16, 4>;
+    else k = one ? k_sell_residual<NF, VT, 1> : k_sell_residual<NF, VT, 4>;
+    launch_pdl(k, sell_grid(a), sell_block(), 0, s, a, b, x, v.r, sc);
+}
+
+template <int NF, typename VT>
+void sell_spmv(const MgHier &h, VecRef z, const GmresVecs &G, cudaStream_t s) {
+    const SellA a = sell_of(h.lv[0], false);
+    void (*k)(SellA, VecRef, double *, const GScalars *) =
+        sell_lpr(a.n_rows) == 1 ? k_sell_spmv<NF, VT, 1> : k_sell_spmv<NF, VT, 4>;
+    launch_pdl(k, sell_grid(a), sell_block(), 0, s, a, z, G.w, (const GScalars *)G.sc);
+}
+
+// Next basis vector and the finest level's zero-start sweep (none when the
+// finest level is the dense one).
+template <int NF>
+void sell_next(const MgHier &h, const GmresVecs &G, int start, cudaStream_t s) {
+    const MgLevel &v = h.lv[0];
+    launch_pdl(k_gm_next_smooth<NF>, std::max(1, nblk(v.A.n_rows, 128)), 128, 0, s, v.A.n_rows, G, start,
+               (const double *)(h.nl > 1 ? v.Minv : nullptr), v.x, mg_omega());
+}
+
+// One V-cycle on v_k, result in Z[k].  The zero-start sweep of every level comes
+// with its right-hand side (sell_next, k_sell_restrict).
+template <int NF, typename VT>
+void sell_vcycle(const MgHier &h, const GmresVecs &G, VecRef z, cudaStream_t s) {
+    const int last = h.nl - 1;
+    const GScalars *sc = G.sc;
+    const VecRef v0{G.V, G.n};
+    double *cur[kMgMaxLevels], *oth[kMgMaxLevels];
+    for (int l = 0; l < last; ++l) {
+        const MgLevel &v = h.lv[l], &c = h.lv[l + 1];
+        const VecRef b = l == 0 ? v0 : VecRef{v.b, 0};
+        double *x = v.x, *y = v.x2;
+        for (int it = 1; it < mg_sweeps(l); ++it) {
+            sell_jacobi<NF, VT>(h, l, b, x, VecRef{y, 0}, sc, s);
+            std::swap(x, y);
+        }
+        sell_residual<NF, VT>(h, l, b, x, sc, s);
+        {
+            ProfScope ps(PC_MG_TRANSFER, s, 8.0 * NF * (v.A.n_rows + c.A.n_rows));
+            launch_pdl(k_sell_restrict<NF>, nblk(c.A.n_rows, 128), 128, 0, s, c.A.n_rows, v.A.n_rows,
+                       (const int *)c.child, (const uint8_t *)v.fixed, (const double *)v.r, c.b,
+                       (const double *)(l + 1 < last ? c.Minv : nullptr), c.x, mg_omega(), sc);
+        }
+        cur[l] = x;
+        oth[l] = y;
+    }
+    const MgLevel &lc = h.lv[last];
+    const VecRef bl = last == 0 ? v0 : VecRef{lc.b, 0};
+    launch_pdl(k_sell_dense_apply, nblk((int64_t)h.dn * 32, kThreads), kThreads, 0, s, (const double *)h.dInv, bl,
+               last == 0 ? z : VecRef{lc.x, 0}, h.dn, sc);
+    cur[last] = lc.x;
+    for (int l = last - 1; l >= 0; --l) {
+        const MgLevel &v = h.lv[l], &c = h.lv[l + 1];
+        const VecRef b = l == 0 ? v0 : VecRef{v.b, 0};
+        double *x = cur[l], *y = oth[l];
+        {
+            ProfScope ps(PC_MG_TRANSFER, s, 8.0 * NF * (2.0 * v.A.n_rows + c.A.n_rows));
+            launch_pdl(k_sell_prolong<NF>, nblk(v.A.n_rows, 128), 128, 0, s, v.A.n_rows, c.A.n_rows,
+                       (const int *)v.parent, (const uint8_t *)v.fixed, (const double *)cur[l + 1], x, sc);
+        }
+        for (int it = 0; it < mg_sweeps(l); ++it) {
+            const bool out = l == 0 && it + 1 == mg_sweeps(0);
+            sell_jacobi<NF, VT>(h, l, b, x, out ? z : VecRef{y, 0}, sc, s);
+            std::swap(x, y);
+        }
+        cur[l] = x;
+    }
 }
 
 template <int NF, typename VT>
@@ -666,12 +844,11 @@ double *mg_tail(const MgHier &h, int l0, const int *skip, cudaStream_t s) {
     return (swaps & 1) ? h.lv[l0].x2 : h.lv[l0].x;
 }
 
-// One V-cycle on h.lv[0].b; returns the buffer that holds the result (the same
+// 3D (block-CSR rows of up to 125 blocks): one V-cycle on h.lv[0].b; returns the buffer that holds the result (the same
 // buffer on every call).  Levels from tail_level() down run fused (mg_tail).
 template <int NF, typename VT>
 double *mg_vcycle(const MgHier &h, const int *skip, cudaStream_t s) {
     const int last = h.nl - 1;
-    const int D = h.lv[0].g.dim;
     const int l0 = tail_level<NF, VT>(h);
     double *cur[kMgMaxLevels], *oth[kMgMaxLevels];
     for (int l = 0; l < l0; ++l) {
@@ -725,11 +902,7 @@ double *mg_vcycle(const MgHier &h, const int *skip, cudaStream_t s) {
                                     tune_rows_block(), 0, s>>>(a, v.b, x, v.r, skip);
         }
         ProfScope ps(PC_MG_TRANSFER, s, vs + 8.0 * c.A.n_rows * NF);
-        if (D == 2)
-            k_mg_restrict_list<2, NF><<<gw_count_launch(nblk(c.A.n_rows, kThreads)), kThreads, 0, s>>>(
-                c.A.n_rows, v.A.n_rows, c.child, v.fixed, v.r, c.b, skip);
-        else
-            k_mg_restrict_list<3, NF><<<gw_count_launch(nblk(c.A.n_rows, kThreads)), kThreads, 0, s>>>(
+        k_mg_restrict_list<3, NF><<<gw_count_launch(nblk(c.A.n_rows, kThreads)), kThreads, 0, s>>>(
                 c.A.n_rows, v.A.n_rows, c.child, v.fixed, v.r, c.b, skip);
         cur[l] = x;
         oth[l] = y;
@@ -747,11 +920,7 @@ double *mg_vcycle(const MgHier &h, const int *skip, cudaStream_t s) {
         double *x = cur[l], *y = oth[l];
         {
         ProfScope ps(PC_MG_TRANSFER, s, 16.0 * v.A.n_rows * NF + 8.0 * c.A.n_rows * NF);
-        if (D == 2)
-            k_mg_prolong_list<2, NF><<<gw_count_launch(nblk(v.A.n_rows, kThreads)), kThreads, 0, s>>>(
-                v.A.n_rows, c.A.n_rows, v.parent, v.fixed, cur[l + 1], x, skip);
-        else
-            k_mg_prolong_list<3, NF><<<gw_count_launch(nblk(v.A.n_rows, kThreads)), kThreads, 0, s>>>(
+        k_mg_prolong_list<3, NF><<<gw_count_launch(nblk(v.A.n_rows, kThreads)), kThreads, 0, s>>>(
                 v.A.n_rows, c.A.n_rows, v.parent, v.fixed, cur[l + 1], x, skip);
         }
         for (int it = 0; it < mg_sweeps(l); ++it) {
@@ -802,6 +971,17 @@ int capture_stream(cudaStream_t *out) {
 template <int NF, typename VT>
 void mg_arnoldi_step(const MgHier &h, const PtrsA &a, const GmresVecs &G, double *Z, int gr, int gv, size_t n,
                      const int *skip, cudaStream_t s) {
+    if (h.lv[0].g.dim == 2) {
+        const VecRef z{Z, G.n};
+        sell_spmv<NF, VT>(h, z, G, s);
+        launch_pdl(k_gm_dots, gv, kThreads, 0, s, G, 0);
+        launch_pdl(k_gm_update, gv, kThreads, 0, s, G, 0);
+        launch_pdl(k_gm_dots, gv, kThreads, 0, s, G, 1);
+        launch_pdl(k_gm_update, gv, kThreads, 0, s, G, 1);
+        sell_next<NF>(h, G, 0, s);
+        sell_vcycle<NF, VT>(h, G, z, s);
+        return;
+    }
     k_gm_spmv_keep<NF, VT><<<gw_count_launch(resident_rows_grid((const void *)k_gm_spmv_keep<NF, VT>, kThreads, a.n_rows)),
                              kThreads, 0, s>>>(a, G, Z);
     k_gm_dots<<<gw_count_launch(gv), kThreads, 0, s>>>(G, 0);
@@ -921,7 +1101,9 @@ int gmres_mg(const gw_grid_t *grid, const gw_bsr_t *A, gw_mg_plan_t *plan_in, co
         rc = (plan_in && plan_in->lag) ? GW_OK : mg_numeric<NF, VT>(h, s);
         // the V-cycle's BF16 copy of the fine level follows the current A on
         // every solve, lagged or not (the fine level's own rows are never lagged)
-        if (!rc && mg_bf16_fine<VT>()) {
+        if (!rc && grid->dim == 2) {
+            rc = sell_values<NF, VT>(h, !(plan_in && plan_in->lag), s);
+        } else if (!rc && mg_bf16_fine<VT>()) {
             const size_t nv = (size_t)A->nnzb * NF * NF;
             k_to_bf16<<<gw_count_launch(red_grid_elems((int64_t)nv)), kThreads, 0, s>>>(
                 (const float *)A->vals, (__nv_bfloat16 *)h.lv[0].pvals, nv);
@@ -950,9 +1132,13 @@ int gmres_mg(const gw_grid_t *grid, const gw_bsr_t *A, gw_mg_plan_t *plan_in, co
     g_last_stalled = 0;
     for (int cycle = 0; cycle < 1000000; ++cycle) {
         k_gm_residual<NF, VT><<<gw_count_launch(gr), kThreads, 0, s>>>(a, G, first, rtol);
-        k_gm_next_flex<<<gw_count_launch(gv), kThreads, 0, s>>>((size_t)n, G, 1, h.lv[0].b);
-        GW_LAUNCHED();
-        G.z = mg_vcycle<NF, VT>(h, skip, s);
+        if (grid->dim == 2) {
+            sell_next<NF>(h, G, 1, s);
+            sell_vcycle<NF, VT>(h, G, VecRef{fv.Z, (size_t)n}, s);
+        } else {
+            k_gm_next_flex<<<gw_count_launch(gv), kThreads, 0, s>>>((size_t)n, G, 1, h.lv[0].b);
+            G.z = mg_vcycle<NF, VT>(h, skip, s);
+        }
         GW_LAUNCHED();
         first = 0;
         GW_CUDA(cudaMemcpyAsync(&hs, G.sc, head, cudaMemcpyDeviceToHost, s));
@@ -983,14 +1169,25 @@ int gmres_mg(const gw_grid_t *grid, const gw_bsr_t *A, gw_mg_plan_t *plan_in, co
                     continue;
                 }
                 const double vb = 8.0 * n * (kk + 2);
-                { ProfScope ps(PC_SPMV, s, spmv_bytes); k_gm_spmv_keep<NF, VT><<<gw_count_launch(gk), kThreads, 0, s>>>(a, G, fv.Z); }
+                const bool flat = grid->dim == 2;
+                const VecRef z{fv.Z, (size_t)n};
+                {
+                    ProfScope ps(PC_SPMV, s, spmv_bytes);
+                    if (flat) sell_spmv<NF, VT>(h, z, G, s);
+                    else k_gm_spmv_keep<NF, VT><<<gw_count_launch(gk), kThreads, 0, s>>>(a, G, fv.Z);
+                }
                 { ProfScope ps(PC_DOTS, s, vb + 8.0 * n); k_gm_dots<<<gw_count_launch(gv), kThreads, 0, s>>>(G, 0); }
                 { ProfScope ps(PC_UPDATE, s, vb + 8.0 * n); k_gm_update<<<gw_count_launch(gv), kThreads, 0, s>>>(G, 0); }
                 const int re = prof_reorth(G.sc, s);
                 { ProfScope ps(PC_DOTS, s, re ? vb : 0.0); k_gm_dots<<<gw_count_launch(gv), kThreads, 0, s>>>(G, 1); }
                 { ProfScope ps(PC_UPDATE, s, re ? vb + 8.0 * n : 0.0); k_gm_update<<<gw_count_launch(gv), kThreads, 0, s>>>(G, 1); }
-                { ProfScope ps(PC_NEXT, s, 8.0 * n * 3); k_gm_next_flex<<<gw_count_launch(gv), kThreads, 0, s>>>((size_t)n, G, 0, h.lv[0].b); }
-                mg_vcycle<NF, VT>(h, skip, s);
+                {
+                    ProfScope ps(PC_NEXT, s, 8.0 * n * 3);
+                    if (flat) sell_next<NF>(h, G, 0, s);
+                    else k_gm_next_flex<<<gw_count_launch(gv), kThreads, 0, s>>>((size_t)n, G, 0, h.lv[0].b);
+                }
+                if (flat) sell_vcycle<NF, VT>(h, G, z, s);
+                else mg_vcycle<NF, VT>(h, skip, s);
             }
             GW_LAUNCHED();
             GW_CUDA(cudaMemcpyAsync(&hs, G.sc, head, cudaMemcpyDeviceToHost, s));

@@ -15,6 +15,12 @@
 namespace gw {
 namespace {  // internal linkage: each translation unit compiles the kernels it launches
 
+// Programmatic dependent launch: pdl_wait() returns once every earlier kernel of
+// the chain has completed (at once in a kernel launched without the attribute);
+// pdl_release() lets the next kernel of the chain start.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 constexpr int kRedBlocks = 148 * 8;  // grid size of reduction kernels (multiple of the B200 SM count)
 
 struct KScalars {
@@ -718,6 +724,8 @@ __global__ void k_gm_spmv(PtrsA A, GmresVecs G) {
 // (v_i, w) for i <= k; block partials reduced in block order by the last block
 // (pass 0 also (w, w) as item k + 1, and the decision on pass 1)
 __global__ void k_gm_dots(GmresVecs G, int pass) {
+    pdl_wait();
+    pdl_release();
     if (G.sc->cycle_done) return;
     if (pass == 1 && !G.sc->reorth) return;  // uniform over the grid
     const int k = G.sc->k;
@@ -780,6 +788,8 @@ __global__ void k_gm_dots(GmresVecs G, int pass) {
 // k_gm_dots decided against a second pass (pass 1 then has nothing to do),
 // pass 1 otherwise.
 __global__ void k_gm_update(GmresVecs G, int pass) {
+    pdl_wait();
+    pdl_release();
     if (G.sc->cycle_done) return;
     GScalars *sc = G.sc;
     const bool second = sc->reorth;  // set by k_gm_dots pass 0; uniform over the grid

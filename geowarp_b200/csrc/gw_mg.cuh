@@ -521,17 +521,19 @@ __global__ void k_to_bf16(const float *__restrict__ in, __nv_bfloat16 *__restric
 // dependent loads instead of three per child.  The lists keep the loop order
 // of k_mg_restrict / k_mg_prolong, so the sums are bitwise the same.
 
-// child[R * 3^D + q]: fine row of child q (q = ox+1 + 3 (oy+1) [+ 9 (oz+1)]) of
-// coarse row R, -1 where the child is outside the lattice or inactive
+// child[R * 3^D + q] (3D; child[q * n_rows + R] in 2D): fine row of child q
+// (q = ox+1 + 3 (oy+1) [+ 9 (oz+1)]) of coarse row R, -1 where the child is
+// outside the lattice or inactive
 template <int D>
 __global__ void k_mg_children(Lat Lf, PtrsA Af, Lat Lc, PtrsA Ac, int *__restrict__ child) {
     constexpr int CN = D == 2 ? 9 : 27;
     const int R = blockIdx.x * blockDim.x + threadIdx.x;
     if (R >= Ac.n_rows) return;
-    int *out = child + (size_t)R * CN;
+    const size_t st = D == 2 ? (size_t)Ac.n_rows : 1;  // stride over q
+    int *out = child + (D == 2 ? (size_t)R : (size_t)R * CN);
     const int I = Ac.row2node[R];
     if (!in_range(I, lat_size(Lc), GS_RESTRICT)) {
-        for (int q = 0; q < CN; ++q) out[q] = -1;
+        for (int q = 0; q < CN; ++q) out[q * st] = -1;
         return;
     }
     int C[3];
@@ -548,20 +550,21 @@ __global__ void k_mg_children(Lat Lf, PtrsA Af, Lat Lc, PtrsA Ac, int *__restric
                     fr = Af.node2row[lat_id(Lf, ci)];
                     if (fr < 0 || !in_range(fr, Af.n_rows, GS_RESTRICT)) fr = -1;
                 }
-                out[q] = fr;
+                out[q * st] = fr;
             }
 }
 
-// parent[r * 2^D + q]: coarse rows of fine row r in k_mg_prolong's loop order,
-// -1 where that parent is outside the lattice or inactive, -2 past the
-// parity count (the weight of every parent is 1 / that count)
+// parent[r * 2^D + q] (3D; parent[q * n_rows + r] in 2D): coarse rows of fine
+// row r in k_mg_prolong's loop order, -1 where that parent is outside the
+// lattice or inactive, -2 past the parity count (the weight of every parent is 1 / that count)
 template <int D>
 __global__ void k_mg_parents(Lat Lf, PtrsA Af, Lat Lc, PtrsA Ac, int *__restrict__ parent) {
     constexpr int PN = D == 2 ? 4 : 8;
     const int r = blockIdx.x * blockDim.x + threadIdx.x;
     if (r >= Af.n_rows) return;
-    int *out = parent + (size_t)r * PN;
-    for (int q = 0; q < PN; ++q) out[q] = -2;
+    const size_t st = D == 2 ? (size_t)Af.n_rows : 1;  // stride over q
+    int *out = parent + (D == 2 ? (size_t)r : (size_t)r * PN);
+    for (int q = 0; q < PN; ++q) out[q * st] = -2;
     const int node = Af.row2node[r];
     if (!in_range(node, lat_size(Lf), GS_PROLONG)) return;
     int c[3];
@@ -582,7 +585,7 @@ __global__ void k_mg_parents(Lat Lf, PtrsA Af, Lat Lc, PtrsA Ac, int *__restrict
                     R = Ac.node2row[cid];
                     if (R < 0 || !in_range(R, Ac.n_rows, GS_PROLONG)) R = -1;
                 }
-                out[q] = R;
+                out[q * st] = R;
             }
 }
 
