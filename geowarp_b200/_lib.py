@@ -77,7 +77,7 @@ class MgPlan(C.Structure):
     _fields_ = [("levels", C.c_int32), ("dense_n", C.c_int32), ("n_rows", C.c_int32 * MG_MAX_LEVELS),
                 ("nnzb", C.c_int32 * MG_MAX_LEVELS), ("nf", C.c_int32), ("fine_n_rows", C.c_int32),
                 ("fine_nnzb", C.c_int32), ("lag", C.c_int32), ("workspace", C.c_void_p),
-                ("row_ptr", C.c_void_p), ("cols", C.c_void_p), ("last_iters", C.c_int32), ("pad0", C.c_int32)]
+                ("row_ptr", C.c_void_p), ("cols", C.c_void_p), ("last_iters", C.c_int32), ("last_rate", C.c_int32)]
 
 
 class Adjoint(C.Structure):

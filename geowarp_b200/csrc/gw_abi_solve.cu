@@ -104,6 +104,8 @@ int krylov_nf(const gw_bsr_t *A, int method, int precond, const double *b, doubl
 }  // namespace
 
 namespace {
+// block partials of a GMRES solve: the Gram-Schmidt items, or two values per block of k_gm_residual
+constexpr int kGmresPartials = kGsPartials > 2 * kRedBlocks ? kGsPartials : 2 * kRedBlocks;
 // second Gram-Schmidt passes of the last GMRES solve on this host thread
 thread_local int g_last_reorths = 0;
 // whether the last GMRES solve on this host thread stopped on stagnation
@@ -132,21 +134,68 @@ class StallWatch {
     std::vector<double> hist_;
 };
 
+// Launches one kernel of the Arnoldi step with programmatic dependent launch.
+template <typename... KA, typename... A>
+void launch_pdl(void (*k)(KA...), int grid, int block, size_t smem, cudaStream_t s, A... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(gw_count_launch(grid));
+    cfg.blockDim = dim3(block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute at;
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    (void)cudaLaunchKernelEx(&cfg, k, KA(args)...);  // checked by the caller's GW_LAUNCHED / end of capture
+}
+
+// The Gram-Schmidt kernels of one column: both passes, or the first one alone.
+void gs_dots(const GmresVecs &G, int restart, int pass, cudaStream_t s) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(gw_count_launch(gs_dots_blocks(G.n)), (restart + 1 + kGsGroup - 1) / kGsGroup);
+    cfg.blockDim = dim3(kGsThreads);
+    cfg.stream = s;
+    cudaLaunchAttribute at;
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    (void)cudaLaunchKernelEx(&cfg, k_gm_dots, G, pass);
+}
+void gs_update(const GmresVecs &G, int pass, cudaStream_t s) {
+    launch_pdl(k_gm_update, gs_update_blocks(G.n), kGsThreads, 0, s, G, pass);
+}
+template <int NF>
+void gs_next(int n_rows, const GmresVecs &G, int start, const double *Minv, double *zout, double scale, cudaStream_t s) {
+    // block 0 closes the column, the others take one row per thread
+    launch_pdl(k_gm_next<NF>, 1 + nblk(n_rows, kGsThreads), kGsThreads, 0, s, n_rows, G, start, Minv, zout, scale);
+}
+
 // Profiling only: whether column k takes the second Gram-Schmidt pass (read
-// after pass 0), so that the timed pass-1 launches are credited with the bytes
-// they move.  Timed runs without profiling never read it.
+// after pass 0), so that the timed launches queue it where it is needed.  Runs
+// without profiling never read it.
 int prof_reorth(GScalars *sc, cudaStream_t s) {
-    if (!g_prof_on) return 1;
     int re = 1;
     if (cudaMemcpyAsync(&re, &sc->reorth, sizeof(int), cudaMemcpyDeviceToHost, s) != cudaSuccess) return 1;
     if (cudaStreamSynchronize(s) != cudaSuccess) return 1;
     return re;
 }
 
+// The Gram-Schmidt kernels of a column; profiled runs queue the second pass only
+// where the column takes it.
+void gs_column(const GmresVecs &G, int restart, double vb, cudaStream_t s) {
+    const double n8 = 8.0 * G.n;
+    { ProfScope ps(PC_DOTS, s, vb + n8); gs_dots(G, restart, 0, s); }
+    { ProfScope ps(PC_UPDATE, s, vb + n8); gs_update(G, 0, s); }
+    if (g_prof_on && !prof_reorth(G.sc, s)) return;
+    { ProfScope ps(PC_DOTS, s, vb); gs_dots(G, restart, 1, s); }
+    { ProfScope ps(PC_UPDATE, s, vb + n8); gs_update(G, 1, s); }
+}
 int64_t gmres_ws_bytes(int64_t n_rows, int nf, int restart) {
     const int64_t n = n_rows * nf;
     return align256(8 * n * (restart + 1)) + 2 * align256(8 * n) + align256(8 * n_rows * nf * nf) +
-           align256(8 * (int64_t)kRedBlocks * (kGmresMaxRestart + 1)) + align256(sizeof(GScalars));
+           align256(8 * (int64_t)kGmresPartials) + align256(sizeof(GScalars));
 }
 
 template <int NF, typename VT>
@@ -162,7 +211,7 @@ int gmres(const gw_bsr_t *A, int precond, const double *b, double *x, double rto
     G.w = (double *)w; w += align256(8 * n);
     G.z = (double *)w; w += align256(8 * n);
     G.Minv = (double *)w; w += align256(8 * (int64_t)nr * NF * NF);
-    G.partials = (double *)w; w += align256(8 * (int64_t)kRedBlocks * (kGmresMaxRestart + 1));
+    G.partials = (double *)w; w += align256(8 * (int64_t)kGmresPartials);
     G.sc = (GScalars *)w;
     G.x = x; G.b = b; G.n = (size_t)n;
     const size_t head = offsetof(GScalars, H);
@@ -174,7 +223,7 @@ int gmres(const gw_bsr_t *A, int precond, const double *b, double *x, double rto
     const int D = (A->mask_words == 1) ? 2 : 3;
     k_precond_setup<NF, VT><<<gw_count_launch(nblk(nr, kThreads)), kThreads, 0, s>>>(a, D, precond, G.Minv);
     GW_LAUNCHED();
-    const int gr = red_grid_rows(nr), ge = red_grid_elems(nr), gv = red_grid_elems(n);
+    const int gr = red_grid_rows(nr), ge = red_grid_elems(nr);
     GScalars h;
     memset(&h, 0, head);
     int first = 1;
@@ -182,7 +231,7 @@ int gmres(const gw_bsr_t *A, int precond, const double *b, double *x, double rto
     g_last_stalled = 0;
     for (int cycle = 0; cycle < 1000000; ++cycle) {
         k_gm_residual<NF, VT><<<gw_count_launch(gr), kThreads, 0, s>>>(a, G, first, rtol);
-        k_gm_next<NF><<<gw_count_launch(ge), kThreads, 0, s>>>(nr, G, 1);
+        gs_next<NF>(nr, G, 1, G.Minv, G.z, 1.0, s);
         GW_LAUNCHED();
         first = 0;
         GW_CUDA(cudaMemcpyAsync(&h, G.sc, head, cudaMemcpyDeviceToHost, s));
@@ -195,13 +244,9 @@ int gmres(const gw_bsr_t *A, int precond, const double *b, double *x, double rto
         for (;;) {
             for (int it = 0; it < chunk; ++it, ++kk) {
                 const double vb = 8.0 * n * (kk + 2);
-                { ProfScope ps(PC_SPMV, s, spmv_bytes); k_gm_spmv<NF, VT><<<gw_count_launch(gr), kThreads, 0, s>>>(a, G); }
-                { ProfScope ps(PC_DOTS, s, vb + 8.0 * n); k_gm_dots<<<gw_count_launch(gv), kThreads, 0, s>>>(G, 0); }
-                { ProfScope ps(PC_UPDATE, s, vb + 8.0 * n); k_gm_update<<<gw_count_launch(gv), kThreads, 0, s>>>(G, 0); }
-                const int re = prof_reorth(G.sc, s);
-                { ProfScope ps(PC_DOTS, s, re ? vb : 0.0); k_gm_dots<<<gw_count_launch(gv), kThreads, 0, s>>>(G, 1); }
-                { ProfScope ps(PC_UPDATE, s, re ? vb + 8.0 * n : 0.0); k_gm_update<<<gw_count_launch(gv), kThreads, 0, s>>>(G, 1); }
-                { ProfScope ps(PC_NEXT, s, 8.0 * n * 3 + 8.0 * nr * NF * NF); k_gm_next<NF><<<gw_count_launch(ge), kThreads, 0, s>>>(nr, G, 0); }
+                { ProfScope ps(PC_SPMV, s, spmv_bytes); launch_pdl(k_gm_spmv<NF, VT>, gr, kThreads, 0, s, a, G); }
+                gs_column(G, restart, vb, s);
+                { ProfScope ps(PC_NEXT, s, 8.0 * n * 3 + 8.0 * nr * NF * NF); gs_next<NF>(nr, G, 0, G.Minv, G.z, 1.0, s); }
             }
             GW_LAUNCHED();
             GW_CUDA(cudaMemcpyAsync(&h, G.sc, head, cudaMemcpyDeviceToHost, s));
@@ -390,7 +435,7 @@ void mg_carve_flex(Bump &bp, FlexVecs &fv, int64_t n0, int restart) {
     fv.V = (double *)bp.take(8 * n0 * (restart + 1));
     fv.Z = (double *)bp.take(8 * n0 * restart);
     fv.w = (double *)bp.take(8 * n0);
-    fv.partials = (double *)bp.take(8 * (int64_t)kRedBlocks * (kGmresMaxRestart + 1));
+    fv.partials = (double *)bp.take(8 * (int64_t)kGmresPartials);
     fv.sc = (GScalars *)bp.take(sizeof(GScalars));
 }
 
@@ -557,22 +602,6 @@ int mg_numeric(MgHier &h, cudaStream_t s) {
 }
 
 // -------------------------------------------------------------- 2D: sliced rows
-// Launches one kernel of the Arnoldi step with programmatic dependent launch.
-template <typename... KA, typename... A>
-void launch_pdl(void (*k)(KA...), int grid, int block, size_t smem, cudaStream_t s, A... args) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(gw_count_launch(grid));
-    cfg.blockDim = dim3(block);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = s;
-    cudaLaunchAttribute at;
-    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at.val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = &at;
-    cfg.numAttrs = 1;
-    (void)cudaLaunchKernelEx(&cfg, k, KA(args)...);  // checked by the caller's GW_LAUNCHED / end of capture
-}
-
 SellA sell_of(const MgLevel &v, bool bf16) {
     SellA a;
     a.n_rows = v.A.n_rows;
@@ -656,17 +685,19 @@ void sell_spmv(const MgHier &h, VecRef z, const GmresVecs &G, cudaStream_t s) {
     launch_pdl(k, sell_grid(a), sell_block(), 0, s, a, z, G.w, (const GScalars *)G.sc);
 }
 
-// Next basis vector and the finest level's zero-start sweep (none when the
-// finest level is the dense one).
+// Next basis vector and what the V-cycle starts from: in 2D the finest level's
+// zero-start sweep (nothing when the finest level is the dense one), in 3D its
+// right-hand side.
 template <int NF>
-void sell_next(const MgHier &h, const GmresVecs &G, int start, cudaStream_t s) {
+void mg_next(const MgHier &h, const GmresVecs &G, int start, cudaStream_t s) {
     const MgLevel &v = h.lv[0];
-    launch_pdl(k_gm_next_smooth<NF>, std::max(1, nblk(v.A.n_rows, 128)), 128, 0, s, v.A.n_rows, G, start,
-               (const double *)(h.nl > 1 ? v.Minv : nullptr), v.x, mg_omega());
+    const bool flat = v.g.dim == 2, smooth = flat && h.nl > 1;
+    gs_next<NF>(v.A.n_rows, G, start, smooth ? v.Minv : nullptr, flat ? (smooth ? v.x : nullptr) : v.b,
+                smooth ? mg_omega() : 1.0, s);
 }
 
 // One V-cycle on v_k, result in Z[k].  The zero-start sweep of every level comes
-// with its right-hand side (sell_next, k_sell_restrict).
+// with its right-hand side (mg_next, k_sell_restrict).
 template <int NF, typename VT>
 void sell_vcycle(const MgHier &h, const GmresVecs &G, VecRef z, cudaStream_t s) {
     const int last = h.nl - 1;
@@ -968,34 +999,34 @@ int capture_stream(cudaStream_t *out) {
     return GW_OK;
 }
 
+// The next basis vector (start: the first of a cycle) and its V-cycle.
 template <int NF, typename VT>
-void mg_arnoldi_step(const MgHier &h, const PtrsA &a, const GmresVecs &G, double *Z, int gr, int gv, size_t n,
+void mg_step_tail(const MgHier &h, GmresVecs &G, VecRef z, int start, const int *skip, cudaStream_t s) {
+    { ProfScope ps(PC_NEXT, s, 8.0 * G.n * 3); mg_next<NF>(h, G, start, s); }
+    if (h.lv[0].g.dim == 2) sell_vcycle<NF, VT>(h, G, z, s);
+    else G.z = mg_vcycle<NF, VT>(h, skip, s);
+}
+
+// One Arnoldi step and the V-cycle of the new basis vector.
+template <int NF, typename VT>
+void mg_arnoldi_step(const MgHier &h, const PtrsA &a, GmresVecs &G, double *Z, int restart,
                      const int *skip, cudaStream_t s) {
-    if (h.lv[0].g.dim == 2) {
-        const VecRef z{Z, G.n};
-        sell_spmv<NF, VT>(h, z, G, s);
-        launch_pdl(k_gm_dots, gv, kThreads, 0, s, G, 0);
-        launch_pdl(k_gm_update, gv, kThreads, 0, s, G, 0);
-        launch_pdl(k_gm_dots, gv, kThreads, 0, s, G, 1);
-        launch_pdl(k_gm_update, gv, kThreads, 0, s, G, 1);
-        sell_next<NF>(h, G, 0, s);
-        sell_vcycle<NF, VT>(h, G, z, s);
-        return;
+    const VecRef z{Z, G.n};
+    const bool flat = h.lv[0].g.dim == 2;
+    {
+        ProfScope ps(PC_SPMV, s, (double)h.lv[0].A.nnzb * (NF * NF * sizeof(VT) + 4) + 4.0 * (a.n_rows + 1) + 24.0 * G.n);
+        if (flat) sell_spmv<NF, VT>(h, z, G, s);
+        else k_gm_spmv_keep<NF, VT><<<gw_count_launch(resident_rows_grid((const void *)k_gm_spmv_keep<NF, VT>, kThreads, a.n_rows)),
+                                      kThreads, 0, s>>>(a, G, Z);
     }
-    k_gm_spmv_keep<NF, VT><<<gw_count_launch(resident_rows_grid((const void *)k_gm_spmv_keep<NF, VT>, kThreads, a.n_rows)),
-                             kThreads, 0, s>>>(a, G, Z);
-    k_gm_dots<<<gw_count_launch(gv), kThreads, 0, s>>>(G, 0);
-    k_gm_update<<<gw_count_launch(gv), kThreads, 0, s>>>(G, 0);
-    k_gm_dots<<<gw_count_launch(gv), kThreads, 0, s>>>(G, 1);
-    k_gm_update<<<gw_count_launch(gv), kThreads, 0, s>>>(G, 1);
-    k_gm_next_flex<<<gw_count_launch(gv), kThreads, 0, s>>>(n, G, 0, h.lv[0].b);
-    mg_vcycle<NF, VT>(h, skip, s);
+    gs_column(G, restart, 8.0 * G.n * (restart / 2), s);
+    mg_step_tail<NF, VT>(h, G, z, 0, skip, s);
 }
 
 // Returns the cached (or newly captured) graph of one Arnoldi step.
 template <int NF, typename VT>
-int mg_step_graph(const MgHier &h, const gw_grid_t &grid, const gw_bsr_t *A, const GmresVecs &G, double *Z, void *ws,
-                  int restart, int gr, int gv, size_t n, const int *skip, cudaGraphExec_t *exec, int64_t *nodes) {
+int mg_step_graph(const MgHier &h, const gw_grid_t &grid, const gw_bsr_t *A, GmresVecs &G, double *Z, void *ws,
+                  int restart, const int *skip, cudaGraphExec_t *exec, int64_t *nodes) {
     MgGraphKey k;
     memset(&k, 0, sizeof(k));
     GW_CUDA(cudaGetDevice(&k.device));
@@ -1029,7 +1060,7 @@ int mg_step_graph(const MgHier &h, const gw_grid_t &grid, const gw_bsr_t *A, con
     PtrsA a = make_ptrs(*A);
     const int64_t before = g_launches;
     GW_CUDA(cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal));
-    mg_arnoldi_step<NF, VT>(h, a, G, Z, gr, gv, n, skip, cs);
+    mg_arnoldi_step<NF, VT>(h, a, G, Z, restart, skip, cs);
     cudaGraph_t graph;
     const cudaError_t ce = cudaStreamEndCapture(cs, &graph);
     const int64_t count = g_launches - before;
@@ -1123,7 +1154,7 @@ int gmres_mg(const gw_grid_t *grid, const gw_bsr_t *A, gw_mg_plan_t *plan_in, co
     const double eta2 = ::pow(10.0, -0.1 * g_tune[GW_TUNE_GS_CANCEL]);
     GW_CUDA(cudaMemcpyAsync(&G.sc->gs_eta2, &eta2, sizeof(double), cudaMemcpyHostToDevice, s));
     const int gr = red_grid_rows(nr), gv = red_grid_elems(n);
-    const int gk = resident_rows_grid((const void *)k_gm_spmv_keep<NF, VT>, kThreads, nr);
+    const VecRef z{fv.Z, (size_t)n};
     const int *skip = &G.sc->cycle_done;
     GScalars hs;
     memset(&hs, 0, head);
@@ -1132,73 +1163,50 @@ int gmres_mg(const gw_grid_t *grid, const gw_bsr_t *A, gw_mg_plan_t *plan_in, co
     g_last_stalled = 0;
     for (int cycle = 0; cycle < 1000000; ++cycle) {
         k_gm_residual<NF, VT><<<gw_count_launch(gr), kThreads, 0, s>>>(a, G, first, rtol);
-        if (grid->dim == 2) {
-            sell_next<NF>(h, G, 1, s);
-            sell_vcycle<NF, VT>(h, G, VecRef{fv.Z, (size_t)n}, s);
-        } else {
-            k_gm_next_flex<<<gw_count_launch(gv), kThreads, 0, s>>>((size_t)n, G, 1, h.lv[0].b);
-            G.z = mg_vcycle<NF, VT>(h, skip, s);
-        }
+        GW_LAUNCHED();
+        mg_step_tail<NF, VT>(h, G, z, 1, skip, s);
         GW_LAUNCHED();
         first = 0;
         GW_CUDA(cudaMemcpyAsync(&hs, G.sc, head, cudaMemcpyDeviceToHost, s));
         GW_CUDA(cudaStreamSynchronize(s));
         if (hs.done) break;
         if (stall.stalled(hs.beta)) { g_last_stalled = 1; break; }
-        // Arnoldi steps queued before the next host check: the previous
-        // solve's iteration count to start with (Newton solves of a step look
-        // alike), then the iterations left at the observed convergence rate.
-        // Steps queued past convergence still launch their (early-exiting)
-        // kernels, so the estimate trims them without adding host reads.
-        const int hint = plan_in ? plan_in->last_iters : 0;
-        int chunk = hint > 0 ? std::min(std::max(hint, 2), 16) : 4;
-        int kk = 0;
-        const double spmv_bytes = (double)A->nnzb * (NF * NF * sizeof(VT) + 4) + 4.0 * (nr + 1) + 24.0 * n;
-        cudaGraphExec_t step_graph = nullptr;
-        int64_t step_nodes = 0;
-        if (!g_prof_on) {  // timed runs launch kernel by kernel, bracketed by events
-            rc = mg_step_graph<NF, VT>(h, *grid, A, G, fv.Z, ws, restart, gr, gv, (size_t)n, skip, &step_graph,
-                                       &step_nodes);
-            if (rc) return rc;
-        }
+        // Arnoldi steps queued before the next host check.  A step queued past
+        // convergence costs as much as one that counts, a check 10-15 us of idle
+        // device: nine tenths of the steps that the previous solve's convergence
+        // rate predicts (solves of one load step contract alike), then what the
+        // observed rate leaves.
+        int chunk = 4;
+        if (plan_in && plan_in->last_rate > 0 && hs.tol > 0.0 && hs.beta > hs.tol)
+            chunk = (int)std::min(0.9 * ::log(hs.beta / hs.tol) / (1e-3 * plan_in->last_rate), 1e6);
+        else if (plan_in && plan_in->last_iters > 0)
+            chunk = std::min(plan_in->last_iters, 16);
+        chunk = std::min(std::max(chunk, 1), std::min(restart, std::max(max_iter - hs.iters, 1)));
         for (;;) {
-            for (int it = 0; it < chunk; ++it, ++kk) {
+            cudaGraphExec_t step_graph = nullptr;
+            int64_t step_nodes = 0;
+            if (!g_prof_on) {  // timed runs launch kernel by kernel, bracketed by events
+                rc = mg_step_graph<NF, VT>(h, *grid, A, G, fv.Z, ws, restart, skip, &step_graph, &step_nodes);
+                if (rc) return rc;
+            }
+            for (int it = 0; it < chunk; ++it) {
                 if (step_graph) {
                     GW_CUDA(cudaGraphLaunch(step_graph, s));
                     g_launches += step_nodes;
-                    continue;
+                } else {
+                    mg_arnoldi_step<NF, VT>(h, a, G, fv.Z, restart, skip, s);
                 }
-                const double vb = 8.0 * n * (kk + 2);
-                const bool flat = grid->dim == 2;
-                const VecRef z{fv.Z, (size_t)n};
-                {
-                    ProfScope ps(PC_SPMV, s, spmv_bytes);
-                    if (flat) sell_spmv<NF, VT>(h, z, G, s);
-                    else k_gm_spmv_keep<NF, VT><<<gw_count_launch(gk), kThreads, 0, s>>>(a, G, fv.Z);
-                }
-                { ProfScope ps(PC_DOTS, s, vb + 8.0 * n); k_gm_dots<<<gw_count_launch(gv), kThreads, 0, s>>>(G, 0); }
-                { ProfScope ps(PC_UPDATE, s, vb + 8.0 * n); k_gm_update<<<gw_count_launch(gv), kThreads, 0, s>>>(G, 0); }
-                const int re = prof_reorth(G.sc, s);
-                { ProfScope ps(PC_DOTS, s, re ? vb : 0.0); k_gm_dots<<<gw_count_launch(gv), kThreads, 0, s>>>(G, 1); }
-                { ProfScope ps(PC_UPDATE, s, re ? vb + 8.0 * n : 0.0); k_gm_update<<<gw_count_launch(gv), kThreads, 0, s>>>(G, 1); }
-                {
-                    ProfScope ps(PC_NEXT, s, 8.0 * n * 3);
-                    if (flat) sell_next<NF>(h, G, 0, s);
-                    else k_gm_next_flex<<<gw_count_launch(gv), kThreads, 0, s>>>((size_t)n, G, 0, h.lv[0].b);
-                }
-                if (flat) sell_vcycle<NF, VT>(h, G, z, s);
-                else mg_vcycle<NF, VT>(h, skip, s);
             }
             GW_LAUNCHED();
             GW_CUDA(cudaMemcpyAsync(&hs, G.sc, head, cudaMemcpyDeviceToHost, s));
             GW_CUDA(cudaStreamSynchronize(s));
             if (hs.cycle_done) break;
-            int next = chunk < 16 ? chunk * 2 : 16;
+            int next = std::min(chunk < 16 ? chunk * 2 : 16, restart - hs.k);
             if (hs.k > 0 && hs.beta > 0.0 && hs.resid > 0.0 && hs.resid < hs.beta && hs.tol > 0.0) {
                 const double rate = ::pow(hs.resid / hs.beta, 1.0 / hs.k);
                 if (rate < 1.0) {
                     const double left = ::ceil(::log(hs.tol / hs.resid) / ::log(rate));
-                    next = left < 1.0 ? 1 : (left > 16.0 ? 16 : (int)left);
+                    next = (int)std::min(std::max(left, 1.0), (double)(restart - hs.k));
                 }
             }
             chunk = next;
@@ -1211,7 +1219,12 @@ int gmres_mg(const gw_grid_t *grid, const gw_bsr_t *A, gw_mg_plan_t *plan_in, co
     *iters = hs.iters;
     g_last_reorths = hs.reorths;
     *relres = (hs.bnorm > 0.0) ? hs.resid / hs.bnorm : 0.0;
-    if (plan_in) plan_in->last_iters = hs.iters;
+    if (plan_in) {
+        plan_in->last_iters = hs.iters;
+        plan_in->last_rate = 0;
+        if (hs.iters > 0 && hs.resid > 0.0 && hs.resid < hs.bnorm)
+            plan_in->last_rate = (int)(1e3 * ::log(hs.bnorm / hs.resid) / hs.iters);
+    }
     rc = guard_check(s, "multigrid GMRES");
     if (rc) return rc;
     if (hs.status == ST_NAN) return GW_ENAN;

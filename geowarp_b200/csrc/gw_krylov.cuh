@@ -154,6 +154,33 @@ __device__ __forceinline__ void load_vec(const double *__restrict__ p, double ou
     }
 }
 
+// one row's vector through the ordinary (coherent) path: 16-byte accesses where
+// the row starts are aligned (NF = 2, 4: buffers are; a basis vector of n
+// unknowns is when n is even, and n is a multiple of NF)
+template <int NF>
+__device__ __forceinline__ void load_rw(const double *p, double out[NF]) {
+    if constexpr (NF == 2 || NF == 4) {
+#pragma unroll
+        for (int q = 0; q < NF / 2; ++q) {
+            const double2 v = reinterpret_cast<const double2 *>(p)[q];
+            out[2 * q] = v.x; out[2 * q + 1] = v.y;
+        }
+    } else {
+#pragma unroll
+        for (int g = 0; g < NF; ++g) out[g] = p[g];
+    }
+}
+template <int NF>
+__device__ __forceinline__ void store_rw(double *p, const double v[NF]) {
+    if constexpr (NF == 2 || NF == 4) {
+#pragma unroll
+        for (int q = 0; q < NF / 2; ++q) reinterpret_cast<double2 *>(p)[q] = make_double2(v[2 * q], v[2 * q + 1]);
+    } else {
+#pragma unroll
+        for (int g = 0; g < NF; ++g) p[g] = v[g];
+    }
+}
+
 // Block rows are processed by groups of kLPR lanes, kRowsPerWarp rows per
 // warp in flight: the lanes of a group take consecutive blocks of their row
 // (kLPR x 16 bytes per step for 2x2 FP32 blocks: one 128-byte line) and a
@@ -607,21 +634,20 @@ namespace {  // internal linkage: each translation unit compiles the kernels it 
 // ---------------------------------------------------------------- restarted GMRES(m)
 // Right-preconditioned GMRES with classical Gram-Schmidt and a
 // re-orthogonalisation pass when needed.  Column k of the Arnoldi process is
-// six kernels:
-//   spmv:  w = A z_k                       (z_k = Minv v_k)
-//   dots:  h_i = (v_i, w), i <= k, and (w, w)   (pass 0); the last block
-//          decides the second pass: ||w - V h||^2 = (w, w) - sum h_i^2 below
+// four kernels:
+//   spmv:  w = A z_k                       (z_k = Minv v_k, or a V-cycle)
+//   dots:  block partials of (v_i, w), i <= k, and (w, w)
+//   upd:   every block sums the partials to h; w -= V h; block partials of
+//          ||w||^2; block 0 stores h.  ||w - V h||^2 = (w, w) - sum h_i^2 below
 //          gs_eta2 (w, w) (by default 1/100: the projection removed more than
-//          90% of w's norm) means V h lost more than ~10 ulp of orthogonality
-//          and the pass is repeated
-//   upd:   w -= V h                        (pass 0)
-//   dots:  h2_i = (v_i, w)                 (pass 1, only when needed)
-//   upd:   w -= V h2 (only when needed) ; ||w||; last block: Hessenberg
-//          column, Givens rotation, residual estimate, cycle/convergence
-//          flags, k += 1
-//   next:  v_k = w / ||w|| ; z_k = Minv v_k
-// The skipped pass reads no basis vector, so an Arnoldi step without strong
-// cancellation reads the basis twice instead of four times.
+//          90% of w's norm) means V h lost more than ~10 ulp of orthogonality and
+//          a second pass (dots and upd with pass = 1) is needed
+//   next:  every block sums ||w||; v_{k+1} = w / ||w||, z_{k+1}; meanwhile block 0
+//          closes the column: Givens rotation, residual estimate, cycle /
+//          convergence flags, k += 1
+// No kernel ends in a grid-wide reduction: its consumer sums the partials in
+// block order (deterministic).  The second pass is queued with every column and
+// returns at once where the first one is enough.
 // Robust for the nonsymmetric, indefinite Jacobians of the penalty footing
 // and the u-p saddle-point systems, on which BiCGSTAB breaks down.
 constexpr int kGmresMaxRestart = 128;
@@ -634,6 +660,7 @@ struct GScalars {
     int cycle_done, done, status, iters, max_iter, restart;
     unsigned ticket;
     int reorth;      // column k takes the second Gram-Schmidt pass
+    int kn;          // basis vector `next` forms (its own copy: block 0 advances k meanwhile)
     int reorths;     // second passes taken in this solve
     double H[kGmresMaxRestart + 1][kGmresMaxRestart];
     double cs[kGmresMaxRestart], sn[kGmresMaxRestart];
@@ -681,6 +708,7 @@ __global__ void k_gm_residual(PtrsA A, GmresVecs G, int first, double rtol) {
         sc->resid = sc->beta;
         sc->k = 0;
         sc->cycle_done = 0;
+        sc->reorth = sc->kn = 0;
         sc->g[0] = sc->beta;
         for (int i = 1; i <= kGmresMaxRestart; ++i) sc->g[i] = 0.0;
         if (!isfinite(sc->beta)) { sc->status = ST_NAN; sc->done = 1; sc->cycle_done = 1; }
@@ -688,27 +716,11 @@ __global__ void k_gm_residual(PtrsA A, GmresVecs G, int first, double rtol) {
     }
 }
 
-// v_k = w / s ; z_k = Minv v_k   (s = beta at a cycle start, ||w|| afterwards)
-template <int NF>
-__global__ void k_gm_next(int n_rows, GmresVecs G, int start) {
-    if (G.sc->cycle_done) return;
-    const int k = G.sc->k;
-    if (!in_range(k, G.sc->restart + 1, GS_KRYLOV_K)) return;
-    const double ih = 1.0 / (start ? G.sc->beta : G.sc->wnorm);
-    double *vn = G.V + (size_t)k * G.n;
-    for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < n_rows; r += gridDim.x * blockDim.x) {
-        double v[NF], z[NF];
-#pragma unroll
-        for (int f = 0; f < NF; ++f) { v[f] = G.w[(size_t)r * NF + f] * ih; vn[(size_t)r * NF + f] = v[f]; }
-        apply_minv<NF>(G.Minv, r, v, z);
-#pragma unroll
-        for (int f = 0; f < NF; ++f) G.z[(size_t)r * NF + f] = z[f];
-    }
-}
-
 // w = A z_k
 template <int NF, typename VT>
 __global__ void k_gm_spmv(PtrsA A, GmresVecs G) {
+    pdl_wait();
+    pdl_release();
     if (G.sc->cycle_done) return;
     const int nw = gridDim.x * (blockDim.x >> 5) * kRowsPerWarp;
     for (int rb = (blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * kRowsPerWarp; rb < A.n_rows; rb += nw) {
@@ -721,131 +733,379 @@ __global__ void k_gm_spmv(PtrsA A, GmresVecs G) {
     }
 }
 
-// (v_i, w) for i <= k; block partials reduced in block order by the last block
-// (pass 0 also (w, w) as item k + 1, and the decision on pass 1)
-__global__ void k_gm_dots(GmresVecs G, int pass) {
+// ---------------------------------------------------------------- Gram-Schmidt
+// What bounds these kernels: the basis, read once by dots and once by upd (8 (k + 1) n
+// bytes each), and on systems below ~50k unknowns the latency of the reduction.
+// Dots and update of column 8, B200: 532k unknowns 49 us as one kernel each with a
+// last-block reduction -> 12 + 11 us; 52k unknowns 20 -> 2 + 4 us; 864 unknowns with a
+// 100-vector basis (3D node-block GMRES): one iteration 90 -> 46 us.
+constexpr int kGsThreads = 256;
+constexpr int kGsBlocks = 296;                    // element blocks: two per SM
+constexpr int kGsItems = kGmresMaxRestart + 1;    // (v_i, w), i <= k < restart, and (w, w)
+constexpr int kGsGroup = 8;                       // items per block of k_gm_dots
+constexpr int kGsSplitMax = 16384;                // unknowns up to which k_gm_update splits the basis over warps
+// partials: dots item i of element block b at [i * kGsBlocks + b]; ||w||^2 after them
+constexpr int kGsPartials = (kGsItems + 1) * kGsBlocks;
+
+// element blocks of k_gm_dots (gridDim.x) and of k_gm_update for n unknowns
+__host__ __device__ inline int gs_dots_blocks(size_t n) {
+    const size_t b = (n / 2 + kGsThreads - 1) / kGsThreads;
+    return b < 1 ? 1 : (b > (size_t)kGsBlocks ? kGsBlocks : (int)b);
+}
+__host__ __device__ inline int gs_update_blocks(size_t n) {
+    const size_t per = n <= (size_t)kGsSplitMax ? 64 : 2 * kGsThreads;
+    const size_t b = (n + per - 1) / per;
+    return b < 1 ? 1 : (b > (size_t)kGsBlocks ? kGsBlocks : (int)b);
+}
+// a warp's sum in a fixed tree, valid in every lane
+__device__ __forceinline__ double warp_sum(double v) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
+}
+
+// one thread's share of inner products g .. g + CNT - 1 (CNT = 0: cnt of them, at
+// run time); item k + 1 is (w, w)
+template <bool PAIR, int CNT>
+__device__ __forceinline__ void gs_dots_body(const GmresVecs &G, int g, int cnt, int k, double acc[kGsGroup]) {
+    const size_t n = G.n, nv = PAIR ? n / 2 : n;
+    const size_t T = (size_t)gridDim.x * kGsThreads;
+    constexpr int M = CNT ? CNT : kGsGroup;
+#pragma unroll 2
+    for (size_t e = (size_t)blockIdx.x * kGsThreads + threadIdx.x; e < nv; e += T) {
+        if (PAIR) {
+            const double2 w = reinterpret_cast<const double2 *>(G.w)[e];
+            double2 x[M];
+#pragma unroll
+            for (int v = 0; v < M; ++v)
+                if (CNT || v < cnt)
+                    x[v] = reinterpret_cast<const double2 *>((CNT || g + v <= k) ? G.V + (size_t)(g + v) * n : G.w)[e];
+#pragma unroll
+            for (int v = 0; v < M; ++v)
+                if (CNT || v < cnt) acc[v] += x[v].x * w.x + x[v].y * w.y;
+        } else {
+            const double w = G.w[e];
+            double x[M];
+#pragma unroll
+            for (int v = 0; v < M; ++v)
+                if (CNT || v < cnt) x[v] = ((CNT || g + v <= k) ? G.V + (size_t)(g + v) * n : G.w)[e];
+#pragma unroll
+            for (int v = 0; v < M; ++v)
+                if (CNT || v < cnt) acc[v] += x[v] * w;
+        }
+    }
+}
+
+// Block (bx, by): elements of block bx against the eight items from 8 by on, so a
+// thread has eight independent loads per element in flight and small systems
+// still spread over the basis.  The eight sums of a warp are reduced together
+// (each exchange halves what a lane keeps: 9 shuffles instead of 40).
+__global__ void __launch_bounds__(kGsThreads) k_gm_dots(GmresVecs G, int pass) {
     pdl_wait();
     pdl_release();
     if (G.sc->cycle_done) return;
     if (pass == 1 && !G.sc->reorth) return;  // uniform over the grid
     const int k = G.sc->k;
-    if (!in_range(k, G.sc->restart, GS_KRYLOV_K)) return;  // uniform over the grid: no block takes the ticket
-    const int m = pass == 0 ? k + 1 : k;                     // last item (k < restart <= kGmresMaxRestart)
-    const size_t n = G.n;
-    __shared__ double sh[kGmresMaxRestart + 1];
-    __shared__ double wsq;
-    __shared__ bool last;
-    const size_t per = (n + gridDim.x - 1) / gridDim.x;
-    const size_t r0 = (size_t)blockIdx.x * per, r1 = min(n, r0 + per);
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
-    for (int i = warp; i <= m; i += nwarp) {
-        const double *vi = i <= k ? G.V + (size_t)i * n : G.w;
-        double s = 0.0;
-        for (size_t q = r0 + lane; q < r1; q += 32) s += vi[q] * G.w[q];
+    if (!in_range(k, G.sc->restart, GS_KRYLOV_K)) return;
+    const int items = pass == 0 ? k + 2 : k + 1;  // k < restart <= kGmresMaxRestart
+    const int g = blockIdx.y * kGsGroup;
+    if (g >= items) return;
+    const int cnt = min(kGsGroup, items - g);
+    double a[kGsGroup];
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
-        if (lane == 0) sh[i] = s;
+    for (int v = 0; v < kGsGroup; ++v) a[v] = 0.0;
+    const bool full = g + kGsGroup <= k + 1;  // eight basis vectors
+    if (G.n & 1) {
+        if (full) gs_dots_body<false, kGsGroup>(G, g, cnt, k, a);
+        else gs_dots_body<false, 0>(G, g, cnt, k, a);
+    } else {
+        if (full) gs_dots_body<true, kGsGroup>(G, g, cnt, k, a);
+        else gs_dots_body<true, 0>(G, g, cnt, k, a);
     }
-    __syncthreads();
-    for (int i = threadIdx.x; i <= m; i += blockDim.x) G.partials[(size_t)blockIdx.x * (kGmresMaxRestart + 1) + i] = sh[i];
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        __threadfence();
-        last = (atomicAdd(&G.sc->ticket, 1u) == gridDim.x - 1);
-    }
-    __syncthreads();
-    if (!last) return;
-    __threadfence();
-    // one warp per basis vector: lanes take the block partials in a fixed
-    // stride, then a fixed shuffle tree (deterministic)
-    for (int i = warp; i <= m; i += nwarp) {
-        double s = 0.0;
-        for (int bb = lane; bb < (int)gridDim.x; bb += 32)
-            s += ((volatile double *)G.partials)[(size_t)bb * (kGmresMaxRestart + 1) + i];
+    __shared__ double sh[kGsThreads / 32][kGsGroup];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
-        if (lane == 0) {
-            if (i > k) wsq = s;
-            else if (pass == 0) G.sc->H[i][k] = s;
-            else G.sc->h2[i] = s;
+    for (int h = kGsGroup / 2, o = 16; h > 0; h >>= 1, o >>= 1) {
+        const bool up = lane & o;
+#pragma unroll
+        for (int j = 0; j < h; ++j) {
+            const double keep = up ? a[j + h] : a[j], send = up ? a[j] : a[j + h];
+            a[j] = keep + __shfl_xor_sync(0xffffffffu, send, o);
         }
     }
+    a[0] += __shfl_xor_sync(0xffffffffu, a[0], 2);
+    a[0] += __shfl_xor_sync(0xffffffffu, a[0], 1);
+    // lane bits 4, 3, 2 now select the item's bits 2, 1, 0
+    if ((lane & 3) == 0) sh[warp][(lane >> 4 & 1) * 4 + (lane >> 3 & 1) * 2 + (lane >> 2 & 1)] = a[0];
     __syncthreads();
-    if (threadIdx.x == 0) {
-        if (pass == 0) {
-            double rem = wsq;
-            for (int i = 0; i <= k; ++i) rem -= G.sc->H[i][k] * G.sc->H[i][k];
-            const int re = !(rem >= G.sc->gs_eta2 * wsq);  // also when rem or wsq is not finite
-            G.sc->reorth = re;
-            G.sc->reorths += re;
-        }
-        G.sc->ticket = 0u;
+    if (threadIdx.x < cnt) {
+        double s = 0.0;
+#pragma unroll
+        for (int w = 0; w < kGsThreads / 32; ++w) s += sh[w][threadIdx.x];
+        G.partials[(size_t)(g + threadIdx.x) * kGsBlocks + blockIdx.x] = s;
     }
 }
 
-// w -= V c (c = H[.][k] on pass 0, h2 on pass 1).  The pass that ends the
-// projection closes column k with ||w||, summed as it writes w: pass 0 when
-// k_gm_dots decided against a second pass (pass 1 then has nothing to do),
-// pass 1 otherwise.
-__global__ void k_gm_update(GmresVecs G, int pass) {
+// w -= V c (c = the first pass's h, or the second's correction), block partials of
+// ||w||^2.  SPLIT (small systems): a block takes 64 elements (32 for odd n) and
+// its warps every eighth basis vector each, so a column of 100 vectors is a
+// chain of 13 loads; otherwise a thread runs over the basis with eight loads in
+// flight.
+template <bool SPLIT, bool PAIR>
+__device__ __forceinline__ double gs_update_body(const GmresVecs &G, int k, const double *coef) {
+    const size_t n = G.n;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    constexpr int NW = kGsThreads / 32;
+    constexpr int E = PAIR ? 2 : 1;
+    double d = 0.0;
+    if (SPLIT) {
+        __shared__ double part[NW][64];
+        const size_t tiles = (n + 32 * E - 1) / (32 * E);
+        for (size_t t = blockIdx.x; t < tiles; t += gridDim.x) {
+            const size_t q = t * 32 * E + lane * E;
+            double s0 = 0.0, s1 = 0.0;
+            if (q < n) {
+#pragma unroll 8
+                for (int i = warp; i <= k; i += NW) {
+                    const double c = coef[i];
+                    if (PAIR) {
+                        const double2 v = *reinterpret_cast<const double2 *>(G.V + (size_t)i * n + q);
+                        s0 += c * v.x;
+                        s1 += c * v.y;
+                    } else {
+                        s0 += c * G.V[(size_t)i * n + q];
+                    }
+                }
+            }
+            part[warp][lane * E] = s0;
+            if (PAIR) part[warp][lane * E + 1] = s1;
+            __syncthreads();
+            const size_t p = t * 32 * E + threadIdx.x;
+            if (threadIdx.x < 32 * E && p < n) {
+                double s = 0.0;
+#pragma unroll
+                for (int w = 0; w < NW; ++w) s += part[w][threadIdx.x];
+                const double w = G.w[p] - s;
+                G.w[p] = w;
+                d += w * w;
+            }
+            __syncthreads();
+        }
+    } else {
+        const size_t nv = n / E, T = (size_t)gridDim.x * kGsThreads;
+#pragma unroll 2
+        for (size_t e = (size_t)blockIdx.x * kGsThreads + threadIdx.x; e < nv; e += T) {
+            if (PAIR) {
+                double2 w = reinterpret_cast<const double2 *>(G.w)[e];
+#pragma unroll 8
+                for (int i = 0; i <= k; ++i) {
+                    const double2 v = reinterpret_cast<const double2 *>(G.V + (size_t)i * n)[e];
+                    w.x -= coef[i] * v.x;
+                    w.y -= coef[i] * v.y;
+                }
+                reinterpret_cast<double2 *>(G.w)[e] = w;
+                d += w.x * w.x + w.y * w.y;
+            } else {
+                double w = G.w[e];
+#pragma unroll 8
+                for (int i = 0; i <= k; ++i) w -= coef[i] * G.V[(size_t)i * n + e];
+                G.w[e] = w;
+                d += w * w;
+            }
+        }
+    }
+    return d;
+}
+
+__global__ void __launch_bounds__(kGsThreads) k_gm_update(GmresVecs G, int pass) {
     pdl_wait();
     pdl_release();
-    if (G.sc->cycle_done) return;
     GScalars *sc = G.sc;
-    const bool second = sc->reorth;  // set by k_gm_dots pass 0; uniform over the grid
-    if (pass == 1 && !second) return;  // before reading k: pass 0 has advanced it
+    if (sc->cycle_done) return;
+    if (pass == 1 && !sc->reorth) return;  // uniform over the grid
     const int k = sc->k;
     if (!in_range(k, sc->restart, GS_KRYLOV_K)) return;  // uniform over the grid
-    const size_t n = G.n;
-    __shared__ double coef[kGmresMaxRestart + 1];
-    for (int i = threadIdx.x; i <= k; i += blockDim.x) coef[i] = pass == 0 ? sc->H[i][k] : sc->h2[i];
-    __syncthreads();
-    double d[1] = {0.0};
-    for (size_t q = (size_t)blockIdx.x * blockDim.x + threadIdx.x; q < n; q += (size_t)gridDim.x * blockDim.x) {
-        double w = G.w[q];
-        for (int i = 0; i <= k; ++i) w -= coef[i] * G.V[(size_t)i * n + q];
-        G.w[q] = w;
-        d[0] += w * w;
+    __shared__ double coef[kGsItems + 1];
+    __shared__ double red[kGsThreads / 32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int items = pass == 0 ? k + 2 : k + 1, nb = gs_dots_blocks(G.n);
+    for (int i = warp; i < items; i += kGsThreads / 32) {
+        double s = 0.0;
+#pragma unroll 5
+        for (int b = lane; b < nb; b += 32) s += G.partials[(size_t)i * kGsBlocks + b];
+        s = warp_sum(s);
+        if (lane == 0) coef[i] = s;
     }
-    if (pass == 0 && second) return;  // pass 1 closes the column
-    if (grid_reduce<1>(d, G.partials, &sc->ticket) && threadIdx.x == 0) {
-        if (pass == 1)
-            for (int i = 0; i <= k; ++i) sc->H[i][k] += sc->h2[i];
-        const double hn = ::sqrt(d[0]);
-        sc->wnorm = hn;
-        sc->H[k + 1][k] = hn;
-        for (int i = 0; i < k; ++i) {  // previous rotations
-            const double a = sc->H[i][k], b2 = sc->H[i + 1][k];
-            sc->H[i][k] = sc->cs[i] * a + sc->sn[i] * b2;
-            sc->H[i + 1][k] = -sc->sn[i] * a + sc->cs[i] * b2;
+    __syncthreads();
+    if (blockIdx.x == 0 && warp == 0) {
+        if (pass == 0) {
+            double q = 0.0;
+            for (int i = lane; i <= k; i += 32) {
+                sc->H[i][k] = coef[i];
+                q += coef[i] * coef[i];
+            }
+            q = warp_sum(q);
+            if (lane == 0) {
+                const double wsq = coef[k + 1];
+                const int re = !(wsq - q >= sc->gs_eta2 * wsq);  // also when not finite
+                sc->reorth = re;
+                sc->reorths += re;
+                sc->kn = k + 1;
+            }
+        } else {
+            for (int i = lane; i <= k; i += 32) sc->H[i][k] += coef[i];
         }
-        const double a = sc->H[k][k], b2 = sc->H[k + 1][k];
-        const double rr = ::sqrt(a * a + b2 * b2);
-        double c = 1.0, s = 0.0;
-        if (rr > 0.0) { c = a / rr; s = b2 / rr; }
-        sc->cs[k] = c;
-        sc->sn[k] = s;
-        sc->H[k][k] = rr;
-        sc->H[k + 1][k] = 0.0;
-        sc->g[k + 1] = -s * sc->g[k];
-        sc->g[k] = c * sc->g[k];
-        sc->resid = fabs(sc->g[k + 1]);
-        sc->iters += 1;
-        sc->k = k + 1;
-        if (!isfinite(sc->resid)) { sc->status = ST_NAN; sc->cycle_done = 1; sc->done = 1; return; }
-        if (sc->resid <= sc->tol || hn == 0.0 || k + 1 >= sc->restart || sc->iters >= sc->max_iter) sc->cycle_done = 1;
+    }
+    const bool split = G.n <= (size_t)kGsSplitMax, odd = G.n & 1;
+    double d;
+    if (split) d = odd ? gs_update_body<true, false>(G, k, coef) : gs_update_body<true, true>(G, k, coef);
+    else d = odd ? gs_update_body<false, false>(G, k, coef) : gs_update_body<false, true>(G, k, coef);
+    d = warp_sum(d);
+    if (lane == 0) red[warp] = d;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        double s = 0.0;
+#pragma unroll
+        for (int w = 0; w < kGsThreads / 32; ++w) s += red[w];
+        G.partials[(size_t)kGsItems * kGsBlocks + blockIdx.x] = s;
     }
 }
 
-// end of a cycle: y = H^{-1} g by back substitution (one thread)
+// Closes column k with ||w|| = hn (one warp): rotations of the earlier columns,
+// the new one, residual estimate and flags.
+__device__ __forceinline__ void gs_close(GScalars *sc, int k, double hn) {
+    __shared__ double h[kGmresMaxRestart + 1], cs[kGmresMaxRestart], sn[kGmresMaxRestart];
+    const int lane = threadIdx.x & 31;
+    for (int i = lane; i <= k; i += 32) {
+        h[i] = sc->H[i][k];
+        if (i < k) { cs[i] = sc->cs[i]; sn[i] = sc->sn[i]; }
+    }
+    __syncwarp();
+    if (lane == 0) {
+        double a = h[0];
+        for (int i = 0; i < k; ++i) {  // previous rotations
+            const double b2 = h[i + 1];
+            h[i] = cs[i] * a + sn[i] * b2;
+            a = -sn[i] * a + cs[i] * b2;
+        }
+        const double rr = ::sqrt(a * a + hn * hn);
+        double c = 1.0, s = 0.0;
+        if (rr > 0.0) { c = a / rr; s = hn / rr; }
+        h[k] = rr;
+        const double gk = sc->g[k], next = -s * gk;
+        sc->wnorm = hn;
+        sc->cs[k] = c;
+        sc->sn[k] = s;
+        sc->H[k + 1][k] = 0.0;
+        sc->g[k + 1] = next;
+        sc->g[k] = c * gk;
+        sc->resid = fabs(next);
+        const int it = sc->iters + 1;
+        sc->iters = it;
+        sc->k = k + 1;
+        if (!isfinite(next)) { sc->status = ST_NAN; sc->cycle_done = 1; sc->done = 1; }
+        else if (fabs(next) <= sc->tol || hn == 0.0 || k + 1 >= sc->restart || it >= sc->max_iter) sc->cycle_done = 1;
+    }
+    __syncwarp();
+    for (int i = lane; i <= k; i += 32) sc->H[i][k] = h[i];
+}
+
+// v_{k+1} = w / ||w|| (v_0 = w / beta at a cycle start) -> V, and
+//   zout = scale Minv v   (node-block preconditioner, or a smoother's zero-start sweep), or
+//   zout = v              (Minv nullptr: a V-cycle's right-hand side), or nothing (zout nullptr).
+// Block 0 closes the column (one warp; not at a start) while the others work:
+// they read kn, which the close leaves alone, and a
+// cycle_done that appears under them only spares them a vector no one reads.
+template <int NF>
+__global__ void __launch_bounds__(kGsThreads) k_gm_next(int n_rows, GmresVecs G, int start, const double *Minv,
+                                                        double *zout, double scale) {
+    GScalars *sc = G.sc;
+    const int r = ((int)blockIdx.x - 1) * kGsThreads + threadIdx.x;
+    const bool own = blockIdx.x > 0 && r < n_rows;
+    double M[NF * NF];  // written before this solve's Arnoldi steps: loaded ahead of the wait
+    if (Minv && own)
+#pragma unroll
+        for (int i = 0; i < NF * NF; ++i) M[i] = __ldg(Minv + (size_t)r * NF * NF + i);
+    pdl_wait();
+    pdl_release();
+    double v[NF];
+    if (own) load_rw<NF>(G.w + (size_t)r * NF, v);
+    if (sc->cycle_done) return;
+    const int kn = sc->kn;
+    if (!in_range(kn, sc->restart + 1, GS_KRYLOV_K)) return;  // V holds restart + 1 vectors
+    double hn;
+    __shared__ double red[kGsThreads / 32];
+    if (start) {
+        hn = sc->beta;
+    } else {
+        const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nb = gs_update_blocks(G.n);
+        double s = 0.0;
+        for (int b = threadIdx.x; b < nb; b += kGsThreads) s += G.partials[(size_t)kGsItems * kGsBlocks + b];
+        s = warp_sum(s);
+        if (lane == 0) red[warp] = s;
+        __syncthreads();
+        s = 0.0;
+#pragma unroll
+        for (int w = 0; w < kGsThreads / 32; ++w) s += red[w];
+        hn = ::sqrt(s);
+    }
+    if (blockIdx.x == 0) {
+        if (!start && threadIdx.x < 32) gs_close(sc, kn - 1, hn);
+        return;
+    }
+    if (!own) return;
+    const double ih = 1.0 / hn;
+#pragma unroll
+    for (int f = 0; f < NF; ++f) v[f] *= ih;
+    store_rw<NF>(G.V + (size_t)kn * G.n + (size_t)r * NF, v);
+    if (!zout) return;
+    if (Minv) {
+        double z[NF];
+#pragma unroll
+        for (int i = 0; i < NF; ++i) {
+            double t = 0.0;
+#pragma unroll
+            for (int j = 0; j < NF; ++j) t += M[i * NF + j] * v[j];
+            z[i] = scale * t;
+        }
+        store_rw<NF>(zout + (size_t)r * NF, z);
+    } else {
+        store_rw<NF>(zout + (size_t)r * NF, v);
+    }
+}
+
+// End of a cycle: y = H^{-1} g by back substitution, one warp, by columns: a
+// lane keeps the right-hand sides of rows lane, lane + 32, ... and the loads of
+// the next column do not wait for this one's y.
 __global__ void k_gm_solve_y(GScalars *sc) {
-    if (threadIdx.x != 0 || blockIdx.x != 0 || sc->done) return;
-    const int k = sc->k;
+    if (sc->done) return;
+    const int k = sc->k, lane = threadIdx.x;
     if (!in_range(k, sc->restart + 1, GS_KRYLOV_K)) return;
+    constexpr int R = kGmresMaxRestart / 32;
+    double g[R], h[R];
+#pragma unroll
+    for (int q = 0; q < R; ++q) {
+        const int r = lane + 32 * q;
+        g[q] = r < k ? sc->g[r] : 0.0;
+        h[q] = r < k ? sc->H[r][k - 1] : 0.0;
+    }
     for (int i = k - 1; i >= 0; --i) {
-        double s = sc->g[i];
-        for (int q = i + 1; q < k; ++q) s -= sc->H[i][q] * sc->y[q];
-        sc->y[i] = (sc->H[i][i] != 0.0) ? s / sc->H[i][i] : 0.0;
+        double hn[R];
+#pragma unroll
+        for (int q = 0; q < R; ++q) hn[q] = (i > 0 && lane + 32 * q < i) ? sc->H[lane + 32 * q][i - 1] : 0.0;
+        double gi = 0.0, hi = 0.0;
+#pragma unroll
+        for (int q = 0; q < R; ++q)
+            if (i >> 5 == q) { gi = g[q]; hi = h[q]; }
+        gi = __shfl_sync(0xffffffffu, gi, i & 31);
+        hi = __shfl_sync(0xffffffffu, hi, i & 31);
+        const double y = hi != 0.0 ? gi / hi : 0.0;
+        if (lane == 0) sc->y[i] = y;
+#pragma unroll
+        for (int q = 0; q < R; ++q) {
+            g[q] -= h[q] * y;
+            h[q] = hn[q];
+        }
     }
 }
 

@@ -770,20 +770,6 @@ __global__ void k_mg_dense_apply(const double *__restrict__ Inv, const double *_
 }
 
 // ---------------------------------------------------------------- flexible GMRES glue
-// v_k = w / s -> V[k] and the cycle's right-hand side
-__global__ void k_gm_next_flex(size_t n, GmresVecs G, int start, double *__restrict__ mg_b) {
-    if (G.sc->cycle_done) return;
-    const int k = G.sc->k;
-    if (!in_range(k, G.sc->restart + 1, GS_KRYLOV_K)) return;  // V holds restart + 1 vectors
-    const double ih = 1.0 / (start ? G.sc->beta : G.sc->wnorm);
-    double *vn = G.V + (size_t)k * G.n;
-    for (size_t q = (size_t)blockIdx.x * blockDim.x + threadIdx.x; q < n; q += (size_t)gridDim.x * blockDim.x) {
-        const double v = G.w[q] * ih;
-        vn[q] = v;
-        mg_b[q] = v;
-    }
-}
-
 // w = A z_k, and z_k -> Z[k] (z is the V-cycle's output)
 template <int NF, typename VT>
 __global__ void k_gm_spmv_keep(PtrsA A, GmresVecs G, double *__restrict__ Z) {

@@ -78,31 +78,6 @@ __device__ __forceinline__ void unit_get(const uint2 &v, double *o) {
 }
 template <typename T> __device__ __forceinline__ T sell_ld(const T *p) { return __ldg(p); }
 
-// vector of one row, through the ordinary (coherent) path
-template <int NF>
-__device__ __forceinline__ void vec_ld(const double *p, double out[NF]) {
-    if constexpr (NF == 2 || NF == 4) {
-#pragma unroll
-        for (int q = 0; q < NF / 2; ++q) {
-            const double2 v = reinterpret_cast<const double2 *>(p)[q];
-            out[2 * q] = v.x; out[2 * q + 1] = v.y;
-        }
-    } else {
-#pragma unroll
-        for (int g = 0; g < NF; ++g) out[g] = p[g];
-    }
-}
-template <int NF>
-__device__ __forceinline__ void vec_st(double *p, const double v[NF]) {
-    if constexpr (NF == 2 || NF == 4) {
-#pragma unroll
-        for (int q = 0; q < NF / 2; ++q) reinterpret_cast<double2 *>(p)[q] = make_double2(v[2 * q], v[2 * q + 1]);
-    } else {
-#pragma unroll
-        for (int g = 0; g < NF; ++g) p[g] = v[g];
-    }
-}
-
 // The columns and values of a chunk's first PF trips in registers, the rest
 // streamed; PF keeps the prefetched values within about 72 registers.
 template <int NF, typename VT, int LPR>
@@ -133,7 +108,7 @@ struct SellRow {
         double b[NF * NF], xv[NF];
 #pragma unroll
         for (int u = 0; u < NU; ++u) unit_get(v[u], b + u * (NF * NF / NU));
-        vec_ld<NF>(x, xv);
+        load_rw<NF>(x, xv);
 #pragma unroll
         for (int f = 0; f < NF; ++f)
 #pragma unroll
@@ -259,8 +234,48 @@ __global__ void k_sell_values(SellJobs js) {
 struct VecRef {
     double *p;
     size_t stride;
-    __device__ __forceinline__ double *at(int k) const { return p + (size_t)k * stride; }
+    // a fixed buffer's address does not wait for k
+    __device__ __forceinline__ double *at(int k) const { return stride ? p + (size_t)k * stride : p; }
 };
+
+// Whether this step's kernel has work: the state is read here, and on small
+// levels (LPR > 1) tested only before the stores, so that the vector loads do not
+// wait for it (a step queued past convergence computes on stale vectors and
+// stores nothing); on large ones such a step must not move the matrix.
+struct StepState {
+    int k;
+    bool off;
+};
+__device__ __forceinline__ StepState step_state(const GScalars *sc) {
+    StepState st;
+    st.k = sc->k;
+    st.off = sc->cycle_done || (unsigned)st.k >= (unsigned)sc->restart;  // Z holds restart vectors
+    if (st.off) st.k = 0;
+    return st;
+}
+// one row's smoother block
+template <int NF>
+__device__ __forceinline__ void minv_ld(const double *Minv, int r, double M[NF * NF]) {
+    if constexpr (NF == 2 || NF == 4) {
+#pragma unroll
+        for (int q = 0; q < NF * NF / 2; ++q) {
+            const double2 v = __ldg(reinterpret_cast<const double2 *>(Minv + (size_t)r * NF * NF) + q);
+            M[2 * q] = v.x; M[2 * q + 1] = v.y;
+        }
+    } else {
+#pragma unroll
+        for (int i = 0; i < NF * NF; ++i) M[i] = __ldg(Minv + (size_t)r * NF * NF + i);
+    }
+}
+template <int NF>
+__device__ __forceinline__ void minv_mul(const double M[NF * NF], const double v[NF], double z[NF]) {
+#pragma unroll
+    for (int i = 0; i < NF; ++i) {
+        z[i] = 0.0;
+#pragma unroll
+        for (int j = 0; j < NF; ++j) z[i] += M[i * NF + j] * v[j];
+    }
+}
 
 // x_out = x_in + omega Minv (b - A x_in)
 template <int NF, typename VT, int LPR>
@@ -270,31 +285,39 @@ __global__ void __launch_bounds__(256) k_sell_jacobi(SellA A, const double *Minv
     const int nw = gridDim.x * (blockDim.x >> 5);
     int c = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     SellRow<NF, VT, LPR> row;
-    if (c < A.n_chunks) row.load(A, c, lane);
+    double M[NF * NF];
+    auto fetch = [&]() {
+        row.load(A, c, lane);
+        const int r = c * (32 / LPR) + lane / LPR;
+        if (r < A.n_rows && sub == 0) minv_ld<NF>(Minv, r, M);
+    };
+    if (c < A.n_chunks) fetch();
     pdl_wait();
     pdl_release();
-    if (sc->cycle_done || !in_range(sc->k, sc->restart, GS_KRYLOV_K)) return;
-    const double *bp = b.at(sc->k);
-    double *xo = x_out.at(sc->k);
+    const StepState st = step_state(sc);
+    if (LPR == 1 && st.off) return;
+    const double *bp = b.at(st.k);
+    double *xo = x_out.at(st.k);
     while (c < A.n_chunks) {
         const int r = c * (32 / LPR) + lane / LPR;
         const bool own = r < A.n_rows && sub == 0;
         double t[NF], z[NF], xi[NF], acc[NF];
         if (own) {
-            vec_ld<NF>(bp + (size_t)r * NF, t);
-            vec_ld<NF>(x_in + (size_t)r * NF, xi);
+            load_rw<NF>(bp + (size_t)r * NF, t);
+            load_rw<NF>(x_in + (size_t)r * NF, xi);
         }
         row.mul(A, c, lane, x_in, acc);
+        if (LPR > 1 && st.off) return;
         if (own) {
 #pragma unroll
             for (int f = 0; f < NF; ++f) t[f] -= acc[f];
-            apply_minv<NF>(Minv, r, t, z);
+            minv_mul<NF>(M, t, z);
 #pragma unroll
             for (int f = 0; f < NF; ++f) z[f] = xi[f] + omega * z[f];
-            vec_st<NF>(xo + (size_t)r * NF, z);
+            store_rw<NF>(xo + (size_t)r * NF, z);
         }
         c += nw;
-        if (c < A.n_chunks) row.load(A, c, lane);
+        if (c < A.n_chunks) fetch();
     }
 }
 
@@ -309,18 +332,20 @@ __global__ void __launch_bounds__(256) k_sell_residual(SellA A, VecRef b, const 
     if (c < A.n_chunks) row.load(A, c, lane);
     pdl_wait();
     pdl_release();
-    if (sc->cycle_done || !in_range(sc->k, sc->restart, GS_KRYLOV_K)) return;
-    const double *bp = b.at(sc->k);
+    const StepState st = step_state(sc);
+    if (LPR == 1 && st.off) return;
+    const double *bp = b.at(st.k);
     while (c < A.n_chunks) {
         const int r = c * (32 / LPR) + lane / LPR;
         const bool own = r < A.n_rows && sub == 0;
         double t[NF], acc[NF];
-        if (own) vec_ld<NF>(bp + (size_t)r * NF, t);
+        if (own) load_rw<NF>(bp + (size_t)r * NF, t);
         row.mul(A, c, lane, x, acc);
+        if (LPR > 1 && st.off) return;
         if (own) {
 #pragma unroll
             for (int f = 0; f < NF; ++f) t[f] -= acc[f];
-            vec_st<NF>(r_out + (size_t)r * NF, t);
+            store_rw<NF>(r_out + (size_t)r * NF, t);
         }
         c += nw;
         if (c < A.n_chunks) row.load(A, c, lane);
@@ -337,41 +362,16 @@ __global__ void __launch_bounds__(256) k_sell_spmv(SellA A, VecRef z, double *w,
     if (c < A.n_chunks) row.load(A, c, lane);
     pdl_wait();
     pdl_release();
-    if (sc->cycle_done || !in_range(sc->k, sc->restart, GS_KRYLOV_K)) return;  // Z holds restart vectors
-    const double *zp = z.at(sc->k);
+    const StepState st = step_state(sc);
+    if (st.off) return;
+    const double *zp = z.at(st.k);
     while (c < A.n_chunks) {
         const int r = c * (32 / LPR) + lane / LPR;
         double acc[NF];
         row.mul(A, c, lane, zp, acc);
-        if (r < A.n_rows && sub == 0) vec_st<NF>(w + (size_t)r * NF, acc);
+        if (r < A.n_rows && sub == 0) store_rw<NF>(w + (size_t)r * NF, acc);
         c += nw;
         if (c < A.n_chunks) row.load(A, c, lane);
-    }
-}
-
-// v_k = w / s -> V[k], and the finest level's zero-start sweep x_1 = omega Minv v_k
-// (Minv nullptr: V[k] only)
-template <int NF>
-__global__ void k_gm_next_smooth(int n_rows, GmresVecs G, int start, const double *Minv, double *x1, double omega) {
-    pdl_wait();
-    pdl_release();
-    const GScalars *sc = G.sc;
-    if (sc->cycle_done) return;
-    const int k = sc->k;
-    if (!in_range(k, sc->restart + 1, GS_KRYLOV_K)) return;  // V holds restart + 1 vectors
-    const double ih = 1.0 / (start ? sc->beta : sc->wnorm);
-    double *vn = G.V + (size_t)k * G.n;
-    for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < n_rows; r += gridDim.x * blockDim.x) {
-        double v[NF], z[NF];
-        vec_ld<NF>(G.w + (size_t)r * NF, v);
-#pragma unroll
-        for (int f = 0; f < NF; ++f) v[f] *= ih;
-        vec_st<NF>(vn + (size_t)r * NF, v);
-        if (!Minv) continue;
-        apply_minv<NF>(Minv, r, v, z);
-#pragma unroll
-        for (int f = 0; f < NF; ++f) z[f] *= omega;
-        vec_st<NF>(x1 + (size_t)r * NF, z);
     }
 }
 
@@ -392,13 +392,12 @@ __global__ void k_sell_restrict(int nc, int nf_rows, const int *child, const uin
             if (fr[q] >= 0 && !in_range(fr[q], nf_rows, GS_RESTRICT)) fr[q] = -1;
             fx[q] = fr[q] >= 0 ? __ldg(ffixed + fr[q]) : 0;
         }
-        if (Minv)
-#pragma unroll
-            for (int i = 0; i < NF * NF; ++i) M[i] = __ldg(Minv + (size_t)R * NF * NF + i);
+        if (Minv) minv_ld<NF>(Minv, R, M);
     }
     pdl_wait();
     pdl_release();
-    if (R >= nc || sc->cycle_done) return;
+    if (R >= nc) return;
+    const bool off = sc->cycle_done;  // tested before the stores: the loads do not wait for it
     double acc[NF];
 #pragma unroll
     for (int f = 0; f < NF; ++f) acc[f] = 0.0;
@@ -407,37 +406,34 @@ __global__ void k_sell_restrict(int nc, int nf_rows, const int *child, const uin
         if (fr[q] < 0) continue;
         const double w = (q % 3 == 1 ? 1.0 : 0.5) * (q / 3 == 1 ? 1.0 : 0.5);
         double v[NF];
-        vec_ld<NF>(rf + (size_t)fr[q] * NF, v);
+        load_rw<NF>(rf + (size_t)fr[q] * NF, v);
 #pragma unroll
         for (int f = 0; f < NF; ++f)
             if (!((fx[q] >> f) & 1)) acc[f] += w * v[f];
     }
-    vec_st<NF>(bc + (size_t)R * NF, acc);
+    if (off) return;
+    store_rw<NF>(bc + (size_t)R * NF, acc);
     if (!Minv) return;
     double z[NF];
+    minv_mul<NF>(M, acc, z);
 #pragma unroll
-    for (int i = 0; i < NF; ++i) {
-        z[i] = 0.0;
-#pragma unroll
-        for (int j = 0; j < NF; ++j) z[i] += M[i * NF + j] * acc[j];
-        z[i] *= omega;
-    }
-    vec_st<NF>(x1 + (size_t)R * NF, z);
+    for (int f = 0; f < NF; ++f) z[f] *= omega;
+    store_rw<NF>(x1 + (size_t)R * NF, z);
 }
 
 // x = Inv b on the dense level (one warp per row)
 __global__ void k_sell_dense_apply(const double *Inv, VecRef b, VecRef x, int n, const GScalars *sc) {
     pdl_wait();
     pdl_release();
-    if (sc->cycle_done || !in_range(sc->k, sc->restart, GS_KRYLOV_K)) return;
-    const double *bp = b.at(sc->k);
-    double *xp = x.at(sc->k);
+    const StepState st = step_state(sc);
+    const double *bp = b.at(st.k);
+    double *xp = x.at(st.k);
     const int nw = gridDim.x * (blockDim.x >> 5), lane = threadIdx.x & 31;
     for (int i = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); i < n; i += nw) {
         double s = 0.0;
         for (int j = lane; j < n; j += 32) s += Inv[(size_t)i * n + j] * bp[j];
         for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
-        if (lane == 0) xp[i] = s;
+        if (lane == 0 && !st.off) xp[i] = s;
     }
 }
 
@@ -455,27 +451,29 @@ __global__ void k_sell_prolong(int n_rows, int nc, const int *parent, const uint
     }
     pdl_wait();
     pdl_release();
-    if (r >= n_rows || sc->cycle_done) return;
+    if (r >= n_rows) return;
+    const bool off = sc->cycle_done;  // tested before the store: the loads do not wait for it
     int cnt = 0;
 #pragma unroll
     for (int q = 0; q < 4; ++q) cnt += R[q] != -2;
     const double w = cnt == 1 ? 1.0 : (cnt == 2 ? 0.5 : 0.25);
     double acc[NF], x[NF];
-    vec_ld<NF>(xf + (size_t)r * NF, x);
+    load_rw<NF>(xf + (size_t)r * NF, x);
 #pragma unroll
     for (int f = 0; f < NF; ++f) acc[f] = 0.0;
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
         if (R[q] < 0 || !in_range(R[q], nc, GS_PROLONG)) continue;
         double v[NF];
-        vec_ld<NF>(xc + (size_t)R[q] * NF, v);
+        load_rw<NF>(xc + (size_t)R[q] * NF, v);
 #pragma unroll
         for (int f = 0; f < NF; ++f) acc[f] += w * v[f];
     }
 #pragma unroll
     for (int f = 0; f < NF; ++f)
         if (!((fx >> f) & 1)) x[f] += acc[f];
-    vec_st<NF>(xf + (size_t)r * NF, x);
+    if (off) return;
+    store_rw<NF>(xf + (size_t)r * NF, x);
 }
 
 }  // namespace

@@ -341,10 +341,11 @@ int gw_bsr_gmres_solve(const gw_bsr_t *A, int32_t prec, int32_t precond, const d
  * lags.  The caller must have run one solve with lag = 0 on this plan and
  * workspace first.  A plan is accepted only for the pattern it was built from:
  * the same workspace, row count, block count and row_ptr / cols arrays
- * (GW_EINVAL otherwise).  The solve writes its iteration count to
- * plan_host->last_iters: the next solve with the plan queues that many
- * Arnoldi steps before its first host check (a caller that rebuilds the plan
- * may carry the value over). */
+ * (GW_EINVAL otherwise).  The solve writes its iteration count
+ * and convergence rate to plan_host->last_iters and last_rate: the next solve
+ * with the plan queues nine tenths of the Arnoldi steps that the rate predicts
+ * before its first host check (a caller that rebuilds the plan may carry the
+ * values over). */
 #define GW_MG_MAX_LEVELS 20
 typedef struct gw_mg_plan {
     int32_t levels;                     /* levels holding a matrix; the last one is solved densely */
@@ -356,7 +357,7 @@ typedef struct gw_mg_plan {
     const void *workspace;              /* the coarse patterns live in this workspace              */
     const void *row_ptr, *cols;         /* pattern arrays of the matrix the plan was built from    */
     int32_t last_iters;                 /* iterations of the last solve with this plan (0: none)    */
-    int32_t pad0;
+    int32_t last_rate;                  /* 1000 ln(|b| / |r|) per iteration of it (0: none)         */
 } gw_mg_plan_t;
 int64_t gw_gmres_mg_workspace_bytes(const gw_grid_t *grid, int32_t n_rows, int32_t nf, int32_t restart);
 int gw_mg_plan_build(const gw_grid_t *grid, const gw_bsr_t *A, void *workspace, int64_t workspace_bytes,
