@@ -303,8 +303,15 @@ extern "C" int gw_return_map(const gw_material_t *mat, int32_t n, const double *
     MatConst mc = make_matconst(*mat);
     const double nu = mat->poisson_ratio, E = mat->youngs_modulus;
     const double lam = E * nu / ((1.0 + nu) * (1.0 - 2.0 * nu)), mu = E / (2.0 * (1.0 + nu));
-    k_return_map<<<gw_count_launch(nblk(n, kThreads)), kThreads, 0, S(stream)>>>(mc, lam, mu, n, e_trial, eps_v_total, pi_old, pi_new,
-                                                                e_out, tau_out, dtau_de_out);
+    auto k = k_return_map<GW_MODEL_HENCKY>;
+    switch (mc.model) {
+        case GW_MODEL_J2: k = k_return_map<GW_MODEL_J2>; break;
+        case GW_MODEL_DP: k = k_return_map<GW_MODEL_DP>; break;
+        case GW_MODEL_NORSAND: k = k_return_map<GW_MODEL_NORSAND>; break;
+        default: break;  // the elastic models return the trial state
+    }
+    k<<<gw_count_launch(nblk(n, 128)), 128, 0, S(stream)>>>(mc, lam, mu, n, e_trial, eps_v_total, pi_old, pi_new, e_out,
+                                                            tau_out, dtau_de_out);
     GW_LAUNCHED();
     return GW_OK;
 }

@@ -32,11 +32,13 @@ GW_HD R sq(R x) { return x * x; }
 // Value plus N directional derivatives.  Used to differentiate the fixed-count
 // local Newton iterations of the return maps exactly (the quantity Warp's tape
 // differentiates in the reference) and to get the algorithmic tangent
-// d tau_A / d e_trial_B.
+// d tau_A / d e_trial_B.  N = 0 carries the value alone through the same
+// operations (a quotient by a scalar is a product with its reciprocal), so a
+// value-only pass takes the decisions of the differentiated one.
 template <int N, typename R>
 struct Dual {
     R v;
-    R d[N];
+    R d[N > 0 ? N : 1];
     GW_HD Dual() : v(0) {
 #pragma unroll
         for (int i = 0; i < N; ++i) d[i] = 0;
@@ -143,33 +145,57 @@ template <int N, typename R> GW_HD Dual<N, R> gpow(const Dual<N, R> &a, R p) {
 }
 
 // ---------------------------------------------------------------- generic small linear algebra
-// Solve the 4x4 system M x = b by Gaussian elimination with partial pivoting
-// on the value part; works for any scalar type with +,-,*,/.
-template <typename T>
-GW_HD void solve4(T M[4][4], T b[4], T x[4]) {
+// Solve M X = B (4 x 4, NR right-hand sides, in place) by Gaussian elimination
+// with partial pivoting on the value part; any scalar type with +,-,*,/.  Rows
+// are exchanged by compare-and-swap at fixed indices, so the arrays stay in
+// registers.
+template <int NR, typename T>
+GW_HD void solve4n(T M[4][4], T B[4][NR]) {
 #pragma unroll
     for (int c = 0; c < 4; ++c) {
         int piv = c;
         auto best = fabs(val(M[c][c]));
+#pragma unroll
         for (int r = c + 1; r < 4; ++r) {
             auto a = fabs(val(M[r][c]));
             if (a > best) { best = a; piv = r; }
         }
-        if (piv != c) {
-            for (int k = 0; k < 4; ++k) { T t = M[c][k]; M[c][k] = M[piv][k]; M[piv][k] = t; }
-            T t = b[c]; b[c] = b[piv]; b[piv] = t;
+#pragma unroll
+        for (int r = c + 1; r < 4; ++r) {
+            if (piv == r) {
+#pragma unroll
+                for (int k = c; k < 4; ++k) { T t = M[c][k]; M[c][k] = M[r][k]; M[r][k] = t; }
+#pragma unroll
+                for (int k = 0; k < NR; ++k) { T t = B[c][k]; B[c][k] = B[r][k]; B[r][k] = t; }
+            }
         }
+#pragma unroll
         for (int r = c + 1; r < 4; ++r) {
             T f = M[r][c] / M[c][c];
-            for (int k = c; k < 4; ++k) M[r][k] = M[r][k] - f * M[c][k];
-            b[r] = b[r] - f * b[c];
+#pragma unroll
+            for (int k = c + 1; k < 4; ++k) M[r][k] = M[r][k] - f * M[c][k];
+#pragma unroll
+            for (int k = 0; k < NR; ++k) B[r][k] = B[r][k] - f * B[c][k];
         }
     }
-    for (int r = 3; r >= 0; --r) {
-        T s = b[r];
-        for (int k = r + 1; k < 4; ++k) s = s - M[r][k] * x[k];
-        x[r] = s / M[r][r];
-    }
+#pragma unroll
+    for (int r = 3; r >= 0; --r)
+#pragma unroll
+        for (int q = 0; q < NR; ++q) {
+            T s = B[r][q];
+#pragma unroll
+            for (int k = r + 1; k < 4; ++k) s = s - M[r][k] * B[k][q];
+            B[r][q] = s / M[r][r];
+        }
+}
+template <typename T>
+GW_HD void solve4(T M[4][4], T b[4], T x[4]) {
+    T B[4][1];
+#pragma unroll
+    for (int r = 0; r < 4; ++r) B[r][0] = b[r];
+    solve4n<1, T>(M, B);
+#pragma unroll
+    for (int r = 0; r < 4; ++r) x[r] = B[r][0];
 }
 
 template <typename R>

@@ -7,6 +7,8 @@
 //   Drucker-Prager     problems/material_tests/triaxial_DruckerPrager.py:119-412
 //   NorSand            problems/material_tests/triaxial_NorSand.py:155-400
 #pragma once
+#include <type_traits>
+
 #include "gw_math.cuh"
 #include "../../include/geowarp_b200.h"
 
@@ -120,21 +122,80 @@ GW_HD void dp_invariants(const T e[3], LT lam, LT mu, T tau[3], T &P, T S[3], T 
     Q = gsqrt(S[0] * S[0] + S[1] * S[1] + S[2] * S[2]) * R(1.224744871391589);
 }
 
+// residual of the local problem at (e, dl): e - e_trial + dl grad g, and the yield function
+template <typename T, typename R>
+GW_HD void dp_residual(const T etr[3], const MatConst &c, const T tau[3], const T &P, const T &Q, const T e[3],
+                       const T &dl, T gg[3], T rhs[4]) {
+    dp_grad(tau, Q, R(c.A_psi), R(c.B_psi), R(c.sf), gg);
+#pragma unroll
+    for (int i = 0; i < 3; ++i) rhs[i] = e[i] - etr[i] + dl * gg[i];
+    rhs[3] = dp_yield(P, Q, R(c.A_phi), R(c.B_phi), R(c.sf));
+}
+// its Jacobian in (e, dl)
+template <typename T, typename R, typename LT>
+GW_HD void dp_jacobian(LT lam, LT mu, const MatConst &c, const T tau[3], const T S[3], const T &Q, const T &dl,
+                       const T gg[3], T M[4][4]) {
+    const LT a_d = lam + 2.0 * mu, a_o = lam;  // elastic_a = lam 1 1^T + 2 mu I
+    T gf[3], hg[3][3];
+    dp_grad(tau, Q, R(c.A_phi), R(c.B_phi), R(c.sf), gf);
+    dp_hess(S, Q, R(c.A_psi), R(c.sf), hg);
+    // (hess_g @ a)_ij = sum_k hg_ik a_kj ;  grad_f_eps_j = sum_i gf_i a_ij
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+#pragma unroll
+        for (int j = 0; j < 3; ++j) {
+            T hge = hg[i][0] * (j == 0 ? a_d : a_o) + hg[i][1] * (j == 1 ? a_d : a_o) + hg[i][2] * (j == 2 ? a_d : a_o);
+            M[i][j] = (i == j ? T(R(1)) : T(R(0))) + dl * hge;
+        }
+        M[i][3] = gg[i];
+    }
+#pragma unroll
+    for (int j = 0; j < 3; ++j)
+        M[3][j] = gf[0] * (j == 0 ? a_d : a_o) + gf[1] * (j == 1 ? a_d : a_o) + gf[2] * (j == 2 ? a_d : a_o);
+    M[3][3] = T(R(0));
+}
+// one local Newton iteration on (e, dl); x: the step it took
+template <typename T, typename R, typename LT>
+GW_HD void dp_iterate(const T etr[3], LT lam, LT mu, const MatConst &c, T tau[3], T &P, T S[3], T &Q, T e[3], T &dl,
+                      T x[4]) {
+    T gg[3], rhs[4], M[4][4];
+    dp_residual<T, R>(etr, c, tau, P, Q, e, dl, gg, rhs);
+    dp_jacobian<T, R, LT>(lam, mu, c, tau, S, Q, dl, gg, M);
+    solve4(M, rhs, x);
+#pragma unroll
+    for (int i = 0; i < 3; ++i) e[i] = e[i] - x[i];
+    dl = dl - x[3];
+    dp_invariants<T, R, LT>(e, lam, mu, tau, P, S, Q);
+}
+
+template <typename R> GW_HD void set_lane(Dual<4, R> &a, int l, R v) { a.d[l] = v; }
+template <typename R> GW_HD R lane_of(const Dual<4, R> &a, int l) { return a.d[l]; }
+
+// The reference runs ten local iterations and differentiates all of them.  In
+// duals that is ten 4 x 4 eliminations of five-component numbers: 5.1 ms for a
+// million points with their tangent, bound by FP64 issue and spills.  Here the
+// iterations run on values; where they have converged, the derivative is that of
+// the fixed point, -M^-1 d(residual)/d(trial) at the converged state: M is the
+// exact Jacobian, and the step's own derivative there adds dM times a step of
+// round-off size.  Ten steps in duals remain for states whose iteration has not
+// converged (at the cone's tip).
 template <typename T, typename R, typename LT>
 GW_HD void rm_dp(const T etr[3], LT lam, LT mu, const MatConst &c, T e[3]) {
-    const R Af = R(c.A_phi), Bf = R(c.B_phi), Ap = R(c.A_psi), Bp = R(c.B_psi), sf = R(c.sf);
-    T tau[3], P, S[3], Q;
-    dp_invariants<T, R, LT>(etr, lam, mu, tau, P, S, Q);
+    typedef Dual<0, R> V;
+    const R Af = R(c.A_phi), Bf = R(c.B_phi), sf = R(c.sf);
+    const V lv = V(val(lam)), mv = V(val(mu));
+    V etv[3], ev[3], tv[3], Pv, Sv[3], Qv;
 #pragma unroll
-    for (int i = 0; i < 3; ++i) e[i] = etr[i];
-    T y0 = dp_yield(P, Q, Af, Bf, sf);
+    for (int i = 0; i < 3; ++i) { etv[i] = V(val(etr[i])); ev[i] = etv[i]; e[i] = etr[i]; }
+    dp_invariants<V, R, V>(etv, lv, mv, tv, Pv, Sv, Qv);
+    V y0 = dp_yield(Pv, Qv, Af, Bf, sf);
     if (val(y0) < R(1e-10)) return;     // elastic
-    if (c.dp_cutoff && val(P) >= R(0)) return;  // apex return not implemented in the reference (:347-349)
+    if (c.dp_cutoff && val(Pv) >= R(0)) return;  // apex return not implemented in the reference (:347-349)
     if (!c.dp_cutoff && Bf > R(0)) {
         // extension: at or beyond the tip P_tip = A (1 - sf) / B no cone state is
         // reachable; return to the tip (isotropic state), continuous with the cone return
         const R p_tip = Af * (R(1) - sf) / Bf;
-        if (val(P) >= p_tip) {
+        if (val(Pv) >= p_tip) {
             const LT K3 = (lam + 2.0 * mu / 3.0) * 3.0;
             // the tip state is fixed (zero exact tangent); a nonzero tip_tangent keeps
             // that fraction of the trial strain's derivative, value unchanged
@@ -144,36 +205,55 @@ GW_HD void rm_dp(const T etr[3], LT lam, LT mu, const MatConst &c, T e[3]) {
             return;
         }
     }
-    T dl = T(R(0));
-    const LT a_d = lam + 2.0 * mu, a_o = lam;  // elastic_a = lam 1 1^T + 2 mu I
+    // all ten iterations on the value, fewer where one left (e, dl) as it was (the
+    // rest would repeat it): a state on the yield surface decides elastic or
+    // plastic in the next load step by its last bits, so these must not change
+    V dlv = V(R(0));
+    bool conv = false;
     for (int it = 0; it < 10; ++it) {
-        T gg[3], gf[3], hg[3][3];
-        dp_grad(tau, Q, Ap, Bp, sf, gg);
-        dp_grad(tau, Q, Af, Bf, sf, gf);
-        dp_hess(S, Q, Ap, sf, hg);
-        T y = dp_yield(P, Q, Af, Bf, sf);
-        T M[4][4], rhs[4], x[4];
-#pragma unroll
-        for (int i = 0; i < 3; ++i) {
-            rhs[i] = e[i] - etr[i] + dl * gg[i];
-            // (hess_g @ a)_ij = sum_k hg_ik a_kj ;  grad_f_eps_j = sum_i gf_i a_ij
-#pragma unroll
-            for (int j = 0; j < 3; ++j) {
-                T hge = hg[i][0] * (j == 0 ? a_d : a_o) + hg[i][1] * (j == 1 ? a_d : a_o) + hg[i][2] * (j == 2 ? a_d : a_o);
-                M[i][j] = (i == j ? T(R(1)) : T(R(0))) + dl * hge;
-            }
-            M[i][3] = gg[i];
-        }
-#pragma unroll
-        for (int j = 0; j < 3; ++j)
-            M[3][j] = gf[0] * (j == 0 ? a_d : a_o) + gf[1] * (j == 1 ? a_d : a_o) + gf[2] * (j == 2 ? a_d : a_o);
-        M[3][3] = T(R(0));
-        rhs[3] = y;
-        solve4(M, rhs, x);
-#pragma unroll
-        for (int i = 0; i < 3; ++i) e[i] = e[i] - x[i];
-        dl = dl - x[3];
+        const R e0 = val(ev[0]), e1 = val(ev[1]), e2 = val(ev[2]), d0 = val(dlv);
+        V x[4];
+        dp_iterate<V, R, V>(etv, lv, mv, c, tv, Pv, Sv, Qv, ev, dlv, x);
+        const R inc = fmax(fmax(fabs(val(x[0])), fabs(val(x[1]))), fabs(val(x[2])));
+        // quadratic convergence: a step of 1e-9 of the deviatoric strain (the scale on
+        // which M varies) leaves M converged to round-off
+        conv = inc <= R(1e-9) * val(Qv) / (R(2) * val(mu)) && fabs(val(x[3])) <= R(1e-9) * fabs(val(dlv));
+        if (val(ev[0]) == e0 && val(ev[1]) == e1 && val(ev[2]) == e2 && val(dlv) == d0) break;
+    }
+    T tau[3], P, S[3], Q, dl, x[4];
+    if (!conv) {
+        dl = T(R(0));
         dp_invariants<T, R, LT>(e, lam, mu, tau, P, S, Q);
+        for (int it = 0; it < 10; ++it) dp_iterate<T, R, LT>(etr, lam, mu, c, tau, P, S, Q, e, dl, x);
+        return;
+    }
+    // residual with the derivatives of the trial strains (and of lam, mu where they carry one)
+    V gv[3], Mv[4][4], B[4][4];
+    dp_grad(tv, Qv, R(c.A_psi), R(c.B_psi), sf, gv);
+    dp_jacobian<V, R, V>(lv, mv, c, tv, Sv, Qv, dlv, gv, Mv);
+    if constexpr (std::is_same<LT, R>::value) {
+#pragma unroll
+        for (int r = 0; r < 4; ++r)
+#pragma unroll
+            for (int l = 0; l < 4; ++l) B[r][l] = r < 3 ? V(-lane_of(etr[r], l)) : V(R(0));
+    } else {
+        T gt[3], rt[4];
+#pragma unroll
+        for (int i = 0; i < 3; ++i) e[i] = T(val(ev[i]));
+        dl = T(val(dlv));
+        dp_invariants<T, R, LT>(e, lam, mu, tau, P, S, Q);
+        dp_residual<T, R>(etr, c, tau, P, Q, e, dl, gt, rt);
+#pragma unroll
+        for (int r = 0; r < 4; ++r)
+#pragma unroll
+            for (int l = 0; l < 4; ++l) B[r][l] = V(lane_of(rt[r], l));
+    }
+    solve4n<4, V>(Mv, B);
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+        e[i] = T(val(ev[i]));
+#pragma unroll
+        for (int l = 0; l < 4; ++l) set_lane(e[i], l, -val(B[i][l]));
     }
 }
 

@@ -570,7 +570,9 @@ __global__ void k_g2p(LaunchConst c, PtrsP p, const double *__restrict__ u_new, 
 }
 
 // ================================================================ single-point return maps
-__global__ void k_return_map(MatConst mc, double lam, double mu, int n, const double *__restrict__ etr,
+// One instantiation per model (MODEL < 0: at run time), so each carries its own code only.
+template <int MODEL>
+__global__ void __launch_bounds__(128) k_return_map(MatConst mc, double lam, double mu, int n, const double *__restrict__ etr,
                              const double *__restrict__ evt, const double *__restrict__ pi_old,
                              double *__restrict__ pi_new, double *__restrict__ e_out, double *__restrict__ tau_out,
                              double *__restrict__ dtau_out) {
@@ -579,7 +581,7 @@ __global__ void k_return_map(MatConst mc, double lam, double mu, int n, const do
     double e[3] = {etr[3 * i], etr[3 * i + 1], etr[3 * i + 2]};
     double tau[3], dt[3][4], eo[3];
     double pn = pi_new ? pi_new[i] : 0.0;
-    principal_model<double>(mc, lam, mu, e, evt ? evt[i] : 0.0, pi_old ? pi_old[i] : 0.0, pn, tau, dt, eo,
+    principal_model<double, MODEL>(mc, lam, mu, e, evt ? evt[i] : 0.0, pi_old ? pi_old[i] : 0.0, pn, tau, dt, eo,
                             dtau_out != nullptr);
     if (pi_new) pi_new[i] = pn;
     for (int k = 0; k < 3; ++k) {
