@@ -488,8 +488,8 @@ int mg_pattern(MgHier &h, const gw_bsr_t *A0, gw_mg_plan_t *plan, cudaStream_t s
         GW_CUDA(cudaMemsetAsync((void *)c.A.stencil, 0, 4 * (size_t)N * mw, s));
         GW_CUDA(cudaMemsetAsync(c.tmp, 0, 4 * ((size_t)nrc + 1), s));
         if (D == 2)
-            k_mg_coarse_stencil<2><<<gw_count_launch(nblk(nrc, kThreads)), kThreads, 0, s>>>(
-                f.L, fa, c.L, nrc, c.A.row2node, (uint32_t *)c.A.stencil, mw, c.tmp);
+            k_mg_coarse_stencil2<<<gw_count_launch(nblk((int64_t)nrc * 32, kThreads)), kThreads, 0, s>>>(
+                f.L, fa, c.L, nrc, c.A.row2node, (uint32_t *)c.A.stencil, c.tmp);
         else
             k_mg_coarse_stencil<3><<<gw_count_launch(nblk(nrc, kThreads)), kThreads, 0, s>>>(
                 f.L, fa, c.L, nrc, c.A.row2node, (uint32_t *)c.A.stencil, mw, c.tmp);
@@ -578,7 +578,7 @@ int mg_numeric(MgHier &h, cudaStream_t s) {
         MgLevel &f = h.lv[l], &c = h.lv[l + 1];
         PtrsA fa = make_ptrs(f.A), ca = make_ptrs(c.A);
         const int nb = c.A.nnzb;
-        if (D == 2) k_mg_rap<2, NF, VT><<<gw_count_launch(nblk(nb, kThreads)), kThreads, 0, s>>>(f.L, fa, f.fixed, c.L, ca, c.blockrow);
+        if (D == 2) k_mg_rap2<NF, VT><<<gw_count_launch(nblk((int64_t)nb * 16, kThreads)), kThreads, 0, s>>>(fa, f.fixed, c.child, c.L, ca, c.blockrow);
         else k_mg_rap<3, NF, VT><<<gw_count_launch(nblk(nb, kThreads)), kThreads, 0, s>>>(f.L, fa, f.fixed, c.L, ca, c.blockrow);
         GW_LAUNCHED();
         const int nrc = c.A.n_rows;
@@ -593,10 +593,15 @@ int mg_numeric(MgHier &h, cudaStream_t s) {
     GW_CUDA(cudaMemsetAsync(h.dM, 0, 8 * (size_t)n * n, s));
     PtrsA ac = make_ptrs(lc.A);
     k_mg_dense_build<NF, VT><<<gw_count_launch(nblk(lc.A.n_rows, kThreads)), kThreads, 0, s>>>(ac, h.dM, n);
-    const size_t smem = 8 * (size_t)n * n;
-    GW_CUDA(cudaFuncSetAttribute(k_mg_dense_invert, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 8 * kMgCoarseMax * kMgCoarseMax));
-    k_mg_dense_invert<<<gw_count_launch(1), 1024, smem, s>>>(h.dM, h.dInv, n);
+    auto inv = k_mg_dense_invert<1>;
+    switch ((n + 31) / 32) {  // columns per lane: n <= kMgCoarseMax = 160
+        case 2: inv = k_mg_dense_invert<2>; break;
+        case 3: inv = k_mg_dense_invert<3>; break;
+        case 4: inv = k_mg_dense_invert<4>; break;
+        case 5: inv = k_mg_dense_invert<5>; break;
+        default: break;
+    }
+    inv<<<gw_count_launch(1), 512, 0, s>>>(h.dM, h.dInv, n);
     GW_LAUNCHED();
     return GW_OK;
 }

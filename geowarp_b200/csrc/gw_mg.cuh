@@ -169,6 +169,46 @@ __global__ void k_mg_coarse_stencil(Lat Lf, PtrsA Af, Lat Lc, int nc_rows, const
     c_count[R] = n;
 }
 
+// The same in 2D, one warp per coarse row: lane q < 9 reads the stencil of child q,
+// then lane t takes offset bit t of every child.  (One thread per row walked
+// 9 children x 25 bits x 4 parents one after the other: 27-65 us a level, now 2-8.)
+__global__ void k_mg_coarse_stencil2(Lat Lf, PtrsA Af, Lat Lc, int nc_rows, const int *__restrict__ c_row2node,
+                                     uint32_t *__restrict__ c_stencil, int *__restrict__ c_count) {
+    const int R = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+    if (R >= nc_rows) return;  // whole warps
+    const int I = c_row2node[R];
+    if (!in_range(I, lat_size(Lc), GS_COARSE_STENCIL)) return;
+    int C[3];
+    lat_coords(Lc, I, C);
+    uint32_t st = 0u;
+    if (lane < 9) {
+        const int ci[3] = {2 * C[0] + lane % 3 - 1, 2 * C[1] + lane / 3 - 1, 0};
+        if (ci[0] >= 0 && ci[0] < Lf.n[0] && ci[1] >= 0 && ci[1] < Lf.n[1]) {
+            const int i = lat_id(Lf, ci);
+            if (Af.node2row[i] >= 0) st = Af.stencil[i];
+        }
+    }
+    const int bx = lane % 5 - 2, by = lane / 5 - 2;
+    uint32_t mask = 0u;
+#pragma unroll
+    for (int q = 0; q < 9; ++q) {
+        const uint32_t m = __shfl_sync(0xffffffffu, st, q);
+        if (lane >= 25 || !((m >> lane) & 1u)) continue;
+        // fine node j at 2 C + t; its parents, relative to C (always within [-2, 2])
+        const int tx = q % 3 - 1 + bx, ty = q / 3 - 1 + by;
+        const int px = tx >> 1, py = ty >> 1;
+        uint32_t row = 1u << (px + 2);
+        if (tx & 1) row |= 1u << (px + 3);
+        mask |= row << (5 * (py + 2));
+        if (ty & 1) mask |= row << (5 * (py + 3));
+    }
+    mask = __reduce_or_sync(0xffffffffu, mask);
+    if (lane == 0) {
+        c_stencil[I] = mask;
+        c_count[R] = __popc(mask);
+    }
+}
+
 // block -> row map of a block-CSR (for one-thread-per-block kernels)
 __global__ void k_mg_blockrow(const int *__restrict__ row_ptr, int n_rows, int nnzb, int *__restrict__ blockrow) {
     const int r = blockIdx.x * blockDim.x + threadIdx.x;
@@ -249,6 +289,86 @@ __global__ void k_mg_rap(Lat Lf, PtrsA Af, const uint8_t *__restrict__ ffixed, L
                             }
                         }
             }
+#pragma unroll
+    for (int f = 0; f < NF; ++f)
+#pragma unroll
+        for (int g = 0; g < NF; ++g) out[f * NF + g] = (VT)acc[f][g];
+}
+
+// The same in 2D, 16 lanes per coarse block: lane q < 9 takes child q of I (and
+// fetches child q of J from the transfer list for the group), so the chain of a
+// block is 9 fine blocks instead of 81 lattice look-ups (205 rows FP64: 60 -> 6 us;
+// all levels under 267k rows FP32: 877 -> 575 us).  The lanes' sums are added in a
+// fixed tree.
+template <int NF, typename VT>
+__global__ void __launch_bounds__(256) k_mg_rap2(PtrsA Af, const uint8_t *__restrict__ ffixed,
+                                                 const int *__restrict__ child, Lat Lc, PtrsA Ac,
+                                                 const int *__restrict__ c_blockrow) {
+    const int jb = (blockIdx.x * blockDim.x + threadIdx.x) >> 4, q = threadIdx.x & 15;
+    const bool on = jb < Ac.nnzb;  // idle groups stay for the shuffles
+    int R = -1, Rc = -1, ox = 0, oy = 0;
+    if (on) {
+        R = c_blockrow[jb];
+        Rc = Ac.cols[jb];
+        if (!in_range(R, Ac.n_rows, GS_RAP_COARSE) || !in_range(Rc, Ac.n_rows, GS_RAP_COARSE)) R = -1;
+    }
+    if (R >= 0) {
+        const int I = Ac.row2node[R], J = Ac.row2node[Rc];
+        if (!in_range(I, lat_size(Lc), GS_RAP_COARSE) || !in_range(J, lat_size(Lc), GS_RAP_COARSE)) {
+            R = -1;
+        } else {  // 2 (C_J - C_I)
+            ox = 2 * (J % Lc.n[0] - I % Lc.n[0]);
+            oy = 2 * (J / Lc.n[0] - I / Lc.n[0]);
+        }
+    }
+    int fr = -1, fc = -1, rp = 0;
+    uint32_t st = 0u;
+    unsigned fi = 0u, fj = 0u;
+    if (R >= 0 && q < 9) {
+        fr = child[(size_t)q * Ac.n_rows + R];
+        fc = child[(size_t)q * Ac.n_rows + Rc];
+        if (fr >= 0 && in_range(fr, Af.n_rows, GS_RAP_FINE)) {
+            st = Af.stencil[Af.row2node[fr]];
+            rp = Af.row_ptr[fr];
+            fi = ffixed[fr];
+        }
+        if (fc >= 0 && in_range(fc, Af.n_rows, GS_RAP_FINE)) fj = ffixed[fc];
+    }
+    const double wi = (q % 3 == 1 ? 1.0 : 0.5) * (q / 3 == 1 ? 1.0 : 0.5);
+    double acc[NF][NF];
+#pragma unroll
+    for (int f = 0; f < NF; ++f)
+#pragma unroll
+        for (int g = 0; g < NF; ++g) acc[f][g] = 0.0;
+    const VT *vals = (const VT *)Af.vals;
+#pragma unroll
+    for (int t = 0; t < 9; ++t) {
+        const int c = __shfl_sync(0xffffffffu, fc, t, 16);
+        const unsigned fx = __shfl_sync(0xffffffffu, fj, t, 16);
+        // offset of child t of J from child q of I
+        const int dx = ox + t % 3 - q % 3, dy = oy + t / 3 - q / 3;
+        if (st == 0u || c < 0 || dx < -2 || dx > 2 || dy < -2 || dy > 2) continue;
+        const int bit = (dx + 2) + 5 * (dy + 2);
+        if (!((st >> bit) & 1u)) continue;
+        const int fb = rp + __popc(st & ((1u << bit) - 1u));
+        if (!in_range(fb, Af.nnzb, GS_RAP_FINE)) continue;
+        double blk[NF * NF];
+        load_block<NF, VT>(vals + (size_t)fb * NF * NF, blk);
+        const double w = wi * (t % 3 == 1 ? 1.0 : 0.5) * (t / 3 == 1 ? 1.0 : 0.5);
+#pragma unroll
+        for (int f = 0; f < NF; ++f)
+#pragma unroll
+            for (int g = 0; g < NF; ++g)
+                if (!((fi >> f) & 1u) && !((fx >> g) & 1u)) acc[f][g] += w * blk[f * NF + g];
+    }
+#pragma unroll
+    for (int f = 0; f < NF; ++f)
+#pragma unroll
+        for (int g = 0; g < NF; ++g)
+#pragma unroll
+            for (int o = 8; o > 0; o >>= 1) acc[f][g] += __shfl_down_sync(0xffffffffu, acc[f][g], o, 16);
+    if (!on || q != 0) return;
+    VT *out = (VT *)Ac.vals + (size_t)jb * NF * NF;  // the coarse levels store the fine level's value type
 #pragma unroll
     for (int f = 0; f < NF; ++f)
 #pragma unroll
@@ -671,88 +791,110 @@ __global__ void k_mg_dense_build(PtrsA A, double *__restrict__ M, int n) {
 }
 
 // Inverse of the coarsest operator by in-place Gauss-Jordan elimination with
-// partial pivoting, one CTA, the matrix held in dynamic shared memory
-// (n <= kMgCoarseMax, n*n doubles).  Step k: swap the pivot row into place,
-// divide row k by the pivot p (a_kk := 1/p), and for every other row i with
-// f = a_ik subtract f * row k (a_ik := -f/p).  The row interchanges are undone
-// at the end by swapping columns in reverse order.  A zero pivot column is
-// replaced by a unit pivot, so a singular coarse operator weakens the
-// preconditioner instead of producing non-finite values.  Pivot ties go to the
-// lowest row: the result is deterministic.
-__global__ void k_mg_dense_invert(const double *__restrict__ M, double *__restrict__ Inv, int n) {
-    extern __shared__ double a[];
-    __shared__ int perm[kMgCoarseMax], colsrc[kMgCoarseMax];
-    __shared__ double fk[kMgCoarseMax], prow[kMgCoarseMax], oldk[kMgCoarseMax];
-    __shared__ int piv_s, unit_s;
-    const int t = threadIdx.x, nt = blockDim.x, lane = t & 31, w = t >> 5;
-    for (int q = t; q < n * n; q += nt) a[q] = M[q];
+// partial pivoting, one CTA of 16 warps.  Step k takes the unused row p of largest
+// |a_pk| (the lowest one on ties) as pivot row without moving it, divides it by
+// the pivot (a_pk := 1/pivot) and subtracts a_ik times it from every other row i
+// (a_ik := -a_ik/pivot).  At the end row p_k, column j hold the inverse's row k,
+// column p_j.  A zero pivot column is replaced by a unit pivot, so a singular
+// coarse operator weakens the preconditioner instead of producing non-finite
+// values.  Deterministic.
+//
+// Bound by the chain of n steps.  With the matrix in shared memory every step
+// moved all of it (read and written: 3,200 wavefronts at n = 160) between three
+// barriers, 4-5.5 us a step.  Here it stays in registers: warp w owns rows w + 16 a,
+// lane l columns l + 32 b (NB = columns per lane), so a step moves the pivot row
+// and column only.  Every warp finds the pivot by itself from the published
+// column (integer max of the bits of |a|), which leaves two barriers.
+// n = 126 / 156 on B200: 502 / 900 us -> 119 / 209 us.
+template <int NB>
+__global__ void __launch_bounds__(512, 1) k_mg_dense_invert(const double *__restrict__ M, double *__restrict__ Inv, int n) {
+    constexpr int NR = 2 * NB;
+    __shared__ double col[2][32 * NB], prow[32 * NB];
+    __shared__ int perm[32 * NB], inv[32 * NB];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    double a[NR][NB];
+#pragma unroll
+    for (int r = 0; r < NR; ++r)
+#pragma unroll
+        for (int b = 0; b < NB; ++b) {
+            const int i = w + 16 * r, j = lane + 32 * b;
+            a[r][b] = (i < n && j < n) ? M[(size_t)i * n + j] : 0.0;
+        }
+    if (lane == 0)
+#pragma unroll
+        for (int r = 0; r < NR; ++r) col[0][w + 16 * r] = a[r][0];
+    unsigned used = 0u;  // bit q: row lane + 32 q has been a pivot row
+#pragma unroll
+    for (int kb = 0; kb < NB; ++kb) {
+        for (int kk = 0; kk < 32; ++kk) {
+            const int k = 32 * kb + kk;
+            if (k >= n) break;
+            const double *c = col[k & 1];
+            __syncthreads();  // column k is published
+            unsigned hi = 0u, lo = 0u;
+            int idx = 0x7fffffff;
+#pragma unroll
+            for (int q = 0; q < NB; ++q) {
+                const int i = lane + 32 * q;
+                if (i >= n || ((used >> q) & 1u)) continue;
+                const double v = fabs(c[i]);
+                const unsigned long long bits = v == v ? (unsigned long long)__double_as_longlong(v) : 0ull;
+                const unsigned h = (unsigned)(bits >> 32), l = (unsigned)bits;
+                if (idx == 0x7fffffff || h > hi || (h == hi && l > lo)) { hi = h; lo = l; idx = i; }
+            }
+            const unsigned mh = __reduce_max_sync(0xffffffffu, hi);
+            const bool in_h = idx != 0x7fffffff && hi == mh;
+            const unsigned ml = __reduce_max_sync(0xffffffffu, in_h ? lo : 0u);
+            const int p = (int)__reduce_min_sync(0xffffffffu, in_h && lo == ml ? (unsigned)idx : 0x7fffffffu);
+            const bool unit = mh == 0u && ml == 0u;  // no nonzero pivot: a unit one in the first unused row
+            const double pinv = unit ? 1.0 : 1.0 / c[p];
+            if (lane == (p & 31)) used |= 1u << (p >> 5);
+            if (threadIdx.x == 0) perm[k] = p;
+            if (w == (p & 15)) {
+                const int pr = p >> 4;
+#pragma unroll
+                for (int r = 0; r < NR; ++r)
+                    if (r == pr)
+#pragma unroll
+                        for (int b = 0; b < NB; ++b) {
+                            const double v = (b == kb && lane == kk) ? pinv : a[r][b] * pinv;
+                            a[r][b] = v;
+                            prow[lane + 32 * b] = v;
+                        }
+            }
+            __syncthreads();  // the pivot row is published
+            double pj[NB];
+#pragma unroll
+            for (int b = 0; b < NB; ++b) pj[b] = prow[lane + 32 * b];
+#pragma unroll
+            for (int r = 0; r < NR; ++r) {
+                const int i = w + 16 * r;
+                const double f = c[i];
+                if (i != p && f != 0.0)
+#pragma unroll
+                    for (int b = 0; b < NB; ++b) a[r][b] = ((b == kb && lane == kk) ? 0.0 : a[r][b]) - f * pj[b];
+            }
+            double *nc = col[(k + 1) & 1];
+            if (kk < 31) {
+                if (lane == kk + 1)
+#pragma unroll
+                    for (int r = 0; r < NR; ++r) nc[w + 16 * r] = a[r][kb];
+            } else if (kb + 1 < NB && lane == 0) {
+#pragma unroll
+                for (int r = 0; r < NR; ++r) nc[w + 16 * r] = a[r][kb + 1 < NB ? kb + 1 : kb];
+            }
+        }
+    }
     __syncthreads();
-    // elimination threads: column j, row group g of G (each keeps its pivot-row
-    // entry in a register; the multipliers fk[i] are broadcast reads)
-    const int G = nt / n, j = t % n, g = t / n;
-    for (int k = 0; k < n; ++k) {
-        // 1. pivot: the first row of largest |a_ik|, i >= k (warp 0)
-        if (w == 0) {
-            double best = -1.0;
-            int bi = k;
-            for (int i = k + lane; i < n; i += 32) {
-                const double v = fabs(a[i * n + k]);
-                if (v > best) { best = v; bi = i; }
-            }
-            for (int o = 16; o > 0; o >>= 1) {
-                const double ov = __shfl_down_sync(0xffffffffu, best, o);
-                const int oi = __shfl_down_sync(0xffffffffu, bi, o);
-                if (ov > best || (ov == best && oi < bi)) { best = ov; bi = oi; }
-            }
-            if (lane == 0) {
-                const int unit = !(best > 0.0);  // no nonzero pivot: unit pivot in place
-                piv_s = unit ? k : bi;
-                unit_s = unit;
-                perm[k] = piv_s;
-            }
-        }
-        __syncthreads();
-        // 2. stage the swapped-in pivot row scaled by 1/pivot, the old row k
-        //    (it moves to row p) and column k of the row-swapped matrix
-        const int p = piv_s, unit = unit_s;
-        const double pinv = 1.0 / (unit ? 1.0 : a[p * n + k]);
-        if (t < n) {
-            const double rp = (unit && t == k) ? 1.0 : a[p * n + t];
-            prow[t] = (t == k) ? pinv : rp * pinv;
-            oldk[t] = a[k * n + t];
-        } else if (t < 2 * n) {
-            const int i = t - n;
-            const int src = (i == k) ? p : (i == p ? k : i);
-            fk[i] = (unit && i == k) ? 1.0 : a[src * n + k];
-        }
-        __syncthreads();
-        // 3. row k := pivot row; every other row i: a_ij -= fk_i prow_j, a_ik := -fk_i / pivot
-        if (g < G) {
-            const double pj = prow[j], ok = oldk[j];
-            for (int i = g; i < n; i += G) {
-                if (i == k) { a[k * n + j] = pj; continue; }
-                const double f = fk[i];
-                const double v = (i == p) ? ok : a[i * n + j];
-                if (j == k) a[i * n + j] = -f * pinv;
-                else a[i * n + j] = (f != 0.0) ? v - f * pj : v;
-            }
-        }
-        __syncthreads();
-    }
-    // undo the row interchanges as column interchanges, last first: compose
-    // them into one column map and apply it while writing out
-    if (t == 0) {
-        for (int q = 0; q < n; ++q) colsrc[q] = q;
-        for (int k = n - 1; k >= 0; --k) {
-            const int p = perm[k];
-            const int tmp = colsrc[k]; colsrc[k] = colsrc[p]; colsrc[p] = tmp;
-        }
-    }
+    for (int k = threadIdx.x; k < n; k += blockDim.x) inv[perm[k]] = k;
     __syncthreads();
-    for (int q = t; q < n * n; q += nt) {
-        const int i = q / n, c = q - i * n;
-        Inv[q] = a[i * n + colsrc[c]];
-    }
+#pragma unroll
+    for (int r = 0; r < NR; ++r)
+#pragma unroll
+        for (int b = 0; b < NB; ++b) {
+            const int i = w + 16 * r, j = lane + 32 * b;
+            if (i < n && j < n) Inv[(size_t)inv[i] * n + perm[j]] = a[r][b];
+        }
 }
 
 // x = Inv b (one warp per row)
