@@ -8,7 +8,6 @@
 #include "gw_host.cuh"
 #include "gw_mg.cuh"
 #include "gw_mg_tail.cuh"
-#include "gw_sell.cuh"
 
 using namespace gw;
 using namespace gwh;
@@ -348,6 +347,7 @@ struct MgHier {
     MgLevel lv[kMgMaxLevels];
     double *dM = nullptr, *dInv = nullptr;
     int dn = 0;
+    unsigned char *timg = nullptr;  // 2D: shared-memory images of the fused tail
 };
 
 gw_grid_t coarse_grid(const gw_grid_t &g) {
@@ -377,6 +377,7 @@ struct FlexVecs {
     double *V, *Z, *w, *partials;
     GScalars *sc;
 };
+constexpr int kTailSmem = 224 * 1024;  // dynamic shared memory of one CTA of the fused tail at most
 void mg_carve_sell(Bump &bp, MgLevel &v, int64_t n_rows, int nf) {
     const int64_t e = sell_elems(n_rows);
     v.scols = (int *)bp.take(4 * e);
@@ -430,6 +431,7 @@ void mg_carve_hier(Bump &bp, MgHier &h, const gw_grid_t &g0, int64_t n_rows0, in
     h.nl = l + 1;  // upper bound; the plan may stop earlier
     h.dM = (double *)bp.take(8 * (int64_t)kMgCoarseMax * kMgCoarseMax);
     h.dInv = (double *)bp.take(8 * (int64_t)kMgCoarseMax * kMgCoarseMax);
+    if (D == 2) h.timg = (unsigned char *)bp.take((int64_t)kTailSmem * kTailMaxCluster);
 }
 void mg_carve_flex(Bump &bp, FlexVecs &fv, int64_t n0, int restart) {
     fv.V = (double *)bp.take(8 * n0 * (restart + 1));
@@ -701,6 +703,169 @@ void mg_next(const MgHier &h, const GmresVecs &G, int start, cudaStream_t s) {
                 smooth ? mg_omega() : 1.0, s);
 }
 
+// -------------------------------------------------------------- fused coarse tail
+// Largest cluster of the tail that the current device keeps resident: 16 CTAs
+// where it can (a size above 8 is not portable), else 8, 0 when neither fits
+// (then every level keeps its own launches).  Queried once per device, before
+// any stream capture (gmres_mg calls it first).
+template <int NF, typename VT>
+int tail_cluster_max() {
+    static int cached[64] = {0};
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
+    const int got = __atomic_load_n(&cached[dev], __ATOMIC_ACQUIRE);
+    if (got) return got > 0 ? got : 0;
+    int size = -1;
+    auto k = k_sell_tail<NF, VT>;
+    if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kTailSmem) == cudaSuccess)
+        for (int cand : {kTailMaxCluster, 8}) {
+            if (cand > 8 && cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess)
+                continue;
+            cudaLaunchConfig_t cfg = {};
+            cfg.gridDim = dim3(cand);
+            cfg.blockDim = dim3(kTailThreads);
+            cfg.dynamicSmemBytes = kTailSmem;
+            cudaLaunchAttribute at;
+            at.id = cudaLaunchAttributeClusterDimension;
+            at.val.clusterDim.x = cand;
+            at.val.clusterDim.y = 1;
+            at.val.clusterDim.z = 1;
+            cfg.attrs = &at;
+            cfg.numAttrs = 1;
+            int n = 0;
+            if (cudaOccupancyMaxActiveClusters(&n, (void *)k, &cfg) == cudaSuccess && n >= 1) {
+                size = cand;
+                break;
+            }
+        }
+    (void)cudaGetLastError();  // a refused query leaves no error behind
+    __atomic_store_n(&cached[dev], size, __ATOMIC_RELEASE);
+    return size > 0 ? size : 0;
+}
+
+struct TailShape {
+    int l0;       // first level of the tail; h.nl - 1: none
+    int cluster;
+    int smem;     // bytes
+};
+// log2 of a level's rows per CTA: a power of two, at least one chunk of 8
+int tail_sh(int n_rows, int cluster) {
+    int sh = 3;
+    while (((int64_t)cluster << sh) < n_rows) ++sh;
+    return sh;
+}
+// shared memory of one CTA; off (may be null): every level's vectors, the dense one's
+// at h.nl - 1, the image's start at h.nl
+template <int NF, typename VT>
+int64_t tail_bytes(const MgHier &h, int l0, int cluster, int *off) {
+    const int last = h.nl - 1;
+    int64_t d = 0, img = sizeof(TailHead);
+    for (int l = l0; l < last; ++l) {
+        const int sh = tail_sh(h.lv[l].A.n_rows, cluster);
+        if (off) off[l] = (int)d;
+        d += 4 * tail_vec<NF>(sh);
+        img += TailPart<NF, VT>(sh, kTailT).bytes();
+    }
+    if (off) off[last] = (int)d;
+    d += (16 * (int64_t)h.dn + 15) / 16 * 16;
+    if (off) off[last + 1] = (int)d;
+    return d + img + tail_dense_bytes(h.dn, h.lv[last].A.n_rows, cluster);
+}
+// First level of at most GW_TUNE_MG_TAIL rows (0: kTailRows) whose rows, with
+// those of the levels below, fit the cluster's shared memory; at least as many
+// CTAs as give each warp one chunk of that level and one row of the dense inverse.
+constexpr int kTailRows = 2048;
+template <int NF, typename VT>
+TailShape tail_shape(const MgHier &h) {
+    const int last = h.nl - 1, cmax = tail_cluster_max<NF, VT>();
+    const int bound = g_tune[GW_TUNE_MG_TAIL] > 0 ? std::min(g_tune[GW_TUNE_MG_TAIL], 16384) : kTailRows;
+    TailShape t{last, 0, 0};
+    if (cmax == 0) return t;
+    for (int l = mg_bf16_fine<VT>() ? 1 : 0; l < last; ++l) {  // the tail reads the solve's own values
+        const int n = h.lv[l].A.n_rows;
+        if (n > bound || sell_lpr(n) != 4) continue;
+        int c = 1;
+        while (c < cmax && (c * kTailWarps * 8 < n || c * kTailWarps < h.dn || tail_bytes<NF, VT>(h, l, c, nullptr) > kTailSmem)) c *= 2;
+        const int64_t b = tail_bytes<NF, VT>(h, l, c, nullptr);
+        if (b > kTailSmem) continue;
+        return TailShape{l, c, (int)b};
+    }
+    return t;
+}
+
+template <int NF, typename VT>
+TailArgs tail_args(const MgHier &h, const TailShape &t) {
+    const int last = h.nl - 1;
+    TailArgs a;
+    memset(&a, 0, sizeof(a));
+    a.l0 = t.l0;
+    a.last = last;
+    a.cluster = t.cluster;
+    int off[kMgMaxLevels + 1];
+    (void)tail_bytes<NF, VT>(h, t.l0, t.cluster, off);
+    for (int l = t.l0; l < last; ++l) {
+        const MgLevel &v = h.lv[l];
+        TailLevel &w = a.lv[l];
+        w.A = sell_of(v, false);
+        w.Minv = v.Minv;
+        w.fixed = v.fixed;
+        w.child = v.child;
+        w.parent = v.parent;
+        w.sh = tail_sh(v.A.n_rows, t.cluster);
+        w.off = off[l];
+        w.sweeps = mg_sweeps(l);
+    }
+    a.dInv = h.dInv;
+    a.dn = h.dn;
+    a.n_last = h.lv[last].A.n_rows;
+    a.child_last = h.lv[last].child;
+    a.off_last = off[last];
+    a.off_img = off[last + 1];
+    a.img = h.timg;
+    a.img_stride = kTailSmem;
+    a.omega = mg_omega();
+    return a;
+}
+
+// The images of the tail's shared memory, after the values they copy (on every
+// solve: the tail may hold the finest level, and its knobs may have changed).
+template <int NF, typename VT>
+int tail_image(const MgHier &h, cudaStream_t s) {
+    const TailShape t = tail_shape<NF, VT>(h);
+    if (t.l0 == h.nl - 1) return GW_OK;
+    k_tail_image<NF, VT><<<dim3(gw_count_launch(t.cluster), h.nl - t.l0), 256, 0, s>>>(tail_args<NF, VT>(h, t));
+    GW_LAUNCHED();
+    return GW_OK;
+}
+
+template <int NF, typename VT>
+void sell_tail(const MgHier &h, const TailShape &t, VecRef b, VecRef out, const GScalars *sc, cudaStream_t s) {
+    TailArgs a = tail_args<NF, VT>(h, t);
+    a.b = b;
+    a.out = out;
+    a.x1 = h.lv[t.l0].x;
+    a.sc = sc;
+    double bytes = 8.0 * h.dn * h.dn;
+    for (int l = t.l0; l + 1 < h.nl; ++l)
+        bytes += (double)h.lv[l].A.nnzb * (NF * NF * sizeof(VT) + 4) + 8.0 * h.lv[l].A.n_rows * NF * (NF + 2);
+    ProfScope ps(PC_MG_TAIL, s, bytes);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(gw_count_launch(t.cluster));
+    cfg.blockDim = dim3(kTailThreads);
+    cfg.dynamicSmemBytes = t.smem;
+    cfg.stream = s;
+    cudaLaunchAttribute at[2];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = t.cluster;
+    at[0].val.clusterDim.y = 1;
+    at[0].val.clusterDim.z = 1;
+    at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 2;
+    (void)cudaLaunchKernelEx(&cfg, k_sell_tail<NF, VT>, a);
+}
+
 // One V-cycle on v_k, result in Z[k].  The zero-start sweep of every level comes
 // with its right-hand side (mg_next, k_sell_restrict).
 template <int NF, typename VT>
@@ -708,8 +873,10 @@ void sell_vcycle(const MgHier &h, const GmresVecs &G, VecRef z, cudaStream_t s) 
     const int last = h.nl - 1;
     const GScalars *sc = G.sc;
     const VecRef v0{G.V, G.n};
+    const TailShape tail = tail_shape<NF, VT>(h);
+    const int l0 = tail.l0;
     double *cur[kMgMaxLevels], *oth[kMgMaxLevels];
-    for (int l = 0; l < last; ++l) {
+    for (int l = 0; l < l0; ++l) {
         const MgLevel &v = h.lv[l], &c = h.lv[l + 1];
         const VecRef b = l == 0 ? v0 : VecRef{v.b, 0};
         double *x = v.x, *y = v.x2;
@@ -727,12 +894,16 @@ void sell_vcycle(const MgHier &h, const GmresVecs &G, VecRef z, cudaStream_t s) 
         cur[l] = x;
         oth[l] = y;
     }
-    const MgLevel &lc = h.lv[last];
-    const VecRef bl = last == 0 ? v0 : VecRef{lc.b, 0};
-    launch_pdl(k_sell_dense_apply, nblk((int64_t)h.dn * 32, kThreads), kThreads, 0, s, (const double *)h.dInv, bl,
-               last == 0 ? z : VecRef{lc.x, 0}, h.dn, sc);
-    cur[last] = lc.x;
-    for (int l = last - 1; l >= 0; --l) {
+    const VecRef bl = l0 == 0 ? v0 : VecRef{h.lv[l0].b, 0};
+    if (l0 < last) {
+        sell_tail<NF, VT>(h, tail, bl, l0 == 0 ? z : VecRef{h.lv[l0].x2, 0}, sc, s);
+        cur[l0] = h.lv[l0].x2;
+    } else {
+        launch_pdl(k_sell_dense_apply, nblk((int64_t)h.dn * 32, kThreads), kThreads, 0, s, (const double *)h.dInv, bl,
+                   last == 0 ? z : VecRef{h.lv[last].x, 0}, h.dn, sc);
+        cur[last] = h.lv[last].x;
+    }
+    for (int l = l0 - 1; l >= 0; --l) {
         const MgLevel &v = h.lv[l], &c = h.lv[l + 1];
         const VecRef b = l == 0 ? v0 : VecRef{v.b, 0};
         double *x = cur[l], *y = oth[l];
@@ -769,125 +940,13 @@ void mg_jacobi(const MgHier &h, int l, const double *b, const double *xin, doubl
     else k_mg_jacobi<NF, VT><<<gw_count_launch(g), tb, 0, s>>>(a, v.Minv, b, xin, xout, mg_omega(), zero, skip);
 }
 
-// Largest cluster of the fused coarse tail for this instantiation on the
-// current device: 16 CTAs where the device can run such a cluster of it, else
-// 8, 0 when neither fits (then every level keeps its own launches).  Queried once
-// per device, before any stream capture (gmres_mg calls it first).
-template <int D, int NF>
-int tail_cluster_size() {
-    static int cached[64] = {0};
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
-    if (cached[dev]) return cached[dev] > 0 ? cached[dev] : 0;
-    int size = -1;
-    for (int cand : {16, 8}) {
-        if (cand > 8 && cudaFuncSetAttribute(k_mg_tail<D, NF>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) !=
-                            cudaSuccess)
-            continue;
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3(cand);
-        cfg.blockDim = dim3(kTailThreads);
-        cudaLaunchAttribute at;
-        at.id = cudaLaunchAttributeClusterDimension;
-        at.val.clusterDim.x = cand;
-        at.val.clusterDim.y = 1;
-        at.val.clusterDim.z = 1;
-        cfg.attrs = &at;
-        cfg.numAttrs = 1;
-        int n = 0;
-        if (cudaOccupancyMaxActiveClusters(&n, (void *)k_mg_tail<D, NF>, &cfg) == cudaSuccess && n >= 1) {
-            size = cand;
-            break;
-        }
-    }
-    (void)cudaGetLastError();  // a refused query leaves no error behind
-    cached[dev] = size;
-    return size > 0 ? size : 0;
-}
-
-template <int NF>
-int tail_cluster_size(int D) { return D == 2 ? tail_cluster_size<2, NF>() : tail_cluster_size<3, NF>(); }
-
-// First level of the fused coarse tail (the first coarse level with at most
-// GW_TUNE_MG_TAIL rows), or h.nl - 1 when the tail is off or has no level to
-// smooth.
-template <int NF, typename VT>
-int tail_level(const MgHier &h) {
-    const int last = h.nl - 1, T = g_tune[GW_TUNE_MG_TAIL];
-    // the fused tail reads FP64 coarse operators: FP64 solves only
-    if (!std::is_same<VT, double>::value) return last;
-    if (T <= 0 || last < 2 || tail_cluster_size<NF>(h.lv[0].g.dim) == 0) return last;
-    for (int l = 1; l < last; ++l)
-        if (h.lv[l].A.n_rows <= T) return l;
-    return last;
-}
-
-// Launches levels l0 .. last of the V-cycle as one cluster and returns the
-// buffer that holds level l0's result (the same one the per-phase path ends in).
-template <int NF>
-double *mg_tail(const MgHier &h, int l0, const int *skip, cudaStream_t s) {
-    const int last = h.nl - 1, D = h.lv[0].g.dim;
-    TailArgs ta;
-    memset(&ta, 0, sizeof(ta));
-    ta.l0 = l0;
-    ta.last = last;
-    ta.dInv = h.dInv;
-    ta.dn = h.dn;
-    ta.omega = mg_omega();
-    ta.skip = skip;
-    double bytes = 8.0 * h.dn * h.dn;
-    for (int l = l0; l <= last; ++l) {
-        const MgLevel &v = h.lv[l];
-        TailLevel &t = ta.lv[l];
-        t.A = make_ptrs(v.A);
-        t.L = v.L;
-        t.Minv = v.Minv;
-        t.b = v.b; t.x = v.x; t.x2 = v.x2; t.r = v.r;
-        t.fixed = v.fixed;
-        t.sweeps = mg_sweeps(l);
-        if (l < last) {
-            const double vs = 8.0 * v.A.n_rows * NF, vc = 8.0 * h.lv[l + 1].A.n_rows * NF;
-            const double mat = (double)v.A.nnzb * (NF * NF * 8 + 4), minv = 8.0 * v.A.n_rows * NF * NF;
-            bytes += (mat + 2 * vs + minv) + (mat + 3 * vs) + (vs + vc) + (2 * vs + vc) + t.sweeps * (mat + 3 * vs + minv);
-        }
-    }
-    // cluster just large enough for two block rows of level l0 per row group
-    // (128 groups per CTA), at most what the device runs
-    const int cmax = tail_cluster_size<NF>(D), need = (h.lv[l0].A.n_rows + 255) / 256;
-    int cl = 1;
-    while (cl < need && cl < cmax) cl *= 2;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(cl);
-    cfg.blockDim = dim3(kTailThreads);
-    cfg.stream = s;
-    cudaLaunchAttribute at;
-    at.id = cudaLaunchAttributeClusterDimension;
-    at.val.clusterDim.x = cl;
-    at.val.clusterDim.y = 1;
-    at.val.clusterDim.z = 1;
-    cfg.attrs = &at;
-    cfg.numAttrs = 1;
-    {
-        ProfScope ps(PC_MG_TAIL, s, bytes);
-        gw_count_launch(cl);
-        if (D == 2) cudaLaunchKernelEx(&cfg, k_mg_tail<2, NF>, ta);
-        else cudaLaunchKernelEx(&cfg, k_mg_tail<3, NF>, ta);
-    }
-    // the buffer the per-phase path would end level l0 in: x on the way down,
-    // alternating with x2 once per sweep
-    const int S = mg_sweeps(l0);
-    const int swaps = (S >= 2 ? 1 + (S - 2) : S - 1) + S;
-    return (swaps & 1) ? h.lv[l0].x2 : h.lv[l0].x;
-}
-
 // 3D (block-CSR rows of up to 125 blocks): one V-cycle on h.lv[0].b; returns the buffer that holds the result (the same
-// buffer on every call).  Levels from tail_level() down run fused (mg_tail).
+// buffer on every call).
 template <int NF, typename VT>
 double *mg_vcycle(const MgHier &h, const int *skip, cudaStream_t s) {
     const int last = h.nl - 1;
-    const int l0 = tail_level<NF, VT>(h);
     double *cur[kMgMaxLevels], *oth[kMgMaxLevels];
-    for (int l = 0; l < l0; ++l) {
+    for (int l = 0; l < last; ++l) {
         const MgLevel &v = h.lv[l], &c = h.lv[l + 1];
         double *x = v.x, *y = v.x2;
         if (mg_sweeps(l) >= 2) {
@@ -943,14 +1002,10 @@ double *mg_vcycle(const MgHier &h, const int *skip, cudaStream_t s) {
         cur[l] = x;
         oth[l] = y;
     }
-    if (l0 < last) {
-        cur[l0] = mg_tail<NF>(h, l0, skip, s);
-    } else {
-        const MgLevel &lc = h.lv[last];
-        k_mg_dense_apply<<<gw_count_launch(nblk((int64_t)h.dn * 32, kThreads)), kThreads, 0, s>>>(h.dInv, lc.b, lc.x, h.dn, skip);
-        cur[last] = lc.x;
-    }
-    for (int l = l0 - 1; l >= 0; --l) {
+    const MgLevel &lc = h.lv[last];
+    k_mg_dense_apply<<<gw_count_launch(nblk((int64_t)h.dn * 32, kThreads)), kThreads, 0, s>>>(h.dInv, lc.b, lc.x, h.dn, skip);
+    cur[last] = lc.x;
+    for (int l = last - 1; l >= 0; --l) {
         const MgLevel &v = h.lv[l], &c = h.lv[l + 1];
         PtrsA a = make_ptrs(v.A), ca = make_ptrs(c.A);
         double *x = cur[l], *y = oth[l];
@@ -1094,7 +1149,7 @@ int gmres_mg(const gw_grid_t *grid, const gw_bsr_t *A, gw_mg_plan_t *plan_in, co
     const int nr = A->n_rows;
     if (nr == 0) { *iters = 0; *relres = 0.0; return GW_OK; }
     const int64_t n = (int64_t)nr * NF;
-    (void)tail_cluster_size<NF>(grid->dim);  // device queries before any stream capture
+    (void)tail_cluster_max<NF, VT>();  // device queries before any stream capture
     {
         const int tb = tune_rows_block();
         (void)resident_rows_grid((const void *)k_mg_jacobi<NF, VT>, tb, 1);
@@ -1138,7 +1193,9 @@ int gmres_mg(const gw_grid_t *grid, const gw_bsr_t *A, gw_mg_plan_t *plan_in, co
         // the V-cycle's BF16 copy of the fine level follows the current A on
         // every solve, lagged or not (the fine level's own rows are never lagged)
         if (!rc && grid->dim == 2) {
-            rc = sell_values<NF, VT>(h, !(plan_in && plan_in->lag), s);
+            const bool fresh = !(plan_in && plan_in->lag);
+            rc = sell_values<NF, VT>(h, fresh, s);
+            if (!rc) rc = tail_image<NF, VT>(h, s);
         } else if (!rc && mg_bf16_fine<VT>()) {
             const size_t nv = (size_t)A->nnzb * NF * NF;
             k_to_bf16<<<gw_count_launch(red_grid_elems((int64_t)nv)), kThreads, 0, s>>>(

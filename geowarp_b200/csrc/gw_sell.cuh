@@ -104,11 +104,10 @@ struct SellRow {
                 for (int u = 0; u < NU; ++u) val[t][u] = sell_ld(vp + (t * NU + u) * 32);
             }
     }
-    static __device__ __forceinline__ void mad(const U v[NU], const double *x, double acc[NF]) {
-        double b[NF * NF], xv[NF];
+    static __device__ __forceinline__ void mad(const U v[NU], const double xv[NF], double acc[NF]) {
+        double b[NF * NF];
 #pragma unroll
         for (int u = 0; u < NU; ++u) unit_get(v[u], b + u * (NF * NF / NU));
-        load_rw<NF>(x, xv);
 #pragma unroll
         for (int f = 0; f < NF; ++f)
 #pragma unroll
@@ -118,9 +117,13 @@ struct SellRow {
     __device__ __forceinline__ void mul(const SellA &A, int c, int lane, const double *x, double acc[NF]) const {
 #pragma unroll
         for (int f = 0; f < NF; ++f) acc[f] = 0.0;
+        double xv[NF];
 #pragma unroll
         for (int t = 0; t < PF; ++t)
-            if (t < trips) mad(val[t], x + (size_t)col[t] * NF, acc);
+            if (t < trips) {
+                load_rw<NF>(x + (size_t)col[t] * NF, xv);
+                mad(val[t], xv, acc);
+            }
         if (PF < T) {
             const int *cp = A.cols + (size_t)c * T * 32 + lane;
             const U *vp = (const U *)A.vals + (size_t)c * T * NU * 32 + lane;
@@ -129,7 +132,8 @@ struct SellRow {
                 U v[NU];
 #pragma unroll
                 for (int u = 0; u < NU; ++u) v[u] = sell_ld(vp + (t * NU + u) * 32);
-                mad(v, x + (size_t)sell_ld(cp + t * 32) * NF, acc);
+                load_rw<NF>(x + (size_t)sell_ld(cp + t * 32) * NF, xv);
+                mad(v, xv, acc);
             }
         }
         if (LPR > 1) {
@@ -140,7 +144,6 @@ struct SellRow {
         }
     }
 };
-
 // ---------------------------------------------------------------- laying a matrix out
 // One warp per chunk: trips and columns (pattern), or the values.
 __global__ void k_sell_pattern(PtrsA A, int lpr, int *__restrict__ trips, int *__restrict__ cols) {

@@ -251,3 +251,30 @@ def test_second_gram_schmidt_passes_do_not_change_the_solution(cuda):
             assert (knob != 0 or re == it) and (knob != 300 or re == 0)
     finally:
         G.lib.gw_tune_set(G.L.TUNE_GS_CANCEL, default)
+
+
+@pytest.mark.parametrize("single", [False, True], ids=["fp64", "mixed"])
+@pytest.mark.parametrize("nx,ny,nf,holes,wide", [
+    (9, 9, 2, 0.05, 0.3),     # one smoothed level: one CTA
+    (15, 15, 1, 0.0, 0.0),    # 256 rows: two CTAs, every chunk whole
+    (30, 16, 2, 0.02, 1.0),   # 25-point rows
+    (41, 27, 3, 0.05, 0.2),
+    (63, 50, 4, 0.0, 0.1),    # rows of a level over several passes of a warp
+    (100, 80, 2, 0.0, 0.1),   # tail below the finest level by default, with it at 16384
+])
+def test_fused_tail_is_bitwise_the_separate_levels(cuda, nx, ny, nf, holes, wide, single):
+    """GW_TUNE_MG_TAIL = 1 leaves every level its own launches; the default and
+    16384 start the cluster at other levels.  Same arithmetic, same bytes."""
+    S = _system(nx, ny, nf, 10, holes, wide)
+    b = np.random.default_rng(4).standard_normal(S["n_rows"] * nf)
+    G = _Gpu(S, single, cuda)
+    default = G.lib.gw_tune_get(G.L.TUNE_MG_TAIL)
+    out = []
+    try:
+        for knob in (1, 0, 16384):
+            assert G.lib.gw_tune_set(G.L.TUNE_MG_TAIL, knob) == G.L.GW_OK
+            out.append(G.solve(b, 12, 1e-30))
+    finally:
+        G.lib.gw_tune_set(G.L.TUNE_MG_TAIL, default)
+    for x, it, rr, rc in out[1:]:
+        assert it == out[0][1] and np.array_equal(x, out[0][0])
