@@ -23,6 +23,20 @@ void assemble_per_model(const LaunchConst &c, const PtrsP &p, const int *perm, c
     }
 }
 
+// 3D: eight particles per CTA (27 threads each) up to two CTAs per SM, then 32, a
+// whole warp's worth of evaluations
+template <bool WANT_K, typename VT>
+int launch_assemble3(const LaunchConst &c, const PtrsP &p, const int *perm, const uint8_t *fm, const double *un,
+                     const double *uo, const PtrsA &a, double *R, double *force, cudaStream_t s) {
+    const int P = p.n <= 8 * 2 * 148 ? 8 : 32;
+    auto k = k_assemble3<WANT_K, VT>;
+    const int smem = P * (int)sizeof(Scatter3<WANT_K>);
+    GW_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 32 * (int)sizeof(Scatter3<WANT_K>)));
+    k<<<gw_count_launch(nblk(p.n, P)), 256, smem, s>>>(c, p, P, perm, fm, un, uo, a, R, force);
+    GW_LAUNCHED();
+    return GW_OK;
+}
+
 template <int KIND>
 int launch_assemble(const LaunchConst &c, const PtrsP &p, const int *perm, const uint8_t *fm, const double *un,
                     const double *uo, const gw_bsr_t *A, int prec, double *R, double *force, const PtrsA &a,
@@ -40,7 +54,13 @@ int launch_assemble(const LaunchConst &c, const PtrsP &p, const int *perm, const
         const bool want_K = A->vals != nullptr;
         const double mat = want_K ? (double)A->nnzb * NF * NF * (prec == GW_PREC_F64 ? 8 : 4) : 0.0;
         ProfScope ps(PC_ASSEMBLE, s, per_p * p.n + grid + mat);
-        if (!want_K) {
+        if constexpr (KIND == GW_KIND_COUPLED3D) {
+            int rc;
+            if (!want_K) rc = launch_assemble3<false, double>(c, p, perm, fm, un, uo, a, R, force, s);
+            else if (prec == GW_PREC_F64) rc = launch_assemble3<true, double>(c, p, perm, fm, un, uo, a, R, force, s);
+            else rc = launch_assemble3<true, float>(c, p, perm, fm, un, uo, a, R, force, s);
+            if (rc) return rc;
+        } else if (!want_K) {
             k_assemble<KIND, false, double><<<gw_count_launch(b), pb, 0, s>>>(c, p, perm, fm, un, uo, a, R, force);
         } else if constexpr (KIND == GW_KIND_SOLID2D) {
             // the 2D solid tangent kernel is instantiated per material, so each

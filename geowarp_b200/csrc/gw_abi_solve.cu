@@ -191,6 +191,18 @@ void gs_column(const GmresVecs &G, int restart, double vb, cudaStream_t s) {
     { ProfScope ps(PC_DOTS, s, vb); gs_dots(G, restart, 1, s); }
     { ProfScope ps(PC_UPDATE, s, vb + n8); gs_update(G, 1, s); }
 }
+// stream of the solvers' graph captures, one per device
+cudaStream_t g_capture_stream[64] = {};
+
+int capture_stream(cudaStream_t *out) {
+    int dev = 0;
+    GW_CUDA(cudaGetDevice(&dev));
+    if (dev < 0 || dev >= 64) return GW_EINVAL;
+    if (!g_capture_stream[dev]) GW_CUDA(cudaStreamCreateWithFlags(&g_capture_stream[dev], cudaStreamNonBlocking));
+    *out = g_capture_stream[dev];
+    return GW_OK;
+}
+
 int64_t gmres_ws_bytes(int64_t n_rows, int nf, int restart) {
     const int64_t n = n_rows * nf;
     return align256(8 * n * (restart + 1)) + 2 * align256(8 * n) + align256(8 * n_rows * nf * nf) +
@@ -223,11 +235,20 @@ int gmres(const gw_bsr_t *A, int precond, const double *b, double *x, double rto
     k_precond_setup<NF, VT><<<gw_count_launch(nblk(nr, kThreads)), kThreads, 0, s>>>(a, D, precond, G.Minv);
     GW_LAUNCHED();
     const int gr = red_grid_rows(nr), ge = red_grid_elems(nr);
+    // a warp per row where the rows alone do not fill the device and are long
+    // enough for it (below 16 blocks most of its lanes would idle)
+    const bool wide = nr <= 8192 && (int64_t)A->nnzb >= 16 * (int64_t)nr;
     GScalars h;
     memset(&h, 0, head);
     int first = 1;
     StallWatch stall;
     g_last_stalled = 0;
+    struct Step {  // graph of kStepCols columns, for this solve only
+        cudaGraphExec_t exec = nullptr;
+        int64_t launches = 0;
+        ~Step() { if (exec) cudaGraphExecDestroy(exec); }
+    } step;
+    constexpr int kStepCols = 8;
     for (int cycle = 0; cycle < 1000000; ++cycle) {
         k_gm_residual<NF, VT><<<gw_count_launch(gr), kThreads, 0, s>>>(a, G, first, rtol);
         gs_next<NF>(nr, G, 1, G.Minv, G.z, 1.0, s);
@@ -237,20 +258,51 @@ int gmres(const gw_bsr_t *A, int precond, const double *b, double *x, double rto
         GW_CUDA(cudaStreamSynchronize(s));
         if (h.done) break;
         if (stall.stalled(h.beta)) { g_last_stalled = 1; break; }
-        int chunk = 4;
-        int kk = 0;  // host-side column estimate (exact until the cycle closes early)
+        int chunk = 8;
+        int kk = 0;  // columns queued in this cycle: at most `restart` of them can count
         const double spmv_bytes = (double)A->nnzb * (NF * NF * sizeof(VT) + 4) + 4.0 * (nr + 1) + 16.0 * n;
-        for (;;) {
-            for (int it = 0; it < chunk; ++it, ++kk) {
-                const double vb = 8.0 * n * (kk + 2);
-                { ProfScope ps(PC_SPMV, s, spmv_bytes); launch_pdl(k_gm_spmv<NF, VT>, gr, kThreads, 0, s, a, G); }
-                gs_column(G, restart, vb, s);
-                { ProfScope ps(PC_NEXT, s, 8.0 * n * 3 + 8.0 * nr * NF * NF); gs_next<NF>(nr, G, 0, G.Minv, G.z, 1.0, s); }
+        auto column = [&](cudaStream_t st) {
+            {
+                ProfScope ps(PC_SPMV, st, spmv_bytes);
+                if (wide) launch_pdl(k_gm_spmv_wide<NF, VT>, nblk(nr, 4), 128, 0, st, a, G);
+                else launch_pdl(k_gm_spmv<NF, VT>, gr, kThreads, 0, st, a, G);
             }
+            gs_column(G, restart, 8.0 * n * (kk + 2), st);
+            ProfScope ps(PC_NEXT, st, 8.0 * n * 3 + 8.0 * nr * NF * NF);
+            gs_next<NF>(nr, G, 0, G.Minv, G.z, 1.0, st);
+        };
+        for (;;) {
+            chunk = std::min(chunk, restart - kk);
+            int it = 0;
+            if (!g_prof_on && (step.exec || kk > 0)) {
+                // a solve that needs more than its first columns replays eight at a
+                // time: six launches of 2-3 us of work each cost the host 20 us
+                if (!step.exec && chunk >= kStepCols) {
+                    cudaStream_t cs;
+                    int rc = capture_stream(&cs);
+                    if (rc) return rc;
+                    const int64_t before = g_launches;
+                    cudaGraph_t graph;
+                    GW_CUDA(cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal));
+                    for (int q = 0; q < kStepCols; ++q) column(cs);
+                    const cudaError_t ce = cudaStreamEndCapture(cs, &graph);
+                    step.launches = g_launches - before;
+                    g_launches = before;  // counted when the graph is replayed
+                    GW_CUDA(ce);
+                    const cudaError_t ie = cudaGraphInstantiate(&step.exec, graph, 0);
+                    cudaGraphDestroy(graph);
+                    GW_CUDA(ie);
+                }
+                for (; step.exec && it + kStepCols <= chunk; it += kStepCols, kk += kStepCols) {
+                    GW_CUDA(cudaGraphLaunch(step.exec, s));
+                    g_launches += step.launches;
+                }
+            }
+            for (; it < chunk; ++it, ++kk) column(s);
             GW_LAUNCHED();
             GW_CUDA(cudaMemcpyAsync(&h, G.sc, head, cudaMemcpyDeviceToHost, s));
             GW_CUDA(cudaStreamSynchronize(s));
-            if (h.cycle_done) break;
+            if (h.cycle_done || kk >= restart) break;
             chunk = chunk < 32 ? chunk * 2 : 32;
         }
         if (h.status) break;
@@ -1048,17 +1100,6 @@ struct MgGraphEntry {
 constexpr int kMgGraphCache = 8;
 MgGraphEntry g_mg_graphs[kMgGraphCache];
 uint64_t g_mg_graph_clock = 0;
-cudaStream_t g_capture_stream[64] = {};
-
-int capture_stream(cudaStream_t *out) {
-    int dev = 0;
-    GW_CUDA(cudaGetDevice(&dev));
-    if (dev < 0 || dev >= 64) return GW_EINVAL;
-    if (!g_capture_stream[dev]) GW_CUDA(cudaStreamCreateWithFlags(&g_capture_stream[dev], cudaStreamNonBlocking));
-    *out = g_capture_stream[dev];
-    return GW_OK;
-}
-
 // The next basis vector (start: the first of a cycle) and its V-cycle.
 template <int NF, typename VT>
 void mg_step_tail(const MgHier &h, GmresVecs &G, VecRef z, int start, const int *skip, cudaStream_t s) {

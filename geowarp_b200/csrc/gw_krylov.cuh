@@ -733,6 +733,61 @@ __global__ void k_gm_spmv(PtrsA A, GmresVecs G) {
     }
 }
 
+// The same with a warp per row, for small systems of long rows (3D: up to 125
+// blocks): eight lanes per row leave 216 rows on 7 CTAs and eight dependent trips
+// per lane (12.8 us for 13,824 4 x 4 FP64 blocks).  The first PF trips' columns and
+// blocks are loaded ahead of the wait; the state is tested before the store.
+template <int NF, typename VT>
+__global__ void __launch_bounds__(128) k_gm_spmv_wide(PtrsA A, GmresVecs G) {
+    const int r = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (r >= A.n_rows) return;  // whole warps
+    constexpr int PF = NF * NF * (int)sizeof(VT) > 64 ? 2 : 3;
+    const VT *vals = (const VT *)A.vals;
+    const int s = __ldg(A.row_ptr + r), e = __ldg(A.row_ptr + r + 1);
+    int col[PF];
+    double bv[PF][NF * NF], acc[NF], xv[NF];
+#pragma unroll
+    for (int t = 0; t < PF; ++t) {
+        const int j = s + lane + 32 * t;
+        col[t] = -1;
+        if (j < e) {
+            col[t] = __ldg(A.cols + j);
+            if (!in_range(col[t], A.n_rows, GS_ROW_MV)) col[t] = -1;
+            load_block<NF, VT>(vals + (size_t)j * NF * NF, bv[t]);
+        }
+    }
+    pdl_wait();
+    pdl_release();
+    const bool off = G.sc->cycle_done;
+#pragma unroll
+    for (int f = 0; f < NF; ++f) acc[f] = 0.0;
+#pragma unroll
+    for (int t = 0; t < PF; ++t)
+        if (col[t] >= 0) {
+            load_rw<NF>(G.z + (size_t)col[t] * NF, xv);
+#pragma unroll
+            for (int f = 0; f < NF; ++f)
+#pragma unroll
+                for (int g = 0; g < NF; ++g) acc[f] += bv[t][f * NF + g] * xv[g];
+        }
+    for (int j = s + lane + 32 * PF; j < e; j += 32) {
+        const int c = __ldg(A.cols + j);
+        if (!in_range(c, A.n_rows, GS_ROW_MV)) continue;
+        double b[NF * NF];
+        load_rw<NF>(G.z + (size_t)c * NF, xv);
+        load_block<NF, VT>(vals + (size_t)j * NF * NF, b);
+#pragma unroll
+        for (int f = 0; f < NF; ++f)
+#pragma unroll
+            for (int g = 0; g < NF; ++g) acc[f] += b[f * NF + g] * xv[g];
+    }
+#pragma unroll
+    for (int f = 0; f < NF; ++f)
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) acc[f] += __shfl_down_sync(0xffffffffu, acc[f], o);
+    if (lane == 0 && !off) store_rw<NF>(G.w + (size_t)r * NF, acc);
+}
+
 // ---------------------------------------------------------------- Gram-Schmidt
 // What bounds these kernels: the basis, read once by dots and once by upd (8 (k + 1) n
 // bytes each), and on systems below ~50k unknowns the latency of the reduction.
@@ -929,12 +984,30 @@ __global__ void __launch_bounds__(kGsThreads) k_gm_update(GmresVecs G, int pass)
     __shared__ double red[kGsThreads / 32];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int items = pass == 0 ? k + 2 : k + 1, nb = gs_dots_blocks(G.n);
-    for (int i = warp; i < items; i += kGsThreads / 32) {
-        double s = 0.0;
-#pragma unroll 5
-        for (int b = lane; b < nb; b += 32) s += G.partials[(size_t)i * kGsBlocks + b];
-        s = warp_sum(s);
-        if (lane == 0) coef[i] = s;
+    if (nb <= 8) {  // a thread per item, all of its partials in flight
+        if (threadIdx.x < items) {
+            double p[8], s = 0.0;
+#pragma unroll
+            for (int b = 0; b < 8; ++b) p[b] = b < nb ? G.partials[(size_t)threadIdx.x * kGsBlocks + b] : 0.0;
+#pragma unroll
+            for (int b = 0; b < 8; ++b) s += p[b];
+            coef[threadIdx.x] = s;
+        }
+    } else {
+        for (int i0 = warp; i0 < items; i0 += 4 * kGsThreads / 32) {  // four items of a warp in flight
+            double s[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll 2
+            for (int b = lane; b < nb; b += 32)
+#pragma unroll
+                for (int q = 0; q < 4; ++q)
+                    if (i0 + q * kGsThreads / 32 < items)
+                        s[q] += G.partials[(size_t)(i0 + q * kGsThreads / 32) * kGsBlocks + b];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                s[q] = warp_sum(s[q]);
+                if (lane == 0 && i0 + q * kGsThreads / 32 < items) coef[i0 + q * kGsThreads / 32] = s[q];
+            }
+        }
     }
     __syncthreads();
     if (blockIdx.x == 0 && warp == 0) {
@@ -983,6 +1056,7 @@ __device__ __forceinline__ void gs_close(GScalars *sc, int k, double hn) {
     __syncwarp();
     if (lane == 0) {
         double a = h[0];
+#pragma unroll 8
         for (int i = 0; i < k; ++i) {  // previous rotations
             const double b2 = h[i + 1];
             h[i] = cs[i] * a + sn[i] * b2;
