@@ -109,8 +109,23 @@ extern "C" int gw_assemble(const gw_grid_t *grid, const gw_material_t *mat, cons
     }
 }
 
-// ==================================================================== deterministic (cell-coloured) assembly
+// ==================================================================== deterministic assembly
 namespace {
+// The workspace: cell starts and ends, boxes, particle records, cell sums.
+struct AsmParts {
+    int64_t cend, box, rec, sums, bytes;
+};
+AsmParts asm_parts(int64_t n_cells, int64_t n, int64_t rec_bytes, int64_t sum_bytes) {
+    AsmParts w;
+    const int64_t c = align256(4 * n_cells);
+    w.cend = c;
+    w.box = 2 * c;
+    w.rec = 3 * c;
+    w.sums = w.rec + align256(rec_bytes * n);
+    w.bytes = w.sums + sum_bytes * (n_cells < n ? n_cells : n);
+    return w;
+}
+
 template <int KIND, typename VT>
 int64_t q_record_bytes() { return QRecord<KIND, VT>::BYTES; }
 
@@ -148,15 +163,16 @@ int assemble_sorted(const LaunchConst &c, const PtrsP &p, const int *perm, const
     const int ncx = c.g.n_grid[0], ncy = c.g.n_grid[1], nc = ncx * ncy;
     // the records written below must fit the caller's workspace (record size
     // of this instantiation, not of another precision)
-    const int64_t need = 2 * align256(4 * (int64_t)nc) + (int64_t)QRecord<KIND, VT>::BYTES * p.n;
-    if (need > ws_bytes) {
+    const AsmParts w = asm_parts(nc, p.n, QRecord<KIND, VT>::BYTES, 8 * CellSums<KIND>::ND);
+    if (w.bytes > ws_bytes) {
         snprintf(g_msg, sizeof(g_msg), "gw_assemble_sorted: workspace of %lld bytes, %lld needed",
-                 (long long)ws_bytes, (long long)need);
+                 (long long)ws_bytes, (long long)w.bytes);
         return GW_EINVAL;
     }
-    int *cstart = (int *)ws;
-    int *cend = (int *)(ws + align256(4 * (int64_t)nc));
-    unsigned char *scratch = (unsigned char *)(ws + 2 * align256(4 * (int64_t)nc));
+    int *cstart = (int *)ws, *cend = (int *)(ws + w.cend), *box = (int *)(ws + w.box);
+    unsigned char *scratch = (unsigned char *)(ws + w.rec);
+    double *sums = (double *)(ws + w.sums);
+    const int by_cell = nc <= p.n;  // the cells' sums by cell, or by their first particle: whichever is fewer
     const int D = KindTraits<KIND>::D, NF = KindTraits<KIND>::NF;
     // algorithmic bytes, each array once: particle state in (x, lp, F_old, b_old,
     // E) and out (F_new, b_new, sigma), the scratch records written and read
@@ -165,19 +181,16 @@ int assemble_sorted(const LaunchConst &c, const PtrsP &p, const int *perm, const
     const double grid = 8.0 * 3 * (double)A->n_rows * NF;
     const double mat = WANT_K ? (double)A->nnzb * NF * NF * sizeof(VT) : 0.0;
     ProfScope ps(PC_ASSEMBLE, s, per_p * p.n + grid + mat);
-    GW_CUDA(cudaMemsetAsync(ws, 0, 2 * align256(4 * (int64_t)nc), s));
+    GW_CUDA(cudaMemsetAsync(ws, 0, w.box, s));  // cells without particles: start = end = 0
     k_cell_ranges<<<gw_count_launch(nblk(p.n, kThreads)), kThreads, 0, s>>>(keys, p.n, nc, cstart, cend);
     GW_LAUNCHED();
     launch_particle_q<KIND, WANT_K, VT>(c, p, perm, un, uo, scratch, force, s);
     GW_LAUNCHED();
-    // nine colour phases in a fixed order
-    for (int ky = 0; ky < 3; ++ky)
-        for (int kx = 0; kx < 3; ++kx) {
-            const int n3 = ((ncx - kx + 2) / 3) * ((ncy - ky + 2) / 3);
-            if (n3 <= 0) continue;
-            k_cell_scatter<KIND, WANT_K, VT><<<gw_count_launch(nblk(n3, kScatterWarps)), 32 * kScatterWarps, 0, s>>>(
-                c, kx, ky, cstart, cend, scratch, fm, a, R);
-        }
+    k_cell_blocks<KIND, WANT_K, VT><<<gw_count_launch(nblk(nc, kCellGroups)), 16 * kCellGroups, 0, s>>>(
+        c, nc, by_cell, cstart, cend, scratch, sums, box);
+    if (A->n_rows > 0)
+        k_row_gather<KIND, WANT_K, VT><<<gw_count_launch(nblk(A->n_rows, kGatherRows)), 32 * kGatherRows, 0, s>>>(
+            c.g, by_cell, cstart, box, sums, fm, a, R);
     GW_LAUNCHED();
     return GW_OK;
 }
@@ -197,8 +210,11 @@ int assemble_sorted_kind(const LaunchConst &c, const PtrsP &p, const int *perm, 
         else
             rc = f64 ? assemble_sorted<KIND, true, double>(c, p, perm, keys, fm, un, uo, A, R, force, a, ws, ws_bytes, s)
                      : assemble_sorted<KIND, true, float>(c, p, perm, keys, fm, un, uo, A, R, force, a, ws, ws_bytes, s);
-        if (rc) return rc;
+        return rc;
     }
+    // no particles: the rows the gather would write are zero, with their identity entries
+    if (A->vals) GW_CUDA(cudaMemsetAsync(A->vals, 0, (prec == GW_PREC_F64 ? 8 : 4) * (size_t)A->nnzb * A->nf * A->nf, s));
+    GW_CUDA(cudaMemsetAsync(R, 0, sizeof(double) * (size_t)A->n_rows * A->nf, s));
     if (A->vals && A->n_rows > 0) {
         if (prec == GW_PREC_F64) k_identity_dirichlet<2, double><<<gw_count_launch(nblk(A->n_rows, kThreads)), kThreads, 0, s>>>(a, fm);
         else k_identity_dirichlet<2, float><<<gw_count_launch(nblk(A->n_rows, kThreads)), kThreads, 0, s>>>(a, fm);
@@ -212,7 +228,8 @@ extern "C" int64_t gw_assemble_workspace_bytes(const gw_grid_t *grid, int32_t n_
     if (!grid || n_particles < 0) return -1;
     if (grid->dim != 2) return 0;  // the 3D kind assembles with atomics and needs no workspace
     const int64_t nc = (int64_t)grid->n_grid[0] * grid->n_grid[1];
-    return 2 * align256(4 * nc) + align256(record_bytes(grid->kind, prec) * (int64_t)n_particles) + 256;
+    const int64_t sum = 8 * (grid->kind == GW_KIND_SOLID2D ? CellSums<GW_KIND_SOLID2D>::ND : CellSums<GW_KIND_COUPLED2D>::ND);
+    return asm_parts(nc, n_particles, record_bytes(grid->kind, prec), sum).bytes;
 }
 
 extern "C" int gw_assemble_sorted(const gw_grid_t *grid, const gw_material_t *mat, const gw_step_t *st,
@@ -237,12 +254,7 @@ extern "C" int gw_assemble_sorted(const gw_grid_t *grid, const gw_material_t *ma
     LaunchConst c = make_lc(grid, mat, st);
     PtrsP p = make_ptrs(*pt);
     PtrsA a = make_ptrs(*A);
-    if (A->vals) {
-        GW_REQUIRE(A->row_ptr && A->cols && A->stencil);
-        const size_t vb = (prec == GW_PREC_F64 ? 8 : 4) * (size_t)A->nnzb * A->nf * A->nf;
-        GW_CUDA(cudaMemsetAsync(A->vals, 0, vb, s));
-    }
-    GW_CUDA(cudaMemsetAsync(R_rows, 0, sizeof(double) * (size_t)A->n_rows * A->nf, s));
+    if (A->vals) GW_REQUIRE(A->row_ptr && A->cols && A->stencil);
     char *ws = (char *)workspace;
     if (grid->kind == GW_KIND_SOLID2D)
         return assemble_sorted_kind<GW_KIND_SOLID2D>(c, p, perm, keys, free_mask, u_new, u_old, A, prec, R_rows, force, a, ws, workspace_bytes, s);

@@ -4,27 +4,32 @@
 // wp.atomic_add per node and field) and of its coloured-AD Jacobian
 // (solvers/sparse_differentiation.py:213-401).
 //
-// Two passes over the particles in cell-sorted order:
+// Three passes:
 //
-//  1. k_particle_q (one thread per particle): kinematics, return map and
-//     stress, written back as F_new / b_new / sigma like the reference, and
-//     the particle's stress resultants Q (FP64) and their derivatives
-//     Dm = dQ/dtheta (FP64, or FP32 in mixed precision) with respect to the
-//     gathered nodal quantities theta (displacement gradient H, ubar, and for
-//     u-p pbar, grad p, dp~).  These go to a scratch record per sorted
-//     particle; there is no scatter in this pass.
+//  1. k_particle_q (one thread per particle, cell-sorted order): kinematics,
+//     return map and stress, written back as F_new / b_new / sigma like the
+//     reference, and the particle's stress resultants Q (FP64) and their
+//     derivatives Dm = dQ/dtheta (FP64, or FP32 in mixed precision) with respect to
+//     the gathered nodal quantities theta (displacement gradient H, ubar, and for
+//     u-p pbar, grad p, dp~).  These go to a scratch record per sorted particle;
+//     there is no scatter in this pass.
 //
-//  2. k_cell_scatter (one warp per occupied cell, nine colour phases): the
-//     particles of one cell share their lower corner, so they touch the same
-//     3 x 3 nodes.  A warp stages each of its cell's records in shared memory
-//     in sorted order and its lanes own the cell's residual entries (slot,
-//     field) and element blocks (slot a, slot b), accumulated in registers
-//     from per-slot columns shared by the warp.  Cells of one colour (cx mod 3, cy mod 3) are
-//     at least three cells apart, so their node sets -- and therefore the
-//     residual rows and matrix rows they touch -- are disjoint: the warp adds
-//     its sums with plain read-modify-writes, without atomics.  The summation
-//     order (phases, cells, particles in sorted order) is fixed, so R and K
-//     are bitwise reproducible from run to run.
+//  2. k_cell_blocks (16 lanes per occupied cell): the particles of one cell share
+//     their lower corner, so they touch the same 3 x 3 nodes.  A lane sums whole
+//     element blocks (slot a, slot b) and residual entries over the cell's
+//     particles in sorted order and leaves them, in FP64, in the cell's buffer.
+//
+//  3. k_row_gather (16 lanes per block row): a row's entries and blocks are the sums
+//     over the up to nine cells that reach its node; it is written once, with its
+//     Dirichlet identity entries.
+//
+// The summation order of a row is fixed (its cells by (cy mod 3, cx mod 3), a cell's
+// particles in sorted order, FP32 blocks rounded after each cell), so R and K are
+// bitwise reproducible.  The former cell scatter kept the order by nine colour
+// phases of cells three apart: nine dependent launches of 8-10 us each however small
+// the problem (640 particles FP64: 79 us), 994 us on 1.03 M particles; the two passes
+// take 9 us and 786 us.  (Rows gathering straight from the records, each read four to
+// nine times: 27 us and 2,135 us.)
 //
 // The residual rows follow residual_rows(): for field j < D
 //   r_a[j] = -sum_k G_a[k] Q_U[k][j] + W_a (Q_S g_j + fx_j) + [j = D-1] W_a Q_PEN,
@@ -39,15 +44,26 @@
 namespace gw {
 namespace {  // internal linkage: each translation unit compiles the kernels it launches
 
-// Scratch record of one sorted particle: doubles x[D], lp[D], Q[NQ], fx[D]
-// (point load and traction per unit weight), then VT Dm[NQ][NT]; padded to 32 bytes.
+// Scratch record of one sorted particle: doubles x[D], lp[D], Q[NQ], fx[D] (point
+// load and traction per unit weight), then VT Dm from a 16-byte boundary; padded to
+// 32 bytes.  The solid kind's only nonzero derivatives are those of Qu with respect
+// to H (4 x 4) and of the footing penalty with respect to ubar (1).
 template <int KIND, typename VT>
 struct QRecord {
     typedef Layout<KIND> L;
     static const int D = KindTraits<KIND>::D;
-    static const int ND = 3 * D + L::NQ;                 // doubles
-    static const int NDM = L::NQ * L::NT;                // tangent entries
+    static const bool UP = KindTraits<KIND>::UP;
+    static const int Q0 = 2 * D, FX = Q0 + L::NQ;
+    static const int ND = (FX + D + 1) / 2 * 2;          // doubles
+    static const int NDM = UP ? L::NQ * L::NT : 17;      // tangent entries
     static const int BYTES = ((ND * 8 + NDM * (int)sizeof(VT)) + 31) / 32 * 32;
+};
+// Sums of one cell, FP64: the blocks (a, b) of its box of ns slots, row a after row a
+// (a row's reader takes ns blocks in a piece), then the slots' residual entries.
+template <int KIND>
+struct CellSums {
+    static const int NF = KindTraits<KIND>::NF;
+    static const int ND = (81 * NF * NF + 9 * NF + 1) / 2 * 2;  // doubles, for the largest box
 };
 
 // sorted keys -> [start, end) of every occupied cell (cells without particles keep start = end = 0)
@@ -98,229 +114,337 @@ __global__ void __launch_bounds__(kThreads) k_particle_q(LaunchConst c, PtrsP p,
     double *rd = (double *)(scratch + (size_t)t * RC::BYTES);
     bool bad = false;
     for (int k = 0; k < D; ++k) {
-        rd[k] = x[k];
-        rd[D + k] = lp[k];
         double f = (p.ext_flag && p.ext_flag[pid]) ? c.st.point_load[k] * ramp : 0.0;
         if (KIND == GW_KIND_COUPLED2D && p.trac_flag && p.trac_flag[pid]) f += c.st.traction[k] * c.g.h[k] / c.st.PPD;
-        rd[2 * D + L::NQ + k] = f;
+        rd[k] = x[k];
+        rd[D + k] = lp[k];
+        rd[RC::FX + k] = f;
     }
     for (int q = 0; q < L::NQ; ++q) {
-        rd[2 * D + q] = ev.Q[q];
+        rd[RC::Q0 + q] = ev.Q[q];
         if (!isfinite(ev.Q[q])) bad = true;
     }
     if (bad) atomicOr(&g_status, ST_NAN);
     if (!WANT_K) return;
     VT *rm = (VT *)(rd + RC::ND);
-    for (int q = 0; q < L::NQ; ++q)
-        for (int tt = 0; tt < L::NT; ++tt) rm[q * L::NT + tt] = (VT)ev.Dm[q][tt];
+    if (RC::UP) {
+        for (int q = 0; q < L::NQ; ++q)
+            for (int tt = 0; tt < L::NT; ++tt) rm[q * L::NT + tt] = (VT)ev.Dm[q][tt];
+    } else {
+        for (int q = 0; q < 4; ++q)
+            for (int tt = 0; tt < 4; ++tt) rm[q * 4 + tt] = (VT)ev.Dm[L::QU + q][L::TH + tt];
+        rm[16] = (VT)ev.Dm[L::QPEN][L::TU];
+    }
 }
 
-// Pass 2: one warp per cell of colour (kx, ky); cells (kx + 3i, ky + 3j).
-// Per particle of the cell (sorted order) the warp stages the record, two
-// lanes evaluate the shape functions of the two axes, nine lanes form the
-// slot weights and the columns C_b[q][g] = dQ_q / du_b[g] of the nine slots in
-// shared memory, and then every lane adds its residual entries and its whole
-// element blocks (a, b) from the shared columns.
-constexpr int kScatterWarps = 4;  // warps per CTA
-template <int KIND, typename VT>
-struct ScatterShared {
-    typedef Layout<KIND> L;
-    static const int NF = KindTraits<KIND>::NF;
-    double W[9], Wavg[9], G[9][2];   // cell-frame slots (0 outside the particle's span)
-    double C[9][L::NQ][NF];          // dQ/du of each slot
-    double axw[2][3], axg[2][3], axa[2][3];
-    int axoff[2], axspan[2];
-    unsigned int inspan;              // bit a: cell slot a lies in the particle's span
-};
+__device__ __forceinline__ void record_row(const float *p, double d[4]) {
+    const float4 v = *reinterpret_cast<const float4 *>(p);
+    d[0] = v.x; d[1] = v.y; d[2] = v.z; d[3] = v.w;
+}
+__device__ __forceinline__ void record_row(const double *p, double d[4]) {
+    const double2 a = reinterpret_cast<const double2 *>(p)[0], b = reinterpret_cast<const double2 *>(p)[1];
+    d[0] = a.x; d[1] = a.y; d[2] = b.x; d[3] = b.y;
+}
 
+// Pass 2: 16 lanes per cell.  The axes of eight particles are evaluated one per
+// lane; then lane l takes block l, l + 16, ... of the cell's box (the union of its
+// particles' spans: 16 blocks where they lie inside one cell, up to 81) and residual
+// entries l, l + 16, one at a time over all the cell's particles, so it holds one
+// block in registers and the SM many cells.  (A cell of more than eight particles
+// evaluates its axes again for each round.)  box[cell]: the box's extents, 0 without
+// particles.
+constexpr int kCellGroups = 8;   // cells per CTA
+constexpr int kCellBatch = 8;
+struct CellAxis {
+    double w[3], g[3], a[3];
+    int off, span;  // corner offset from the cell (a particle clamped at the grid edge), nodes
+};
 template <int KIND, bool WANT_K, typename VT>
-__global__ void __launch_bounds__(32 * kScatterWarps, 6) k_cell_scatter(LaunchConst c, int kx, int ky,
-                                                                     const int *__restrict__ cstart,
-                                                                     const int *__restrict__ cend,
-                                                                     const unsigned char *__restrict__ scratch,
-                                                                     const uint8_t *__restrict__ free_mask, PtrsA A,
-                                                                     double *__restrict__ R) {
+__global__ void __launch_bounds__(16 * kCellGroups) k_cell_blocks(LaunchConst c, int n_cells, int by_cell,
+                                                                  const int *__restrict__ cstart,
+                                                                  const int *__restrict__ cend,
+                                                                  const unsigned char *__restrict__ scratch,
+                                                                  double *__restrict__ sums, int *__restrict__ box) {
     typedef KindTraits<KIND> KT;
     typedef Layout<KIND> L;
     typedef QRecord<KIND, VT> RC;
-    typedef ScatterShared<KIND, VT> SS;
-    static_assert(KT::D == 2, "the cell scatter covers the 2D kinds");
-    const int D = 2, NF = KT::NF, NS = 9;
-    constexpr int NR = NS * NF;             // residual entries of a cell
-    constexpr int NB = NS * NS;             // element blocks of a cell
-    constexpr int PERB = (NB + 31) / 32;    // blocks per lane
-    constexpr int PB = NF == 2 ? 4 : 2;   // particles staged per batch (static shared memory < 48 KB)
-    __shared__ __align__(16) unsigned char rec_sh[kScatterWarps][PB][RC::BYTES];
-    __shared__ SS ssh[kScatterWarps][PB];
-    __shared__ unsigned char inflag[kScatterWarps][PB][NS];
-    const int lane = threadIdx.x & 31, wl = threadIdx.x >> 5;
-    const int ncx = c.g.n_grid[0], ncy = c.g.n_grid[1];
-    const int nx3 = (ncx - kx + 2) / 3, ny3 = (ncy - ky + 2) / 3;
-    const int cw = blockIdx.x * kScatterWarps + wl;
-    if (cw >= nx3 * ny3) return;  // whole warps only: warp-level syncs below
-    const int cx = kx + 3 * (cw % nx3), cy = ky + 3 * (cw / nx3);
-    const int cell = cx + cy * ncx;
+    typedef CellSums<KIND> CS;
+    static_assert(KT::D == 2, "the cell pass covers the 2D kinds");
+    constexpr int D = 2, NF = KT::NF;
+    __shared__ CellAxis axs[kCellGroups][kCellBatch][2];
+    const int lane = threadIdx.x & 15, grp = threadIdx.x >> 4;
+    const int cell = blockIdx.x * kCellGroups + grp;
+    const unsigned gmask = 0xffffu << (threadIdx.x & 16);  // this cell's half of the warp
+    if (cell >= n_cells) return;  // whole groups; group-wide syncs below
     const int p0 = cstart[cell], p1 = cend[cell];
-    if (p1 <= p0) return;
+    if (p1 <= p0) {
+        if (lane == 0) box[cell] = 0;
+        return;
+    }
+    const int ncx = c.g.n_grid[0], cx = cell % ncx, cy = cell / ncx;
     const double ramp = (c.st.current_step + 1.0) / c.st.total_steps;
     const double gv = -c.st.gravity_mag * (c.st.gravity_full ? 1.0 : ramp);
-    double racc = 0.0;
-    double kacc[PERB][NF][NF];
-#pragma unroll
-    for (int e = 0; e < PERB; ++e)
-        for (int f = 0; f < NF; ++f)
-            for (int g = 0; g < NF; ++g) kacc[e][f][g] = 0.0;
-    unsigned int touched = 0u;  // bit e: block e of this lane received a contribution
-    // The cell's particles go in batches of PB: the set-up sections (staging
-    // the records, shape functions, slot weights, columns C_b) run for the
-    // whole batch at once, one (particle, axis / slot) per lane, and the
-    // accumulation then runs over the batch in sorted order, so the sums are
-    // those of one particle at a time.
-    constexpr int NCH = RC::BYTES / 16;
-    for (int t0 = p0; t0 < p1; t0 += PB) {
-        const int np = min(PB, p1 - t0);
-        for (int k = lane; k < np * NCH; k += 32) {
-            const int pp = k / NCH, ch = k % NCH;
-            ((uint4 *)rec_sh[wl][pp])[ch] = ((const uint4 *)(scratch + (size_t)(t0 + pp) * RC::BYTES))[ch];
-        }
-        __syncwarp();
-        if (lane < 2 * np) {  // shape functions: one (particle, axis) per lane
-            const int pp = lane >> 1, k = lane & 1;
-            const double *rd = (const double *)rec_sh[wl][pp];
-            SS &s = ssh[wl][pp];
-            Axis ax;
-            gimp_axis(rd[k], rd[D + k], c.g.h[k], c.g.inv_h[k], ax);
-            for (int i = 0; i < 3; ++i) { s.axw[k][i] = ax.w[i]; s.axg[k][i] = ax.gw[i]; s.axa[k][i] = ax.wavg[i]; }
-            s.axoff[k] = ax.lower - (k == 0 ? cx : cy);
-            s.axspan[k] = ax.span;
-        }
-        __syncwarp();
-        for (int k = lane; k < np * NS; k += 32) {  // cell slot weights (a particle clamped at the grid edge is offset)
-            const int pp = k / NS, sl = k % NS;
-            SS &s = ssh[wl][pp];
-            const int i0 = sl % 3 - s.axoff[0], i1 = sl / 3 - s.axoff[1];
-            const bool in = i0 >= 0 && i0 < s.axspan[0] && i1 >= 0 && i1 < s.axspan[1];
-            const double w0 = in ? s.axw[0][i0] : 0.0, w1 = in ? s.axw[1][i1] : 0.0;
-            s.W[sl] = w0 * w1;
-            s.Wavg[sl] = in ? s.axa[0][i0] * s.axa[1][i1] : 0.0;
-            s.G[sl][0] = in ? s.axg[0][i0] * w1 : 0.0;
-            s.G[sl][1] = in ? w0 * s.axg[1][i1] : 0.0;
-            inflag[wl][pp][sl] = in;
-        }
-        __syncwarp();
-        if (lane < np) {
-            unsigned int bits = 0u;
-            for (int sl = 0; sl < NS; ++sl) bits |= (unsigned int)inflag[wl][lane][sl] << sl;
-            ssh[wl][lane].inspan = bits;
-        }
-        __syncwarp();
-        if (WANT_K)
-            for (int k = lane; k < np * NS; k += 32) {  // columns of slot b of particle pp
-                const int pp = k / NS, b = k % NS;
-                SS &s = ssh[wl][pp];
-                if (!((s.inspan >> b) & 1u)) continue;
-                const VT *Dm = (const VT *)((const double *)rec_sh[wl][pp] + RC::ND);
-                const double Wb = s.W[b], Gb0 = s.G[b][0], Gb1 = s.G[b][1];
-                for (int q = 0; q < L::NQ; ++q) {
-                    const VT *dq = Dm + q * L::NT;
-                    s.C[b][q][0] = (double)dq[L::TH + 0] * Gb0 + (double)dq[L::TH + D] * Gb1;
-                    s.C[b][q][1] = (double)dq[L::TH + 1] * Gb0 + (double)dq[L::TH + D + 1] * Gb1 + (double)dq[L::TU] * Wb;
-                    if (NF > D)
-                        s.C[b][q][NF - 1] = (double)dq[L::TP] * Wb + (double)dq[L::TD] * (Wb - s.Wavg[b]) +
-                                            (double)dq[L::TG] * Gb0 + (double)dq[L::TG + 1] * Gb1;
-                }
-            }
-        __syncwarp();
-        for (int pp = 0; pp < np; ++pp) {
-            const SS &s = ssh[wl][pp];
-            const double *rd = (const double *)rec_sh[wl][pp];
-            const double *Q = rd + 2 * D;
-            const double *fx = rd + 2 * D + L::NQ;
-            if (lane < NR) {  // residual entry (slot a, field f)
-                const int a = lane / NF, f = lane % NF;
-                if ((s.inspan >> a) & 1u) {
-                    const double Wa = s.W[a];
-                    double v;
-                    if (f < D) {
-                        v = -(s.G[a][0] * Q[L::QU + f] + s.G[a][1] * Q[L::QU + D + f]);
-                        v += Wa * (Q[L::QS] * (f == D - 1 ? gv : 0.0) + fx[f]);
-                        if (f == D - 1) v += Wa * Q[L::QPEN];
-                    } else {
-                        v = Wa * Q[L::QM1] + (Wa - s.Wavg[a]) * Q[L::QM3] + s.G[a][0] * Q[L::QM2] + s.G[a][1] * Q[L::QM2 + 1];
-                    }
-                    racc += v;
-                }
-            }
-            if (WANT_K) {
-#pragma unroll
-                for (int e = 0; e < PERB; ++e) {
-                    const int blk = lane + 32 * e;
-                    if (blk >= NB) break;
-                    const int a = blk / NS, b = blk % NS;
-                    if (!((s.inspan >> a) & 1u) || !((s.inspan >> b) & 1u)) continue;
-                    const double Wa = s.W[a], Ga0 = s.G[a][0], Ga1 = s.G[a][1];
-#pragma unroll
-                    for (int g = 0; g < NF; ++g) {
-#pragma unroll
-                        for (int f = 0; f < D; ++f) {
-                            double v = -(Ga0 * s.C[b][L::QU + f][g] + Ga1 * s.C[b][L::QU + D + f][g]);
-                            if (f == D - 1) v += Wa * gv * s.C[b][L::QS][g] + Wa * s.C[b][L::QPEN][g];
-                            kacc[e][f][g] -= v;
-                        }
-                        if (NF > D) {
-                            const double v = Wa * s.C[b][L::QM1][g] + (Wa - s.Wavg[a]) * s.C[b][L::QM3][g] +
-                                             Ga0 * s.C[b][L::QM2][g] + Ga1 * s.C[b][L::QM2 + 1][g];
-                            kacc[e][NF - 1][g] -= v;
-                        }
-                    }
-                    touched |= 1u << e;
-                }
-            }
-        }
-        __syncwarp();  // the next batch reuses the staging buffers
+    auto axes = [&](int t0) {  // axes of the batch from t0 into shared memory; the extent of this lane's
+        const int pp = lane >> 1, k = lane & 1;
+        if (t0 + pp >= p1) return 0;
+        const double *rd = (const double *)(scratch + (size_t)(t0 + pp) * RC::BYTES);
+        Axis ax;
+        gimp_axis(rd[k], rd[D + k], c.g.h[k], c.g.inv_h[k], ax);
+        CellAxis &o = axs[grp][pp][k];
+        for (int i = 0; i < 3; ++i) { o.w[i] = ax.w[i]; o.g[i] = ax.gw[i]; o.a[i] = ax.wavg[i]; }
+        o.off = ax.lower - (k == 0 ? cx : cy);
+        o.span = ax.span;
+        return min(3, max(0, o.off + o.span));
+    };
+    int e0 = 0, e1 = 0;
+    for (int t0 = p0; t0 < p1; t0 += kCellBatch) {
+        const int e = axes(t0);
+        if (lane & 1) e1 = max(e1, e);
+        else e0 = max(e0, e);
     }
-    // exclusive writes: no other cell of this colour touches these rows
-    if (lane < NR) {
-        const int ac = lane / NF, f = lane % NF;
-        const int nxi = cx + ac % 3, nyi = cy + ac / 3;
-        if (nxi <= ncx && nyi <= ncy) {
-            const int node = nxi + nyi * (ncx + 1);
-            const uint8_t fm = free_mask[node];
-            if ((fm >> f) & 1) {
-                const int row = A.node2row[node];
-                if (in_range(row, A.n_rows, GS_ASSEMBLE)) {
-                    if (!isfinite(racc)) atomicOr(&g_status, ST_NAN);
-                    R[(size_t)row * NF + f] += racc;
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1) {
+        e0 = max(e0, __shfl_xor_sync(gmask, e0, o, 16));
+        e1 = max(e1, __shfl_xor_sync(gmask, e1, o, 16));
+    }
+    const int ns = e0 * e1, nb = ns * ns;
+    const bool one = p1 - p0 <= kCellBatch;  // the axes of the only batch are in place
+    const float ins = 1.0f / (float)max(ns, 1), ie0 = 1.0f / (float)max(e0, 1);  // exact quotients of small integers below
+    double *const out = sums + (size_t)(by_cell ? cell : p0) * CS::ND;
+    __syncwarp(gmask);
+
+    for (int q0 = 0; q0 < ns * NF; q0 += 16) {  // residual entries (slot a, field f)
+        const int q = q0 + lane, a = q / NF, f = q % NF;
+        const int ay = (int)(((float)a + 0.5f) * ie0), ax = a - ay * e0;
+        double racc = 0.0;
+        for (int t0 = p0; t0 < p1; t0 += kCellBatch) {
+            if (!one) {
+                __syncwarp(gmask);
+                axes(t0);
+                __syncwarp(gmask);
+            }
+            const int np = q < ns * NF ? min(kCellBatch, p1 - t0) : 0;
+            for (int pp = 0; pp < np; ++pp) {
+                const CellAxis &X = axs[grp][pp][0], &Y = axs[grp][pp][1];
+                const int a0 = ax - X.off, a1 = ay - Y.off;
+                if ((unsigned)a0 >= (unsigned)X.span || (unsigned)a1 >= (unsigned)Y.span) continue;
+                const double *rd = (const double *)(scratch + (size_t)(t0 + pp) * RC::BYTES);
+                const double *Q = rd + RC::Q0;
+                const double Wa = X.w[a0] * Y.w[a1], Ga0 = X.g[a0] * Y.w[a1], Ga1 = X.w[a0] * Y.g[a1];
+                double v;
+                if (f < D) {
+                    v = -(Ga0 * Q[L::QU + f] + Ga1 * Q[L::QU + D + f]);
+                    v += Wa * (Q[L::QS] * (f == D - 1 ? gv : 0.0) + rd[RC::FX + f]);
+                    if (f == D - 1) v += Wa * Q[L::QPEN];
+                } else {
+                    const double Waa = X.a[a0] * Y.a[a1];
+                    v = Wa * Q[L::QM1] + (Wa - Waa) * Q[L::QM3] + Ga0 * Q[L::QM2] + Ga1 * Q[L::QM2 + 1];
                 }
+                racc += v;
             }
         }
+        if (q < ns * NF) out[nb * NF * NF + q] = racc;
+    }
+    if (WANT_K)
+        for (int q0 = 0; q0 < nb; q0 += 16) {
+            const int q = q0 + lane;
+            const int a = (int)(((float)q + 0.5f) * ins), b = q - a * ns;
+            const int ay = (int)(((float)a + 0.5f) * ie0), ax = a - ay * e0;
+            const int by = (int)(((float)b + 0.5f) * ie0), bx = b - by * e0;
+            double kacc[NF][NF];
+#pragma unroll
+            for (int f = 0; f < NF; ++f)
+#pragma unroll
+                for (int g = 0; g < NF; ++g) kacc[f][g] = 0.0;
+            for (int t0 = p0; t0 < p1; t0 += kCellBatch) {
+                if (!one) {
+                    __syncwarp(gmask);
+                    axes(t0);
+                    __syncwarp(gmask);
+                }
+                const int np = q < nb ? min(kCellBatch, p1 - t0) : 0;
+                for (int pp = 0; pp < np; ++pp) {
+                    const CellAxis &X = axs[grp][pp][0], &Y = axs[grp][pp][1];
+                    const int xo = X.off, xs = X.span, yo = Y.off, ys = Y.span;
+                    const int a0 = ax - xo, a1 = ay - yo, b0 = bx - xo, b1 = by - yo;
+                    if ((unsigned)a0 >= (unsigned)xs || (unsigned)a1 >= (unsigned)ys || (unsigned)b0 >= (unsigned)xs ||
+                        (unsigned)b1 >= (unsigned)ys)
+                        continue;
+                    const VT *Dm = (const VT *)((const double *)(scratch + (size_t)(t0 + pp) * RC::BYTES) + RC::ND);
+                    const double Wa = X.w[a0] * Y.w[a1], Ga0 = X.g[a0] * Y.w[a1], Ga1 = X.w[a0] * Y.g[a1];
+                    const double Wb = X.w[b0] * Y.w[b1], Gb0 = X.g[b0] * Y.w[b1], Gb1 = X.w[b0] * Y.g[b1];
+                    if (!RC::UP) {
+                        double C[4][2];  // dQu / du_b
+#pragma unroll
+                        for (int u = 0; u < 4; ++u) {
+                            double d[4];
+                            record_row(Dm + u * 4, d);
+                            C[u][0] = d[0] * Gb0 + d[D] * Gb1;
+                            C[u][1] = d[1] * Gb0 + d[D + 1] * Gb1;
+                        }
+#pragma unroll
+                        for (int g = 0; g < 2; ++g)
+#pragma unroll
+                            for (int f = 0; f < 2; ++f) {
+                                double v = -(Ga0 * C[f][g] + Ga1 * C[D + f][g]);
+                                if (f == 1 && g == 1) v += Wa * ((double)Dm[16] * Wb);
+                                kacc[f][g] -= v;
+                            }
+                    } else {
+                        const double Waa = X.a[a0] * Y.a[a1], Wbb = X.a[b0] * Y.a[b1];
+                        double C[L::NQ][NF];
+#pragma unroll
+                        for (int u = 0; u < L::NQ; ++u) {
+                            const VT *dq = Dm + u * L::NT;
+                            C[u][0] = (double)dq[L::TH + 0] * Gb0 + (double)dq[L::TH + D] * Gb1;
+                            C[u][1] = (double)dq[L::TH + 1] * Gb0 + (double)dq[L::TH + D + 1] * Gb1 + (double)dq[L::TU] * Wb;
+                            C[u][NF - 1] = (double)dq[L::TP] * Wb + (double)dq[L::TD] * (Wb - Wbb) + (double)dq[L::TG] * Gb0 +
+                                           (double)dq[L::TG + 1] * Gb1;
+                        }
+#pragma unroll
+                        for (int g = 0; g < NF; ++g) {
+#pragma unroll
+                            for (int f = 0; f < D; ++f) {
+                                double v = -(Ga0 * C[L::QU + f][g] + Ga1 * C[L::QU + D + f][g]);
+                                if (f == D - 1) v += Wa * gv * C[L::QS][g] + Wa * C[L::QPEN][g];
+                                kacc[f][g] -= v;
+                            }
+                            const double v = Wa * C[L::QM1][g] + (Wa - Waa) * C[L::QM3][g] + Ga0 * C[L::QM2][g] + Ga1 * C[L::QM2 + 1][g];
+                            kacc[NF - 1][g] -= v;
+                        }
+                    }
+                }
+            }
+            if (q < nb) {
+                double *d = out + q * NF * NF;
+#pragma unroll
+                for (int f = 0; f < NF; ++f)
+#pragma unroll
+                    for (int g = 0; g < NF; ++g) d[f * NF + g] = kacc[f][g];
+            }
+        }
+    if (lane == 0) box[cell] = e0 | e1 << 2;
+}
+
+template <int N>
+__device__ __forceinline__ void load_rw_blk(const double *p, double v[N]) {
+    if constexpr (N % 2 == 0) {
+#pragma unroll
+        for (int q = 0; q < N / 2; ++q) {
+            const double2 t = reinterpret_cast<const double2 *>(p)[q];
+            v[2 * q] = t.x; v[2 * q + 1] = t.y;
+        }
+    } else {
+#pragma unroll
+        for (int q = 0; q < N; ++q) v[q] = p[q];
+    }
+}
+
+// Pass 3: a warp per block row.  Lane t < 25 sums the block at stencil bit t, lanes
+// 25 .. 25 + NF - 1 the residual fields, over the cells that reach the node.
+constexpr int kGatherRows = 8;  // rows per CTA
+template <int KIND, bool WANT_K, typename VT>
+__global__ void __launch_bounds__(32 * kGatherRows) k_row_gather(gw_grid_t grid, int by_cell,
+                                                                 const int *__restrict__ cstart,
+                                                                 const int *__restrict__ box,
+                                                                 const double *__restrict__ sums,
+                                                                 const uint8_t *__restrict__ free_mask, PtrsA A,
+                                                                 double *__restrict__ R) {
+    typedef CellSums<KIND> CS;
+    constexpr int NF = CS::NF, BB = NF * NF;
+    const int lane = threadIdx.x & 31;
+    const int r = blockIdx.x * kGatherRows + (threadIdx.x >> 5);
+    const int ncx = grid.n_grid[0], ncy = grid.n_grid[1];
+    if (r >= A.n_rows) return;  // whole warps
+    const int node = A.row2node[r];
+    if (!in_range(node, grid.n_nodes, GS_ASSEMBLE)) return;
+    const int nx = node % (ncx + 1), ny = node / (ncx + 1);
+    const unsigned fa = free_mask[node];
+    // lanes 0-8: the cell of each (cx mod 3, cy mod 3) that reaches this node, in the order of the sums
+    int slot = 0, info = 0;  // info: box extents, and this node's slot (ax, ay)
+    if (lane < 9) {
+        const int kx = lane % 3, ky = lane / 3;
+        const int cx = nx - (nx - kx + 3) % 3, cy = ny - (ny - ky + 3) % 3;
+        if (cx >= 0 && cx < ncx && cy >= 0 && cy < ncy) {
+            const int cell = cx + cy * ncx, b = box[cell], ax = nx - cx, ay = ny - cy;
+            if (ax < (b & 3) && ay < (b >> 2)) {
+                info = b | ax << 4 | ay << 6;
+                slot = by_cell ? cell : cstart[cell];
+            }
+        }
+    }
+    const int ox = lane % 5 - 2, oy = lane / 5 - 2;
+    // what the end needs, loaded ahead of the sums
+    const unsigned st = WANT_K ? A.stencil[node] : 0u;
+    const int base = WANT_K ? A.row_ptr[r] : 0;
+    const int jx = nx + ox, jy = ny + oy;
+    unsigned fb = 0u;
+    if (WANT_K && lane < 25 && jx >= 0 && jx <= ncx && jy >= 0 && jy <= ncy) fb = free_mask[jx + jy * (ncx + 1)];
+    VT blk[WANT_K ? BB : 1];
+#pragma unroll
+    for (int q = 0; q < (WANT_K ? BB : 1); ++q) blk[q] = (VT)0;
+    double rsum = 0.0;
+    // the cells that reach the node (four where particles stay inside their cells, up
+    // to nine), four at a time with their values in flight
+    unsigned left = __ballot_sync(0xffffffffu, info != 0);
+    while (left) {
+        constexpr int M = 4;
+        double v[M][WANT_K ? BB : 1], rv[M];
+        bool on[M];
+#pragma unroll
+        for (int o = 0; o < M; ++o) {
+            on[o] = false;
+            rv[o] = 0.0;
+            const int from = left ? __ffs(left) - 1 : 0;
+            const int in = __shfl_sync(0xffffffffu, info, from), sl = __shfl_sync(0xffffffffu, slot, from);
+            if (!left) continue;  // uniform
+            left &= left - 1u;
+            const int ax = in >> 4 & 3, ay = in >> 6, bx = ax + ox, by = ay + oy;
+            const int e0 = in & 3, e1 = in >> 2 & 3, ns = e0 * e1, a = ax + e0 * ay;
+            const double *src = sums + (size_t)sl * CS::ND;
+            if (lane >= 25) {
+                if (lane < 25 + NF) rv[o] = src[ns * ns * BB + a * NF + lane - 25];
+            } else if (WANT_K && bx >= 0 && by >= 0 && bx < e0 && by < e1) {
+                on[o] = true;
+                load_rw_blk<WANT_K ? BB : 1>(src + (a * ns + bx + e0 * by) * BB, v[o]);
+            }
+        }
+#pragma unroll
+        for (int o = 0; o < M; ++o) {
+            rsum += rv[o];
+            if (WANT_K && on[o])
+#pragma unroll
+                for (int q = 0; q < (WANT_K ? BB : 1); ++q) blk[q] = (VT)((double)blk[q] + v[o][q]);
+        }
+    }
+    if (lane >= 25) {
+        if (lane < 25 + NF) {
+            const int f = lane - 25;
+            const bool free = (fa >> f) & 1u;
+            if (free && !isfinite(rsum)) atomicOr(&g_status, ST_NAN);
+            R[(size_t)r * NF + f] = free ? rsum : 0.0;
+        }
+        return;
     }
     if (!WANT_K) return;
-    VT *vals = (VT *)A.vals;
+    if (!((st >> lane) & 1u)) {  // a contribution outside the pattern, or no diagonal block
+        bool any = lane == 12;
 #pragma unroll
-    for (int e = 0; e < PERB; ++e) {
-        if (!((touched >> e) & 1u)) continue;
-        const int blk = lane + 32 * e;
-        const int ac = blk / NS, bc = blk % NS;
-        const int ax = cx + ac % 3, ay = cy + ac / 3, bx = cx + bc % 3, by = cy + bc / 3;
-        if (ax > ncx || ay > ncy || bx > ncx || by > ncy) continue;
-        const int na = ax + ay * (ncx + 1), nb = bx + by * (ncx + 1);
-        const uint8_t fa = free_mask[na], fb = free_mask[nb];
-        if (!fa || !fb) continue;
-        const int row = A.node2row[na];
-        if (!in_range(row, A.n_rows, GS_ASSEMBLE)) continue;
-        const int o[3] = {bx - ax, by - ay, 0};
-        const int slot = stencil_slot(A.stencil, A.mw, na, offset_bit<2>(o));
-        if (slot < 0) { atomicOr(&g_status, ST_RANGE); continue; }
-        const long long jb = (long long)A.row_ptr[row] + slot;
-        if (!in_range(jb, A.nnzb, GS_ASSEMBLE)) continue;
-        VT *dst = vals + (size_t)jb * NF * NF;
-#pragma unroll
-        for (int f = 0; f < NF; ++f)
-#pragma unroll
-            for (int g = 0; g < NF; ++g)
-                if (((fa >> f) & 1) && ((fb >> g) & 1)) dst[f * NF + g] = (VT)((double)dst[f * NF + g] + kacc[e][f][g]);
+        for (int q = 0; q < (WANT_K ? BB : 1); ++q) any = any || (fa && blk[q] != (VT)0);
+        if (any) atomicOr(&g_status, ST_RANGE);
+        return;
     }
+    const long long jb = (long long)base + __popc(st & ((1u << lane) - 1u));
+    if (!in_range(jb, A.nnzb, GS_ASSEMBLE)) return;
+    VT *dst = (VT *)A.vals + (size_t)jb * BB;
+#pragma unroll
+    for (int f = 0; f < NF; ++f)
+#pragma unroll
+        for (int g = 0; g < NF; ++g) {
+            VT v = (((fa >> f) & 1u) && ((fb >> g) & 1u)) ? blk[WANT_K ? f * NF + g : 0] : (VT)0;
+            if (lane == 12 && f == g && !((fa >> f) & 1u)) v = (VT)1;  // Dirichlet DOF: identity row
+            dst[f * NF + g] = v;
+        }
 }
 
 }  // namespace

@@ -258,10 +258,9 @@ int gw_assemble(const gw_grid_t *grid, const gw_material_t *mat, const gw_step_t
  * replacement of the same reference kernels without atomic scatter.  A
  * particle pass (cell-sorted order, perm and the sorted keys of
  * gw_cell_sort) evaluates each particle's stress resultants and their
- * derivatives into workspace records; then one warp per occupied cell sums
- * its particles' contributions in sorted order into R_rows and A->vals, in
- * nine colour phases of cells three apart (disjoint node sets: plain
- * read-modify-writes, no atomics).  Arguments as gw_assemble plus keys (sorted
+ * derivatives into workspace records; then every block row sums the
+ * contributions of the cells that reach it, in a fixed order of cells and
+ * particles, and is written once (no atomics).  Arguments as gw_assemble plus keys (sorted
  * cell keys), workspace (256-byte aligned) of gw_assemble_workspace_bytes;
  * the 3D kind falls back to gw_assemble (atomic scatter) and needs no
  * workspace.  The footing force is still accumulated atomically. */
