@@ -226,11 +226,7 @@ int gmres(const gw_bsr_t *A, int precond, const double *b, double *x, double rto
     G.sc = (GScalars *)w;
     G.x = x; G.b = b; G.n = (size_t)n;
     const size_t head = offsetof(GScalars, H);
-    GW_CUDA(cudaMemsetAsync(G.sc, 0, head, s));
-    struct { int max_iter, restart; } lim = {max_iter, restart};
-    GW_CUDA(cudaMemcpyAsync(&G.sc->max_iter, &lim, sizeof(lim), cudaMemcpyHostToDevice, s));
-    const double eta2 = ::pow(10.0, -0.1 * g_tune[GW_TUNE_GS_CANCEL]);
-    GW_CUDA(cudaMemcpyAsync(&G.sc->gs_eta2, &eta2, sizeof(double), cudaMemcpyHostToDevice, s));
+    k_gm_begin<<<gw_count_launch(1), 32, 0, s>>>(G.sc, max_iter, restart, ::pow(10.0, -0.1 * g_tune[GW_TUNE_GS_CANCEL]));
     const int D = (A->mask_words == 1) ? 2 : 3;
     k_precond_setup<NF, VT><<<gw_count_launch(nblk(nr, kThreads)), kThreads, 0, s>>>(a, D, precond, G.Minv);
     GW_LAUNCHED();
@@ -313,7 +309,8 @@ int gmres(const gw_bsr_t *A, int precond, const double *b, double *x, double rto
     *iters = h.iters;
     g_last_reorths = h.reorths;
     *relres = (h.bnorm > 0.0) ? h.resid / h.bnorm : 0.0;
-    const int gc = guard_check(s, "GMRES");
+    // the header carries the guard of every kernel up to the last residual
+    const int gc = (h.guard || h.status) ? guard_check(s, "GMRES") : GW_OK;
     if (gc) return gc;
     if (h.status == ST_NAN) return GW_ENAN;
     if (h.resid > h.tol) return GW_ENOCONV;
@@ -399,6 +396,7 @@ struct MgHier {
     MgLevel lv[kMgMaxLevels];
     double *dM = nullptr, *dInv = nullptr;
     int dn = 0;
+    int *counts = nullptr;  // pattern phase: row and block counts of the levels, the index guard
     unsigned char *timg = nullptr;  // 2D: shared-memory images of the fused tail
 };
 
@@ -483,6 +481,7 @@ void mg_carve_hier(Bump &bp, MgHier &h, const gw_grid_t &g0, int64_t n_rows0, in
     h.nl = l + 1;  // upper bound; the plan may stop earlier
     h.dM = (double *)bp.take(8 * (int64_t)kMgCoarseMax * kMgCoarseMax);
     h.dInv = (double *)bp.take(8 * (int64_t)kMgCoarseMax * kMgCoarseMax);
+    h.counts = (int *)bp.take(4 * (kMgMaxLevels + 1));
     if (D == 2) h.timg = (unsigned char *)bp.take((int64_t)kTailSmem * kTailMaxCluster);
 }
 void mg_carve_flex(Bump &bp, FlexVecs &fv, int64_t n0, int restart) {
@@ -503,14 +502,28 @@ int64_t mg_ws_bytes(const gw_grid_t &g0, int64_t n_rows, int nf, int restart) {
 }
 
 // Pattern phase: the coarse active sets, row maps, stencils, row pointers and
-// columns of every level below A0 (two host reads per coarse level: its row
-// count and its block count).  Depends on A0's pattern only.
+// columns of every level below A0 (two host reads: the levels' row counts, then
+// their block counts with the index guard).  Depends on A0's pattern only.
 template <int NF>
 int mg_pattern(MgHier &h, const gw_bsr_t *A0, gw_mg_plan_t *plan, cudaStream_t s) {
     const int D = h.lv[0].g.dim, mw = D == 2 ? 1 : 4;
     const int nl_bound = h.nl;
     h.lv[0].L = lat_of(h.lv[0].g);
     h.lv[0].A = *A0;
+    // active nodes and row counts of every level, read once
+    GW_CUDA(cudaMemsetAsync(h.counts, 0, 4 * kMgMaxLevels, s));
+    for (int q = 0; q + 1 < nl_bound; ++q) {
+        MgLevel &f = h.lv[q], &c = h.lv[q + 1];
+        c.L = lat_of(c.g);
+        k_mg_coarse_flags<<<gw_count_launch(nblk(c.g.n_nodes, kThreads)), kThreads, 0, s>>>(
+            f.L, q == 0 ? (const int *)f.A.node2row : nullptr, q == 0 ? nullptr : f.flags, c.L, c.flags, h.counts + q + 1);
+    }
+    GW_LAUNCHED();
+    int counts[kMgMaxLevels + 1] = {0};
+    if (A0->n_rows * NF > g_tune[GW_TUNE_MG_COARSE]) {
+        GW_CUDA(cudaMemcpyAsync(counts, h.counts, 4 * nl_bound, cudaMemcpyDeviceToHost, s));
+        GW_CUDA(cudaStreamSynchronize(s));
+    }
     int l = 0;
     while (h.lv[l].A.n_rows * NF > g_tune[GW_TUNE_MG_COARSE]) {
         if (l + 1 >= nl_bound) {
@@ -518,27 +531,19 @@ int mg_pattern(MgHier &h, const gw_bsr_t *A0, gw_mg_plan_t *plan, cudaStream_t s
             return GW_EINVAL;
         }
         MgLevel &f = h.lv[l], &c = h.lv[l + 1];
-        c.L = lat_of(c.g);
-        const int N = c.g.n_nodes;
+        const int N = c.g.n_nodes, nrc = counts[l + 1];
         PtrsA fa = make_ptrs(f.A);
-        GW_CUDA(cudaMemsetAsync(c.flags, 0, N, s));
-        k_mg_coarse_flags<<<gw_count_launch(nblk(f.A.n_rows, kThreads)), kThreads, 0, s>>>(f.L, fa, c.L, c.flags);
+        if (nrc <= 0 || nrc > N) {
+            snprintf(g_msg, sizeof(g_msg), "multigrid: empty coarse level");
+            return GW_EINVAL;
+        }
         k_flags_to_int<<<gw_count_launch(nblk(N, kThreads)), kThreads, 0, s>>>(c.flags, N, c.tmp);
         GW_LAUNCHED();
-        GW_CUDA(cudaMemcpyAsync(c.sws, c.tmp + (N - 1), 4, cudaMemcpyDeviceToDevice, s));
         int rc = scan_exclusive(c.tmp, c.tmp, N, c.sws + 64, s);
         if (rc) return rc;
         k_compact<<<gw_count_launch(nblk(N, kThreads)), kThreads, 0, s>>>(c.flags, c.tmp, N, NF, nullptr,
                                                                           (int *)c.A.node2row, (int *)c.A.row2node, nullptr);
-        k_add2<<<gw_count_launch(1), 32, 0, s>>>(c.tmp + (N - 1), c.sws, c.sws + 1);
         GW_LAUNCHED();
-        int nrc = 0;
-        GW_CUDA(cudaMemcpyAsync(&nrc, c.sws + 1, 4, cudaMemcpyDeviceToHost, s));
-        GW_CUDA(cudaStreamSynchronize(s));
-        if (nrc <= 0) {
-            snprintf(g_msg, sizeof(g_msg), "multigrid: empty coarse level");
-            return GW_EINVAL;
-        }
         GW_CUDA(cudaMemsetAsync((void *)c.A.stencil, 0, 4 * (size_t)N * mw, s));
         GW_CUDA(cudaMemsetAsync(c.tmp, 0, 4 * ((size_t)nrc + 1), s));
         if (D == 2)
@@ -550,17 +555,14 @@ int mg_pattern(MgHier &h, const gw_bsr_t *A0, gw_mg_plan_t *plan, cudaStream_t s
         GW_LAUNCHED();
         rc = scan_exclusive(c.tmp, (int *)c.A.row_ptr, nrc + 1, c.sws, s);
         if (rc) return rc;
-        int nnzb = 0;
-        GW_CUDA(cudaMemcpyAsync(&nnzb, c.A.row_ptr + nrc, 4, cudaMemcpyDeviceToHost, s));
-        GW_CUDA(cudaStreamSynchronize(s));
         c.A.n_rows = nrc;
         c.A.nf = NF;
-        c.A.nnzb = nnzb;
+        c.A.nnzb = N * (D == 2 ? 25 : 125);  // its capacity, until the block counts are read below
         c.A.mask_words = mw;
         PtrsA ca = make_ptrs(c.A);
         if (D == 2) k_pattern_fill<2><<<gw_count_launch(nblk(nrc, kThreads)), kThreads, 0, s>>>(c.g, ca, (int *)c.A.cols);
         else k_pattern_fill<3><<<gw_count_launch(nblk(nrc, kThreads)), kThreads, 0, s>>>(c.g, ca, (int *)c.A.cols);
-        k_mg_blockrow<<<gw_count_launch(nblk(nrc, kThreads)), kThreads, 0, s>>>(c.A.row_ptr, nrc, nnzb, c.blockrow);
+        k_mg_blockrow<<<gw_count_launch(nblk(nrc, kThreads)), kThreads, 0, s>>>(c.A.row_ptr, nrc, c.A.nnzb, c.blockrow);
         if (D == 2) {
             k_mg_children<2><<<gw_count_launch(nblk(nrc, kThreads)), kThreads, 0, s>>>(f.L, fa, c.L, ca, c.child);
             k_mg_parents<2><<<gw_count_launch(nblk(f.A.n_rows, kThreads)), kThreads, 0, s>>>(f.L, fa, c.L, ca, f.parent);
@@ -581,6 +583,22 @@ int mg_pattern(MgHier &h, const gw_bsr_t *A0, gw_mg_plan_t *plan, cudaStream_t s
                 make_ptrs(v.A), lpr, v.strips, v.scols);
             GW_LAUNCHED();
         }
+    MgTotals tot;
+    memset(&tot, 0, sizeof(tot));
+    tot.n = h.nl;
+    for (int q = 0; q < h.nl; ++q) {
+        tot.row_ptr[q] = h.lv[q].A.row_ptr;
+        tot.n_rows[q] = h.lv[q].A.n_rows;
+    }
+    k_mg_totals<<<gw_count_launch(1), 32, 0, s>>>(tot, h.counts);
+    GW_LAUNCHED();
+    GW_CUDA(cudaMemcpyAsync(counts, h.counts, 4 * (kMgMaxLevels + 1), cudaMemcpyDeviceToHost, s));
+    GW_CUDA(cudaStreamSynchronize(s));
+    for (int q = 1; q < h.nl; ++q) h.lv[q].A.nnzb = counts[q];
+    if (counts[kMgMaxLevels]) {  // an index guard failed
+        const int gc = guard_check(s, "multigrid plan");
+        if (gc) return gc;
+    }
     memset(plan, 0, sizeof(*plan));
     plan->levels = h.nl;
     plan->dense_n = h.dn;
@@ -1251,11 +1269,7 @@ int gmres_mg(const gw_grid_t *grid, const gw_bsr_t *A, gw_mg_plan_t *plan_in, co
     G.x = x; G.b = b; G.n = (size_t)n;
     G.z = nullptr;
     const size_t head = offsetof(GScalars, H);
-    GW_CUDA(cudaMemsetAsync(G.sc, 0, head, s));
-    struct { int max_iter, restart; } lim = {max_iter, restart};
-    GW_CUDA(cudaMemcpyAsync(&G.sc->max_iter, &lim, sizeof(lim), cudaMemcpyHostToDevice, s));
-    const double eta2 = ::pow(10.0, -0.1 * g_tune[GW_TUNE_GS_CANCEL]);
-    GW_CUDA(cudaMemcpyAsync(&G.sc->gs_eta2, &eta2, sizeof(double), cudaMemcpyHostToDevice, s));
+    k_gm_begin<<<gw_count_launch(1), 32, 0, s>>>(G.sc, max_iter, restart, ::pow(10.0, -0.1 * g_tune[GW_TUNE_GS_CANCEL]));
     const int gr = red_grid_rows(nr), gv = red_grid_elems(n);
     const VecRef z{fv.Z, (size_t)n};
     const int *skip = &G.sc->cycle_done;
@@ -1269,22 +1283,31 @@ int gmres_mg(const gw_grid_t *grid, const gw_bsr_t *A, gw_mg_plan_t *plan_in, co
         GW_LAUNCHED();
         mg_step_tail<NF, VT>(h, G, z, 1, skip, s);
         GW_LAUNCHED();
+        // the first cycle of a plan that has solved before queues its steps at once:
+        // from a zero start |r| / tol is 1 / rtol, and a wrong guess costs steps that
+        // return at once
+        const bool ahead = first && plan_in && plan_in->last_rate > 0 && rtol > 0.0 && rtol < 1.0;
         first = 0;
-        GW_CUDA(cudaMemcpyAsync(&hs, G.sc, head, cudaMemcpyDeviceToHost, s));
-        GW_CUDA(cudaStreamSynchronize(s));
-        if (hs.done) break;
-        if (stall.stalled(hs.beta)) { g_last_stalled = 1; break; }
+        if (!ahead) {
+            GW_CUDA(cudaMemcpyAsync(&hs, G.sc, head, cudaMemcpyDeviceToHost, s));
+            GW_CUDA(cudaStreamSynchronize(s));
+            if (hs.done) break;
+        }
+        if (!ahead && stall.stalled(hs.beta)) { g_last_stalled = 1; break; }
         // Arnoldi steps queued before the next host check.  A step queued past
         // convergence costs as much as one that counts, a check 10-15 us of idle
         // device: nine tenths of the steps that the previous solve's convergence
         // rate predicts (solves of one load step contract alike), then what the
         // observed rate leaves.
         int chunk = 4;
-        if (plan_in && plan_in->last_rate > 0 && hs.tol > 0.0 && hs.beta > hs.tol)
+        if (ahead)
+            chunk = (int)std::min(-0.9 * ::log(rtol) / (1e-3 * plan_in->last_rate), 1e6);
+        else if (plan_in && plan_in->last_rate > 0 && hs.tol > 0.0 && hs.beta > hs.tol)
             chunk = (int)std::min(0.9 * ::log(hs.beta / hs.tol) / (1e-3 * plan_in->last_rate), 1e6);
         else if (plan_in && plan_in->last_iters > 0)
             chunk = std::min(plan_in->last_iters, 16);
         chunk = std::min(std::max(chunk, 1), std::min(restart, std::max(max_iter - hs.iters, 1)));
+        bool counted = false;
         for (;;) {
             cudaGraphExec_t step_graph = nullptr;
             int64_t step_nodes = 0;
@@ -1303,6 +1326,10 @@ int gmres_mg(const gw_grid_t *grid, const gw_bsr_t *A, gw_mg_plan_t *plan_in, co
             GW_LAUNCHED();
             GW_CUDA(cudaMemcpyAsync(&hs, G.sc, head, cudaMemcpyDeviceToHost, s));
             GW_CUDA(cudaStreamSynchronize(s));
+            if (ahead && !counted) {
+                counted = true;
+                (void)stall.stalled(hs.beta);  // the first cycle's entry of the window
+            }
             if (hs.cycle_done) break;
             int next = std::min(chunk < 16 ? chunk * 2 : 16, restart - hs.k);
             if (hs.k > 0 && hs.beta > 0.0 && hs.resid > 0.0 && hs.resid < hs.beta && hs.tol > 0.0) {
@@ -1328,7 +1355,8 @@ int gmres_mg(const gw_grid_t *grid, const gw_bsr_t *A, gw_mg_plan_t *plan_in, co
         if (hs.iters > 0 && hs.resid > 0.0 && hs.resid < hs.bnorm)
             plan_in->last_rate = (int)(1e3 * ::log(hs.bnorm / hs.resid) / hs.iters);
     }
-    rc = guard_check(s, "multigrid GMRES");
+    // the header carries the guard of every kernel up to the last residual
+    rc = (hs.guard || hs.status) ? guard_check(s, "multigrid GMRES") : GW_OK;
     if (rc) return rc;
     if (hs.status == ST_NAN) return GW_ENAN;
     if (hs.resid > hs.tol) return GW_ENOCONV;
@@ -1382,8 +1410,6 @@ extern "C" int gw_mg_plan_build(const gw_grid_t *grid, const gw_bsr_t *A, void *
         case 3: rc = mg_pattern<3>(h, A, plan_host, s); break;
         default: rc = mg_pattern<4>(h, A, plan_host, s); break;
     }
-    if (rc) return rc;
-    rc = guard_check(s, "multigrid plan");
     if (rc) return rc;
     plan_host->workspace = workspace;
     return GW_OK;

@@ -9,6 +9,7 @@
 // iterations in chunks and poll the flag once per chunk.
 #pragma once
 #include <cuda_bf16.h>
+#include <stddef.h>
 
 #include "gw_kernels.cuh"
 
@@ -662,6 +663,7 @@ struct GScalars {
     int reorth;      // column k takes the second Gram-Schmidt pass
     int kn;          // basis vector `next` forms (its own copy: block 0 advances k meanwhile)
     int reorths;     // second passes taken in this solve
+    int guard;       // first failed index guard up to the last residual
     double H[kGmresMaxRestart + 1][kGmresMaxRestart];
     double cs[kGmresMaxRestart], sn[kGmresMaxRestart];
     double g[kGmresMaxRestart + 1];
@@ -675,6 +677,19 @@ struct GmresVecs {
     GScalars *sc;
     size_t n;  // n_rows * NF (stride of V)
 };
+
+// start of a solve: the header cleared, the limits set (one launch for a memset
+// and two host copies)
+__global__ void k_gm_begin(GScalars *sc, int max_iter, int restart, double eta2) {
+    constexpr int head = offsetof(GScalars, H) / 4;
+    for (int i = threadIdx.x; i < head; i += blockDim.x) ((int *)sc)[i] = 0;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        sc->max_iter = max_iter;
+        sc->restart = restart;
+        sc->gs_eta2 = eta2;
+    }
+}
 
 // w = r = b - A x ; beta = ||r|| ; first cycle also ||b|| and the tolerance
 template <int NF, typename VT>
@@ -709,6 +724,7 @@ __global__ void k_gm_residual(PtrsA A, GmresVecs G, int first, double rtol) {
         sc->k = 0;
         sc->cycle_done = 0;
         sc->reorth = sc->kn = 0;
+        sc->guard = *(volatile int *)&g_guard_site;
         sc->g[0] = sc->beta;
         for (int i = 1; i <= kGmresMaxRestart; ++i) sc->g[i] = 0.0;
         if (!isfinite(sc->beta)) { sc->status = ST_NAN; sc->done = 1; sc->cycle_done = 1; }

@@ -91,25 +91,43 @@ __global__ void k_mg_fixed_mask(PtrsA A, uint8_t *__restrict__ fixed) {
 }
 
 // ---------------------------------------------------------------- coarse active set
-__global__ void k_mg_coarse_flags(Lat Lf, PtrsA Af, Lat Lc, uint8_t *__restrict__ cflag) {
-    const int r = blockIdx.x * blockDim.x + threadIdx.x;
-    if (r >= Af.n_rows) return;
-    const int node = Af.row2node[r];
-    if (!in_range(node, lat_size(Lf), GS_COARSE_FLAGS)) return;
-    int c[3];
-    lat_coords(Lf, node, c);
-    int lo[3], cnt[3];
-    for (int k = 0; k < 3; ++k) {
-        lo[k] = c[k] >> 1;
-        cnt[k] = (k < Lf.dim && (c[k] & 1)) ? 2 : 1;
+// A coarse node is active when a fine node it is a parent of is.  One thread per
+// coarse node of the lattice; fine nodes by node2row (level 0) or by their flags, so
+// the levels' counts need no host read in between: *count += active nodes.
+__global__ void k_mg_coarse_flags(Lat Lf, const int *__restrict__ f_node2row, const uint8_t *__restrict__ fflag, Lat Lc,
+                                  uint8_t *__restrict__ cflag, int *__restrict__ count) {
+    const int I = blockIdx.x * blockDim.x + threadIdx.x;
+    bool on = false;
+    if (I < lat_size(Lc)) {
+        int C[3];
+        lat_coords(Lc, I, C);
+        for (int oz = (Lf.dim == 3 ? -1 : 0); oz <= (Lf.dim == 3 ? 1 : 0) && !on; ++oz)
+            for (int oy = -1; oy <= 1 && !on; ++oy)
+                for (int ox = -1; ox <= 1 && !on; ++ox) {
+                    const int ci[3] = {2 * C[0] + ox, 2 * C[1] + oy, 2 * C[2] + oz};
+                    bool in = true;
+                    for (int k = 0; k < Lf.dim; ++k) in = in && ci[k] >= 0 && ci[k] < Lf.n[k];
+                    if (!in) continue;
+                    const int i = lat_id(Lf, ci);
+                    on = f_node2row ? f_node2row[i] >= 0 : fflag[i] != 0;
+                }
+        cflag[I] = on;
     }
-    for (int a = 0; a < cnt[0]; ++a)
-        for (int b = 0; b < cnt[1]; ++b)
-            for (int d = 0; d < cnt[2]; ++d) {
-                const int C[3] = {lo[0] + a, lo[1] + b, lo[2] + d};
-                const int id = lat_id(Lc, C);
-                if (in_range(id, lat_size(Lc), GS_COARSE_FLAGS)) cflag[id] = 1;
-            }
+    const int n = __syncthreads_count(on);
+    if (threadIdx.x == 0 && n) atomicAdd(count, n);
+}
+
+// what the host reads once the patterns are queued: block counts of the levels and
+// the index guard
+struct MgTotals {
+    int n;
+    const int *row_ptr[kMgMaxLevels];
+    int n_rows[kMgMaxLevels];
+};
+__global__ void k_mg_totals(MgTotals t, int *__restrict__ out) {
+    const int l = threadIdx.x;
+    if (l < t.n) out[l] = t.row_ptr[l][t.n_rows[l]];
+    if (l == kMgMaxLevels) out[l] = g_guard_site;
 }
 
 // coarse stencil mask of every coarse row and its block count
