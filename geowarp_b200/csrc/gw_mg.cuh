@@ -572,78 +572,6 @@ __global__ void k_mg_residual(PtrsA A, const double *__restrict__ b, const doubl
     }
 }
 
-// b_c = P^T r_f
-template <int D, int NF>
-__global__ void k_mg_restrict(Lat Lf, PtrsA Af, const uint8_t *__restrict__ ffixed, Lat Lc, PtrsA Ac,
-                              const double *__restrict__ rf, double *__restrict__ bc, const int *__restrict__ skip) {
-    if (skip && *skip) return;
-    const int R = blockIdx.x * blockDim.x + threadIdx.x;
-    if (R >= Ac.n_rows) return;
-    const int I = Ac.row2node[R];
-    if (!in_range(I, lat_size(Lc), GS_RESTRICT)) return;
-    int C[3];
-    lat_coords(Lc, I, C);
-    double acc[NF];
-#pragma unroll
-    for (int f = 0; f < NF; ++f) acc[f] = 0.0;
-    for (int oz = (D == 3 ? -1 : 0); oz <= (D == 3 ? 1 : 0); ++oz)
-        for (int oy = -1; oy <= 1; ++oy)
-            for (int ox = -1; ox <= 1; ++ox) {
-                const int ci[3] = {2 * C[0] + ox, 2 * C[1] + oy, 2 * C[2] + oz};
-                bool in = true;
-                for (int k = 0; k < D; ++k) in = in && ci[k] >= 0 && ci[k] < Lf.n[k];
-                if (!in) continue;
-                const int fr = Af.node2row[lat_id(Lf, ci)];
-                if (fr < 0 || !in_range(fr, Af.n_rows, GS_RESTRICT)) continue;
-                double w = 1.0;
-                for (int k = 0; k < D; ++k) w *= p_weight(ci[k], C[k]);
-                const uint8_t fx = ffixed[fr];
-#pragma unroll
-                for (int f = 0; f < NF; ++f)
-                    if (!((fx >> f) & 1)) acc[f] += w * rf[(size_t)fr * NF + f];
-            }
-#pragma unroll
-    for (int f = 0; f < NF; ++f) bc[(size_t)R * NF + f] = acc[f];
-}
-
-// x_f += P x_c
-template <int D, int NF>
-__global__ void k_mg_prolong(Lat Lf, PtrsA Af, const uint8_t *__restrict__ ffixed, Lat Lc, PtrsA Ac,
-                             const double *__restrict__ xc, double *__restrict__ xf, const int *__restrict__ skip) {
-    if (skip && *skip) return;
-    const int r = blockIdx.x * blockDim.x + threadIdx.x;
-    if (r >= Af.n_rows) return;
-    const int node = Af.row2node[r];
-    if (!in_range(node, lat_size(Lf), GS_PROLONG)) return;
-    int c[3];
-    lat_coords(Lf, node, c);
-    int lo[3], cnt[3];
-    for (int k = 0; k < 3; ++k) {
-        lo[k] = c[k] >> 1;
-        cnt[k] = (k < D && (c[k] & 1)) ? 2 : 1;
-    }
-    double acc[NF];
-#pragma unroll
-    for (int f = 0; f < NF; ++f) acc[f] = 0.0;
-    for (int a = 0; a < cnt[0]; ++a)
-        for (int b = 0; b < cnt[1]; ++b)
-            for (int d = 0; d < cnt[2]; ++d) {
-                const int C[3] = {lo[0] + a, lo[1] + b, lo[2] + d};
-                const int cid = lat_id(Lc, C);
-                if (!in_range(cid, lat_size(Lc), GS_PROLONG)) continue;
-                const int R = Ac.node2row[cid];
-                if (R < 0 || !in_range(R, Ac.n_rows, GS_PROLONG)) continue;
-                double w = 1.0;
-                for (int k = 0; k < D; ++k) w *= p_weight(c[k], C[k]);
-#pragma unroll
-                for (int f = 0; f < NF; ++f) acc[f] += w * xc[(size_t)R * NF + f];
-            }
-    const uint8_t fx = ffixed[r];
-#pragma unroll
-    for (int f = 0; f < NF; ++f)
-        if (!((fx >> f) & 1)) xf[(size_t)r * NF + f] += acc[f];
-}
-
 // BF16 copy of FP32 block values (the V-cycle's copy of a mixed-precision
 // fine level; round to nearest)
 __global__ void k_to_bf16(const float *__restrict__ in, __nv_bfloat16 *__restrict__ out, size_t n) {
@@ -652,12 +580,11 @@ __global__ void k_to_bf16(const float *__restrict__ in, __nv_bfloat16 *__restric
 }
 
 // ---------------------------------------------------------------- transfer lists
-// The transfers above find each child / parent through the lattice
-// (row2node, coordinates, node2row) on every V-cycle.  The pattern phase
-// resolves those lookups once per load step into row lists, so a V-cycle's
-// restriction and prolongation read an index list and then the vector: two
-// dependent loads instead of three per child.  The lists keep the loop order
-// of k_mg_restrict / k_mg_prolong, so the sums are bitwise the same.
+// Restriction is b_c = P^T r_f, prolongation x_f += P x_c.  Finding a child or
+// parent takes three dependent loads (row2node, coordinates, node2row): the
+// pattern phase does that once per load step into row lists, so a V-cycle's
+// transfers read an index list and then the vector.  The lists run over the
+// neighbours x fastest (children) and z fastest (parents), the order of the sums.
 
 // child[R * 3^D + q] (3D; child[q * n_rows + R] in 2D): fine row of child q
 // (q = ox+1 + 3 (oy+1) [+ 9 (oz+1)]) of coarse row R, -1 where the child is
@@ -693,7 +620,7 @@ __global__ void k_mg_children(Lat Lf, PtrsA Af, Lat Lc, PtrsA Ac, int *__restric
 }
 
 // parent[r * 2^D + q] (3D; parent[q * n_rows + r] in 2D): coarse rows of fine
-// row r in k_mg_prolong's loop order, -1 where that parent is outside the
+// row r, z fastest, -1 where that parent is outside the
 // lattice or inactive, -2 past the parity count (the weight of every parent is 1 / that count)
 template <int D>
 __global__ void k_mg_parents(Lat Lf, PtrsA Af, Lat Lc, PtrsA Ac, int *__restrict__ parent) {

@@ -6,7 +6,7 @@ b / |b| and y the minimiser of |b - y A z|, so the solution after max_iter = 1
 shows every entry of the V-cycle.  Lattices: dense level only, two levels,
 levels around the chunk sizes of 8 and 32 rows, 25-point and 9-point rows side
 by side, nodes missing from the active set, fixed DOFs, and a lattice above
-32,768 rows, where a row is one lane's.  Matrices hold FP32-representable values,
+24,576 rows, where a row is one lane's.  Matrices hold FP32-representable values,
 so both precisions solve the same finest system.
 
 Tolerances.  FP64: the library and SciPy sum the same terms in another order:
