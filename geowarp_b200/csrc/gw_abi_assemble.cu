@@ -1,5 +1,5 @@
 // C ABI, residual and element-tangent assembly (declarations and reference
-// citations in include/geowarp_b200.h): the deterministic cell-coloured
+// citations in include/geowarp_b200.h): the deterministic cell-sum
 // assembly of the 2D kinds (gw_assemble_sorted) and the atomic one
 // (gw_assemble, used for the 3D kind).
 #include "gw_host.cuh"

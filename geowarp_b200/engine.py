@@ -196,7 +196,7 @@ class Engine:
         self.norm_dev = torch.zeros(1, **f64)
         self._sort_ws = _Buf(dev)
         self._scan_ws = _Buf(dev)
-        self._asm_ws = _Buf(dev)  # particle records of the cell-coloured assembly
+        self._asm_ws = _Buf(dev)  # records and cell sums of the 2D assembly
         self.deterministic_assembly = True
         self._kry_ws = _Buf(dev)
         self._norm_ws = torch.zeros(16384, dtype=torch.uint8, device=dev)
@@ -391,8 +391,8 @@ class Engine:
         return st
 
     def assemble(self, mat_struct, current_step, total_steps, want_K=True):
-        """Residual and (want_K) element tangent: the deterministic cell-coloured
-        assembly for the 2D kinds, the atomic one for 3D (or when
+        """Residual and (want_K) element tangent: the deterministic assembly
+        (cell sums, then a gather per row) for the 2D kinds, the atomic one for 3D (or when
         deterministic_assembly is False)."""
         g, pt, s = self.grid_struct(), self.particles_struct(), self.stream
         st = self.step_struct(current_step, total_steps)

@@ -440,10 +440,11 @@ int gw_adjoint_residual(const gw_grid_t *grid, const gw_material_t *mat, const g
 
 /* ------------------------------------------------------------ kernel timing
  * Optional CUDA-event timing of the engine's main kernels (off by default):
- * classes 0..12 = k_assemble, k_gm_spmv, k_gm_dots, k_gm_update, k_gm_next,
+ * classes 0..13 = k_assemble, k_gm_spmv, k_gm_dots, k_gm_update, k_gm_next,
  * k_g2p, k_adjoint_g2p, k_adjoint_residual, k_mg_jacobi (finest level),
  * k_mg_residual, k_mg_restrict/prolong, mg_setup (the numeric hierarchy
- * build), k_mg_jacobi (coarse levels).  gw_profile_read synchronises and
+ * build), k_mg_jacobi (coarse levels), k_mg_tail (the fused coarse levels; 2D
+ * row kernels carry the class of the phase they run).  gw_profile_read synchronises and
  * returns the total time, launch count and algorithmic bytes of a class. */
 int gw_profile_enable(int32_t on);
 /* Number of timing classes (k_assemble ... mg_setup) gw_profile_read accepts. */
@@ -466,8 +467,8 @@ const char *gw_profile_name(int32_t cls);
  *   GW_TUNE_ADJOINT_BLOCK   threads per CTA of the adjoint particle kernels,
  *                           32..256, a multiple of 32 (default 128)
  *   GW_TUNE_ROW_WARPS       warps per CTA of the multigrid smoothing and
- *                           residual kernels (four block rows per warp), 1..32
- *                           (default 8)
+ *                           residual kernels, 1..32 (default 8; the 2D
+ *                           kernels use at most 8)
  *   GW_TUNE_MG_COARSE       most unknowns of the dense coarsest multigrid
  *                           level, 8..160 (default 160)
  *   GW_TUNE_MG_ONE_SWEEP    first multigrid level smoothed by one sweep
@@ -487,15 +488,16 @@ const char *gw_profile_name(int32_t cls);
  *                           orthogonality; 3: the classical 1/2; 0: always;
  *                           300: never unless non-finite)
  *   GW_TUNE_MG_TAIL         most block rows of a multigrid level run by the
- *                           fused coarse tail: that level and every coarser
- *                           one go through one launch of one thread-block
- *                           cluster with cluster barriers between the
- *                           phases (bitwise the same V-cycle; the cluster
- *                           has 1 to 16 CTAs, two rows of the first tail
- *                           level per 8-lane group), 0..1048576 (default 0:
- *                           one launch per phase); recaptures the step
- *                           graphs.  It pays where the levels are a few
- *                           hundred rows (launch-bound hierarchies)
+ *                           fused coarse tail (2D): that level and every
+ *                           coarser one go through one launch of one
+ *                           thread-block cluster of 1 to 16 CTAs, with
+ *                           cluster barriers between the phases and the
+ *                           levels' constants and vectors in shared memory
+ *                           (bitwise the same V-cycle).  Levels that do not
+ *                           fit there stay one launch per phase.
+ *                           0..1048576 (default 0: up to 2,048 rows; values
+ *                           above 16,384 act as 16,384; 3D hierarchies run
+ *                           one launch per phase); recaptures the step graphs
  *   GW_TUNE_MG_BF16         1: in mixed-precision multigrid solves the V-cycle
  *                           reads a BF16 copy of the fine-level Jacobian (made
  *                           before each solve; GMRES still applies the FP32

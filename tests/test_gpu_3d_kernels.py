@@ -108,3 +108,69 @@ def test_assembly_groupings_agree(cuda, precision):
     assert float((R - parts[0][0] - parts[1][0]).abs().max()) <= 1e-12 * float(R.abs().max())
     assert float((K - K2).abs().max()) <= tol * float(K.abs().max())
     assert abs(f - parts[0][2] - parts[1][2]) <= 1e-12 * abs(f)
+
+
+@pytest.mark.parametrize("single", [False, True], ids=["fp64", "mixed"])
+@pytest.mark.parametrize("mx,my,mz,nf,holes", [(3, 4, 2, 3, 0.0), (9, 8, 7, 1, 0.1), (11, 7, 9, 3, 0.05), (8, 9, 10, 4, 0.0)])
+def test_multigrid_on_a_3d_lattice(cuda, mx, my, mz, nf, holes, single):
+    """27-point rows on an mx x my x mz lattice with missing nodes: the tolerances
+    of the row tests above."""
+    from geowarp_b200 import _lib as L
+    from geowarp_b200.engine import _p
+    lib = L.load()
+    rng = np.random.default_rng(mx + nf)
+    nn = mx * my * mz
+    active = rng.random(nn) >= holes
+    id_ = np.arange(nn)
+    x, y, z = id_ % mx, id_ // mx % my, id_ // (mx * my)
+    row2node = np.nonzero(active)[0]
+    node2row = np.full(nn, -1)
+    node2row[row2node] = np.arange(row2node.size)
+    stencil = np.zeros((nn, 4), np.uint32)
+    ii, jj, bit = [], [], []
+    for oz in (-1, 0, 1):
+        for oy in (-1, 0, 1):
+            for ox in (-1, 0, 1):
+                q = (ox + 2) + 5 * (oy + 2) + 25 * (oz + 2)
+                ok = (x + ox >= 0) & (x + ox < mx) & (y + oy >= 0) & (y + oy < my) & (z + oz >= 0) & (z + oz < mz) & active
+                j = np.where(ok, id_ + ox + mx * (oy + my * oz), 0)
+                ok &= active[j]
+                stencil[ok, q // 32] |= np.uint32(1 << (q % 32))
+                ii.append(node2row[id_[ok]]); jj.append(node2row[j[ok]]); bit.append(np.full(int(ok.sum()), q))
+    i, j = np.concatenate(ii), np.concatenate(jj)
+    order = np.lexsort((np.concatenate(bit), i))
+    i, j = i[order], j[order]
+    n = row2node.size
+    vals = rng.uniform(-1.0, 0.2, (i.size, nf, nf)).astype(np.float32).astype(np.float64)
+    k = np.arange(nf)
+    d = np.nonzero(i == j)[0]
+    vals[d[:, None], k, k] = 0
+    off = np.zeros((n, nf))
+    np.add.at(off, i, np.abs(vals).sum(2))
+    vals[d[:, None], k, k] = (1.25 * off[i[d]] + 0.1).astype(np.float32)
+    rr_, cc_ = (i[:, None, None] * nf + k[:, None]) + 0 * k[None, :], (j[:, None, None] * nf + k[None, :]) + 0 * k[:, None]
+    M = sp.csr_matrix((vals.ravel(), (rr_.ravel(), cc_.ravel())), shape=(n * nf,) * 2)
+    t = lambda a, dt: torch.as_tensor(np.ascontiguousarray(a).astype(dt), device=cuda)  # noqa: E731
+    keep = dict(row_ptr=t(np.concatenate([[0], np.cumsum(np.bincount(i, minlength=n))]), np.int32), cols=t(j, np.int32),
+                row2node=t(row2node, np.int32), node2row=t(node2row, np.int32),
+                stencil=t(stencil.view(np.int32), np.int32), vals=t(vals, np.float32 if single else np.float64))
+    A, g = L.Bsr(), L.Grid()
+    A.n_rows, A.nf, A.nnzb, A.mask_words = n, nf, i.size, 4
+    for name, v in keep.items():
+        setattr(A, name, _p(v))
+    g.dim, g.nf, g.n_nodes = 3, nf, nn
+    for a, m in enumerate((mx, my, mz)):
+        g.n_grid[a], g.h[a], g.inv_h[a], g.h_nodes[a] = m - 1, 1.0, 1.0, 1.0
+    xs = rng.uniform(-1, 1, n * nf)
+    b = M @ xs
+    bt, xt = torch.as_tensor(b, device=cuda), torch.zeros(n * nf, dtype=torch.float64, device=cuda)
+    nb = lib.gw_gmres_mg_workspace_bytes(C.byref(g), n, nf, 20)
+    ws = torch.full((nb,), 0xFF, dtype=torch.uint8, device=cuda)
+    it, rr = C.c_int32(0), C.c_double(0.0)
+    rc = lib.gw_bsr_gmres_mg_solve(C.byref(g), C.byref(A), L.PREC_F32 if single else L.PREC_F64, None, _p(bt), _p(xt), 1e-12,
+                                   1000, 20, _p(ws), nb, C.byref(it), C.byref(rr), None)
+    torch.cuda.synchronize()
+    got = xt.cpu().numpy()
+    assert rc == L.GW_OK
+    assert np.linalg.norm(M @ got - b) <= 2e-12 * np.linalg.norm(b)
+    assert np.abs(got - xs).max() <= 9 * 2e-12 * np.sqrt(got.size) * np.abs(b).max()
