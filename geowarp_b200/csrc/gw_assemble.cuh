@@ -384,6 +384,7 @@ __global__ void __launch_bounds__(32 * kGatherRows) k_row_gather(gw_grid_t grid,
 #pragma unroll
     for (int q = 0; q < (WANT_K ? BB : 1); ++q) blk[q] = (VT)0;
     double rsum = 0.0;
+    bool touched = false;  // a cell holds this lane's block
     // the cells that reach the node (four where particles stay inside their cells, up
     // to nine), four at a time with their values in flight
     unsigned left = __ballot_sync(0xffffffffu, info != 0);
@@ -412,9 +413,11 @@ __global__ void __launch_bounds__(32 * kGatherRows) k_row_gather(gw_grid_t grid,
 #pragma unroll
         for (int o = 0; o < M; ++o) {
             rsum += rv[o];
-            if (WANT_K && on[o])
+            if (WANT_K && on[o]) {
+                touched = true;
 #pragma unroll
                 for (int q = 0; q < (WANT_K ? BB : 1); ++q) blk[q] = (VT)((double)blk[q] + v[o][q]);
+            }
         }
     }
     if (lane >= 25) {
@@ -427,11 +430,11 @@ __global__ void __launch_bounds__(32 * kGatherRows) k_row_gather(gw_grid_t grid,
         return;
     }
     if (!WANT_K) return;
-    if (!((st >> lane) & 1u)) {  // a contribution outside the pattern, or no diagonal block
-        bool any = lane == 12;
-#pragma unroll
-        for (int q = 0; q < (WANT_K ? BB : 1); ++q) any = any || (fa && blk[q] != (VT)0);
-        if (any) atomicOr(&g_status, ST_RANGE);
+    if (!((st >> lane) & 1u)) {
+        // no diagonal block, or a cell that couples two free nodes outside the pattern (a
+        // node without free DOFs may lie inside a particle's span and have no row: u-p
+        // nodes below the activation weight)
+        if (lane == 12 || (touched && fa && fb)) atomicOr(&g_status, ST_RANGE);
         return;
     }
     const long long jb = (long long)base + __popc(st & ((1u << lane) - 1u));
