@@ -187,7 +187,7 @@ int assemble_sorted(const LaunchConst &c, const PtrsP &p, const int *perm, const
     launch_particle_q<KIND, WANT_K, VT>(c, p, perm, un, uo, scratch, force, s);
     GW_LAUNCHED();
     k_cell_blocks<KIND, WANT_K, VT><<<gw_count_launch(nblk(nc, kCellGroups)), 16 * kCellGroups, 0, s>>>(
-        c, nc, by_cell, cstart, cend, scratch, sums, box);
+        c, nc, by_cell, cstart, cend, scratch, fm, a.node2row, a.n_rows, sums, box);
     if (A->n_rows > 0)
         k_row_gather<KIND, WANT_K, VT><<<gw_count_launch(nblk(A->n_rows, kGatherRows)), 32 * kGatherRows, 0, s>>>(
             c.g, by_cell, cstart, box, sums, fm, a, R);

@@ -164,6 +164,8 @@ __global__ void __launch_bounds__(16 * kCellGroups) k_cell_blocks(LaunchConst c,
                                                                   const int *__restrict__ cstart,
                                                                   const int *__restrict__ cend,
                                                                   const unsigned char *__restrict__ scratch,
+                                                                  const uint8_t *__restrict__ free_mask,
+                                                                  const int *__restrict__ node2row, int n_rows,
                                                                   double *__restrict__ sums, int *__restrict__ box) {
     typedef KindTraits<KIND> KT;
     typedef Layout<KIND> L;
@@ -211,6 +213,11 @@ __global__ void __launch_bounds__(16 * kCellGroups) k_cell_blocks(LaunchConst c,
     const bool one = p1 - p0 <= kCellBatch;  // the axes of the only batch are in place
     const float ins = 1.0f / (float)max(ns, 1), ie0 = 1.0f / (float)max(e0, 1);  // exact quotients of small integers below
     double *const out = sums + (size_t)(by_cell ? cell : p0) * CS::ND;
+    if (lane < ns) {  // a node with free DOFs that no row would gather (a stale row map)
+        const int ay = (int)(((float)lane + 0.5f) * ie0), nx = cx + lane - ay * e0, ny = cy + ay;
+        const int node = nx + ny * (ncx + 1);
+        if (nx <= ncx && ny <= c.g.n_grid[1] && free_mask[node]) in_range(node2row[node], n_rows, GS_ASSEMBLE);
+    }
     __syncwarp(gmask);
 
     for (int q0 = 0; q0 < ns * NF; q0 += 16) {  // residual entries (slot a, field f)

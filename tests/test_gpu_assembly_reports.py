@@ -1,9 +1,12 @@
 """What the 2D assembly reports about a state it cannot place in the matrix, against
 the atomic assembly of the same particles: a contribution outside the pattern sets the
-device status (bit 0), and a node that no row belongs to is not such a contribution.
+device status (bit 0), and a node that no row belongs to is not such a contribution; a free node whose row
+number is outside the matrix (a stale row map) fails the index guard.
 
 R and K of both assemblies are the same terms in another order: 1e-12 of the largest
 entry in FP64, 1e-6 (a few roundings of 2^-24) where K is FP32."""
+import ctypes as C
+
 import numpy as np
 import pytest
 import torch
@@ -77,3 +80,29 @@ def test_contribution_outside_the_pattern_is_reported(cuda, kind, past):
     e.stencil[node] = st & ~(1 << (st.bit_length() - 1))
     assert _assemble(e, mat, True)[2] == 1
     assert _assemble(e, mat, False)[2] == 1
+
+
+@pytest.mark.parametrize("want_K", [True, False])
+@pytest.mark.parametrize("kind", ["solid2d", "coupled2d"])
+@pytest.mark.parametrize("row", [-1, 10000])
+def test_stale_row_map_fails_the_index_guard(cuda, kind, row, want_K):
+    from geowarp_b200 import _lib as L
+    lib = L.load()
+
+    def guard():
+        site, val = C.c_int32(0), C.c_int64(0)
+        assert lib.gw_guard_read(C.byref(site), C.byref(val), e.stream) == L.GW_OK
+        return lib.gw_guard_site_name(site.value).decode(), val.value
+
+    e, mat = _engine(kind, 0.0, "fp64", cuda)
+    R, K, st = _assemble(e, mat, True, want_K)
+    assert st == 0 and guard() == ("none", 0)
+    node = 4 + 4 * 9
+    keep = int(e.node2row[node])
+    e.node2row[node] = row
+    assert _assemble(e, mat, True, want_K)[2] == 1
+    assert guard() == ("assembly scatter", row)
+    e.node2row[node] = keep
+    R1, K1, st = _assemble(e, mat, True, want_K)
+    assert st == 0 and guard() == ("none", 0)
+    assert np.array_equal(R, R1) and np.array_equal(K, K1)
