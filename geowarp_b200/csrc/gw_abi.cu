@@ -317,7 +317,7 @@ extern "C" int gw_return_map(const gw_material_t *mat, int32_t n, const double *
 }
 
 
-extern "C" int64_t gw_launch_count(void) { return g_launches; }
+extern "C" int64_t gw_launch_count(void) { return g_launches.load(); }
 
 extern "C" int gw_tune_set(int32_t knob, int32_t value) {
     switch (knob) {

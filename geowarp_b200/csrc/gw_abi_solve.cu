@@ -2,6 +2,7 @@
 // preconditioned flexible GMRES, the workspace-free Krylov entry point and
 // SpMV (declarations and reference citations in include/geowarp_b200.h).
 #include <algorithm>
+#include <mutex>
 #include <type_traits>
 #include <vector>
 
@@ -191,15 +192,31 @@ void gs_column(const GmresVecs &G, int restart, double vb, cudaStream_t s) {
     { ProfScope ps(PC_DOTS, s, vb); gs_dots(G, restart, 1, s); }
     { ProfScope ps(PC_UPDATE, s, vb + n8); gs_update(G, 1, s); }
 }
-// stream of the solvers' graph captures, one per device
+// Graph of the launches that record(stream) makes, and their number.  The solvers'
+// captures share one stream per device, so one host thread records at a time.
+std::mutex g_capture_mu;
 cudaStream_t g_capture_stream[64] = {};
 
-int capture_stream(cudaStream_t *out) {
+template <typename F>
+int capture_graph(F record, cudaGraphExec_t *exec, int64_t *launches) {
     int dev = 0;
     GW_CUDA(cudaGetDevice(&dev));
     if (dev < 0 || dev >= 64) return GW_EINVAL;
-    if (!g_capture_stream[dev]) GW_CUDA(cudaStreamCreateWithFlags(&g_capture_stream[dev], cudaStreamNonBlocking));
-    *out = g_capture_stream[dev];
+    cudaGraph_t graph;
+    *launches = 0;
+    {
+        std::lock_guard<std::mutex> lk(g_capture_mu);
+        cudaStream_t &cs = g_capture_stream[dev];
+        if (!cs) GW_CUDA(cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking));
+        GW_CUDA(cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal));
+        t_captured = launches;
+        record(cs);
+        t_captured = nullptr;
+        GW_CUDA(cudaStreamEndCapture(cs, &graph));
+    }
+    const cudaError_t ie = cudaGraphInstantiate(exec, graph, 0);
+    cudaGraphDestroy(graph);
+    GW_CUDA(ie);
     return GW_OK;
 }
 
@@ -274,20 +291,11 @@ int gmres(const gw_bsr_t *A, int precond, const double *b, double *x, double rto
                 // a solve that needs more than its first columns replays eight at a
                 // time: six launches of 2-3 us of work each cost the host 20 us
                 if (!step.exec && chunk >= kStepCols) {
-                    cudaStream_t cs;
-                    int rc = capture_stream(&cs);
+                    auto columns = [&](cudaStream_t cs) {
+                        for (int q = 0; q < kStepCols; ++q) column(cs);
+                    };
+                    const int rc = capture_graph(columns, &step.exec, &step.launches);
                     if (rc) return rc;
-                    const int64_t before = g_launches;
-                    cudaGraph_t graph;
-                    GW_CUDA(cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal));
-                    for (int q = 0; q < kStepCols; ++q) column(cs);
-                    const cudaError_t ce = cudaStreamEndCapture(cs, &graph);
-                    step.launches = g_launches - before;
-                    g_launches = before;  // counted when the graph is replayed
-                    GW_CUDA(ce);
-                    const cudaError_t ie = cudaGraphInstantiate(&step.exec, graph, 0);
-                    cudaGraphDestroy(graph);
-                    GW_CUDA(ie);
                 }
                 for (; step.exec && it + kStepCols <= chunk; it += kStepCols, kk += kStepCols) {
                     GW_CUDA(cudaGraphLaunch(step.exec, s));
@@ -1176,22 +1184,12 @@ int mg_step_graph(const MgHier &h, const gw_grid_t &grid, const gw_bsr_t *A, Gmr
         if (victim < 0 || (g_mg_graphs[victim].valid && (!ent.valid || ent.stamp < g_mg_graphs[victim].stamp)))
             victim = e;
     }
-    cudaStream_t cs;
-    int rc = capture_stream(&cs);
-    if (rc) return rc;
     PtrsA a = make_ptrs(*A);
-    const int64_t before = g_launches;
-    GW_CUDA(cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal));
-    mg_arnoldi_step<NF, VT>(h, a, G, Z, restart, skip, cs);
-    cudaGraph_t graph;
-    const cudaError_t ce = cudaStreamEndCapture(cs, &graph);
-    const int64_t count = g_launches - before;
-    g_launches = before;  // counted when the graph is replayed
-    GW_CUDA(ce);
     cudaGraphExec_t ge;
-    const cudaError_t ie = cudaGraphInstantiate(&ge, graph, 0);
-    cudaGraphDestroy(graph);
-    GW_CUDA(ie);
+    int64_t count;
+    auto step = [&](cudaStream_t cs) { mg_arnoldi_step<NF, VT>(h, a, G, Z, restart, skip, cs); };
+    const int rc = capture_graph(step, &ge, &count);
+    if (rc) return rc;
     MgGraphEntry &slot = g_mg_graphs[victim];
     if (slot.valid) GW_CUDA(cudaGraphExecDestroy(slot.exec));
     slot.valid = true;

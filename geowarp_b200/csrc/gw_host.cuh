@@ -3,6 +3,7 @@
 // scans and the index-guard check.  State is held in C++17 inline variables,
 // so every translation unit sees one copy; helpers are static inline.
 #pragma once
+#include <atomic>
 #include <mutex>
 #include <stddef.h>
 #include <stdint.h>
@@ -109,9 +110,11 @@ struct ProfScope {
 };
 // every kernel launch of the library passes its grid size through here, so the
 // host can report how many launches a piece of work took (gw_launch_count)
-inline int64_t g_launches = 0;
+inline std::atomic<int64_t> g_launches{0};
+inline thread_local int64_t *t_captured = nullptr;  // this thread is recording a graph: counted when it is replayed
 static inline int gw_count_launch(int grid) {
-    ++g_launches;
+    if (t_captured) ++*t_captured;
+    else g_launches.fetch_add(1, std::memory_order_relaxed);
     return grid;
 }
 static inline int nblk(int64_t n, int t) { return (int)((n + t - 1) / t); }
