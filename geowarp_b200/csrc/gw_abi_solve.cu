@@ -2,6 +2,7 @@
 // preconditioned flexible GMRES, the workspace-free Krylov entry point and
 // SpMV (declarations and reference citations in include/geowarp_b200.h).
 #include <algorithm>
+#include <memory>
 #include <mutex>
 #include <type_traits>
 #include <vector>
@@ -192,29 +193,42 @@ void gs_column(const GmresVecs &G, int restart, double vb, cudaStream_t s) {
     { ProfScope ps(PC_DOTS, s, vb); gs_dots(G, restart, 1, s); }
     { ProfScope ps(PC_UPDATE, s, vb + n8); gs_update(G, 1, s); }
 }
-// Graph of the launches that record(stream) makes, and their number.  The solvers'
-// captures share one stream per device, so one host thread records at a time.
+// An instantiated graph and the launches it replays.
+struct StepGraph {
+    cudaGraphExec_t exec = nullptr;
+    int64_t launches = 0;
+    StepGraph() = default;
+    StepGraph(const StepGraph &) = delete;
+    ~StepGraph() { if (exec) cudaGraphExecDestroy(exec); }
+    int replay(cudaStream_t s) const {
+        GW_CUDA(cudaGraphLaunch(exec, s));
+        g_launches += launches;
+        return GW_OK;
+    }
+};
+
+// Graph of the launches that record(stream) makes.  The solvers' captures share one
+// stream per device, so one host thread records at a time.
 std::mutex g_capture_mu;
 cudaStream_t g_capture_stream[64] = {};
 
 template <typename F>
-int capture_graph(F record, cudaGraphExec_t *exec, int64_t *launches) {
+int capture_graph(F record, StepGraph *g) {
     int dev = 0;
     GW_CUDA(cudaGetDevice(&dev));
     if (dev < 0 || dev >= 64) return GW_EINVAL;
     cudaGraph_t graph;
-    *launches = 0;
     {
         std::lock_guard<std::mutex> lk(g_capture_mu);
         cudaStream_t &cs = g_capture_stream[dev];
         if (!cs) GW_CUDA(cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking));
         GW_CUDA(cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal));
-        t_captured = launches;
+        t_captured = &g->launches;
         record(cs);
         t_captured = nullptr;
         GW_CUDA(cudaStreamEndCapture(cs, &graph));
     }
-    const cudaError_t ie = cudaGraphInstantiate(exec, graph, 0);
+    const cudaError_t ie = cudaGraphInstantiate(&g->exec, graph, 0);
     cudaGraphDestroy(graph);
     GW_CUDA(ie);
     return GW_OK;
@@ -256,11 +270,7 @@ int gmres(const gw_bsr_t *A, int precond, const double *b, double *x, double rto
     int first = 1;
     StallWatch stall;
     g_last_stalled = 0;
-    struct Step {  // graph of kStepCols columns, for this solve only
-        cudaGraphExec_t exec = nullptr;
-        int64_t launches = 0;
-        ~Step() { if (exec) cudaGraphExecDestroy(exec); }
-    } step;
+    StepGraph step;  // kStepCols columns, for this solve only
     constexpr int kStepCols = 8;
     for (int cycle = 0; cycle < 1000000; ++cycle) {
         k_gm_residual<NF, VT><<<gw_count_launch(gr), kThreads, 0, s>>>(a, G, first, rtol);
@@ -294,12 +304,12 @@ int gmres(const gw_bsr_t *A, int precond, const double *b, double *x, double rto
                     auto columns = [&](cudaStream_t cs) {
                         for (int q = 0; q < kStepCols; ++q) column(cs);
                     };
-                    const int rc = capture_graph(columns, &step.exec, &step.launches);
+                    const int rc = capture_graph(columns, &step);
                     if (rc) return rc;
                 }
                 for (; step.exec && it + kStepCols <= chunk; it += kStepCols, kk += kStepCols) {
-                    GW_CUDA(cudaGraphLaunch(step.exec, s));
-                    g_launches += step.launches;
+                    const int rc = step.replay(s);
+                    if (rc) return rc;
                 }
             }
             for (; it < chunk; ++it, ++kk) column(s);
@@ -1120,15 +1130,22 @@ struct MgGraphKey {
     double *x, *z;
 };
 struct MgGraphEntry {
-    bool valid;
     MgGraphKey key;
-    cudaGraphExec_t exec;
-    int64_t nodes;
+    std::shared_ptr<const StepGraph> graph;  // null: an empty slot
     uint64_t stamp;
 };
 constexpr int kMgGraphCache = 8;
-MgGraphEntry g_mg_graphs[kMgGraphCache];
-uint64_t g_mg_graph_clock = 0;
+// Shared by the host threads: entries change under the lock, and a solve keeps its
+// graph alive, so an entry replaced by another thread goes when that solve is done.
+struct MgGraphs {
+    std::mutex mu;
+    MgGraphEntry e[kMgGraphCache];
+    uint64_t clock = 0;
+};
+MgGraphs &mg_graphs() {
+    static MgGraphs *const g = new MgGraphs();  // not destroyed at exit, when CUDA may be gone
+    return *g;
+}
 // The next basis vector (start: the first of a cycle) and its V-cycle.
 template <int NF, typename VT>
 void mg_step_tail(const MgHier &h, GmresVecs &G, VecRef z, int start, const int *skip, cudaStream_t s) {
@@ -1156,7 +1173,7 @@ void mg_arnoldi_step(const MgHier &h, const PtrsA &a, GmresVecs &G, double *Z, i
 // Returns the cached (or newly captured) graph of one Arnoldi step.
 template <int NF, typename VT>
 int mg_step_graph(const MgHier &h, const gw_grid_t &grid, const gw_bsr_t *A, GmresVecs &G, double *Z, void *ws,
-                  int restart, const int *skip, cudaGraphExec_t *exec, int64_t *nodes) {
+                  int restart, const int *skip, std::shared_ptr<const StepGraph> *out) {
     MgGraphKey k;
     memset(&k, 0, sizeof(k));
     GW_CUDA(cudaGetDevice(&k.device));
@@ -1171,34 +1188,31 @@ int mg_step_graph(const MgHier &h, const gw_grid_t &grid, const gw_bsr_t *A, Gmr
     for (int q = 0; q < 3; ++q) k.n_grid[q] = grid.n_grid[q];
     for (int q = 0; q < h.nl; ++q) { k.n_rows[q] = h.lv[q].A.n_rows; k.nnzb[q] = h.lv[q].A.nnzb; }
     k.A = *A; k.ws = ws; k.b = G.b; k.x = G.x; k.z = G.z;
-    int victim = -1;
-    for (int e = 0; e < kMgGraphCache; ++e) {
-        MgGraphEntry &ent = g_mg_graphs[e];
-        if (ent.valid && memcmp(&ent.key, &k, sizeof(k)) == 0) {
-            ent.stamp = ++g_mg_graph_clock;
-            *exec = ent.exec;
-            *nodes = ent.nodes;
-            return GW_OK;
-        }
-        // an empty slot first, else the least recently used one
-        if (victim < 0 || (g_mg_graphs[victim].valid && (!ent.valid || ent.stamp < g_mg_graphs[victim].stamp)))
-            victim = e;
+    MgGraphs &cache = mg_graphs();
+    {
+        std::lock_guard<std::mutex> lk(cache.mu);
+        for (MgGraphEntry &ent : cache.e)
+            if (ent.graph && memcmp(&ent.key, &k, sizeof(k)) == 0) {
+                ent.stamp = ++cache.clock;
+                *out = ent.graph;
+                return GW_OK;
+            }
     }
     PtrsA a = make_ptrs(*A);
-    cudaGraphExec_t ge;
-    int64_t count;
+    auto made = std::make_shared<StepGraph>();
     auto step = [&](cudaStream_t cs) { mg_arnoldi_step<NF, VT>(h, a, G, Z, restart, skip, cs); };
-    const int rc = capture_graph(step, &ge, &count);
+    const int rc = capture_graph(step, made.get());
     if (rc) return rc;
-    MgGraphEntry &slot = g_mg_graphs[victim];
-    if (slot.valid) GW_CUDA(cudaGraphExecDestroy(slot.exec));
-    slot.valid = true;
-    slot.key = k;
-    slot.exec = ge;
-    slot.nodes = count;
-    slot.stamp = ++g_mg_graph_clock;
-    *exec = ge;
-    *nodes = count;
+    *out = made;
+    std::shared_ptr<const StepGraph> replaced;  // released outside the lock
+    std::lock_guard<std::mutex> lk(cache.mu);
+    MgGraphEntry *slot = &cache.e[0];  // an empty slot first, else the least recently used one
+    for (MgGraphEntry &ent : cache.e)
+        if (slot->graph && (!ent.graph || ent.stamp < slot->stamp)) slot = &ent;
+    replaced = std::move(slot->graph);
+    slot->key = k;
+    slot->graph = std::move(made);
+    slot->stamp = ++cache.clock;
     return GW_OK;
 }
 
@@ -1274,6 +1288,7 @@ int gmres_mg(const gw_grid_t *grid, const gw_bsr_t *A, gw_mg_plan_t *plan_in, co
     const int gr = red_grid_rows(nr), gv = red_grid_elems(n);
     const VecRef z{fv.Z, (size_t)n};
     const int *skip = &G.sc->cycle_done;
+    std::shared_ptr<const StepGraph> step_graph;
     GScalars hs;
     memset(&hs, 0, head);
     int first = 1;
@@ -1310,16 +1325,14 @@ int gmres_mg(const gw_grid_t *grid, const gw_bsr_t *A, gw_mg_plan_t *plan_in, co
         chunk = std::min(std::max(chunk, 1), std::min(restart, std::max(max_iter - hs.iters, 1)));
         bool counted = false;
         for (;;) {
-            cudaGraphExec_t step_graph = nullptr;
-            int64_t step_nodes = 0;
-            if (!g_prof_on) {  // timed runs launch kernel by kernel, bracketed by events
-                rc = mg_step_graph<NF, VT>(h, *grid, A, G, fv.Z, ws, restart, skip, &step_graph, &step_nodes);
+            if (!g_prof_on && !step_graph) {  // timed runs launch kernel by kernel, bracketed by events
+                rc = mg_step_graph<NF, VT>(h, *grid, A, G, fv.Z, ws, restart, skip, &step_graph);
                 if (rc) return rc;
             }
             for (int it = 0; it < chunk; ++it) {
                 if (step_graph) {
-                    GW_CUDA(cudaGraphLaunch(step_graph, s));
-                    g_launches += step_nodes;
+                    rc = step_graph->replay(s);
+                    if (rc) return rc;
                 } else {
                     mg_arnoldi_step<NF, VT>(h, a, G, fv.Z, restart, skip, s);
                 }

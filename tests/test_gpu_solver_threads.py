@@ -87,3 +87,34 @@ def test_node_block_gmres_on_several_host_threads(cuda):
     from geowarp_b200 import _lib as L
     want = _run(lambda t: _Block(t, cuda), 4, 24)
     assert all(rc == L.GW_ENOCONV and it == 9 + 30 * (q % 4) for w in want for q, (rc, it, _) in enumerate(w))
+
+
+class _Multigrid:
+    """A multigrid solve; each restart length is a graph of its own, so the threads
+    together need more graphs than the library keeps."""
+
+    def __init__(self, seed, dev):
+        from test_gpu_mg_rows import _Gpu, _system
+        self.g = _Gpu(_system(20 + seed, 17, 2, seed, 0.02, 0.2), False, dev)
+        g, lib = self.g, self.g.lib
+        n = g.A.n_rows * 2
+        self.nb = lib.gw_gmres_mg_workspace_bytes(C.byref(g.g), g.A.n_rows, 2, 20)
+        self.ws = torch.empty(self.nb, dtype=torch.uint8, device=dev)
+        self.b = torch.as_tensor(np.random.default_rng(seed).standard_normal(n), device=dev)
+        self.x = torch.zeros_like(self.b)
+
+    def solve(self, q):
+        g, s = self.g, torch.cuda.current_stream()
+        self.x.zero_()
+        it, rr = C.c_int32(0), C.c_double(0.0)
+        rc = g.lib.gw_bsr_gmres_mg_solve(C.byref(g.g), C.byref(g.A), g.prec, None, g.p(self.b), g.p(self.x), 1e-300, 25,
+                                         15 + q % 6, g.p(self.ws), self.nb, C.byref(it), C.byref(rr),
+                                         C.c_void_p(s.cuda_stream))
+        s.synchronize()
+        return rc, it.value, self.x.cpu().numpy()
+
+
+def test_multigrid_gmres_on_several_host_threads(cuda):
+    from geowarp_b200 import _lib as L
+    want = _run(lambda t: _Multigrid(t, cuda), 4, 24)
+    assert all(rc == L.GW_ENOCONV and it == 25 for w in want for rc, it, _ in w)
