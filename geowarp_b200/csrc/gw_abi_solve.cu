@@ -271,7 +271,8 @@ int gmres(const gw_bsr_t *A, int precond, const double *b, double *x, double rto
     StallWatch stall;
     g_last_stalled = 0;
     StepGraph step;  // kStepCols columns, for this solve only
-    constexpr int kStepCols = 8;
+    constexpr int kStepCols = 8, kStepFrom = 24;
+    int queued = 0;  // columns of this solve so far
     for (int cycle = 0; cycle < 1000000; ++cycle) {
         k_gm_residual<NF, VT><<<gw_count_launch(gr), kThreads, 0, s>>>(a, G, first, rtol);
         gs_next<NF>(nr, G, 1, G.Minv, G.z, 1.0, s);
@@ -297,9 +298,13 @@ int gmres(const gw_bsr_t *A, int precond, const double *b, double *x, double rto
         for (;;) {
             chunk = std::min(chunk, restart - kk);
             int it = 0;
-            if (!g_prof_on && (step.exec || kk > 0)) {
-                // a solve that needs more than its first columns replays eight at a
-                // time: six launches of 2-3 us of work each cost the host 20 us
+            if (!g_prof_on && (step.exec || queued >= kStepFrom)) {
+                // A long solve replays eight columns at a time: six launches of 2-3 us of
+                // work each cost the host 20 us.  Recording them costs 140-250 us a solve, so
+                // a solve of up to 24 columns launches its kernels.  4,096 rows of 4 x 4 FP64
+                // blocks, recorded after 8 columns -> after 24: 9 columns 727 -> 501 us, 24
+                // columns 840 -> 606, 25 columns 1,166 -> 1,187, 100 columns 3,260 -> 3,270
+                // (the former kernels, no column recorded: 547, 1,267, 1,301, 5,820).
                 if (!step.exec && chunk >= kStepCols) {
                     auto columns = [&](cudaStream_t cs) {
                         for (int q = 0; q < kStepCols; ++q) column(cs);
@@ -307,12 +312,12 @@ int gmres(const gw_bsr_t *A, int precond, const double *b, double *x, double rto
                     const int rc = capture_graph(columns, &step);
                     if (rc) return rc;
                 }
-                for (; step.exec && it + kStepCols <= chunk; it += kStepCols, kk += kStepCols) {
+                for (; step.exec && it + kStepCols <= chunk; it += kStepCols, kk += kStepCols, queued += kStepCols) {
                     const int rc = step.replay(s);
                     if (rc) return rc;
                 }
             }
-            for (; it < chunk; ++it, ++kk) column(s);
+            for (; it < chunk; ++it, ++kk, ++queued) column(s);
             GW_LAUNCHED();
             GW_CUDA(cudaMemcpyAsync(&h, G.sc, head, cudaMemcpyDeviceToHost, s));
             GW_CUDA(cudaStreamSynchronize(s));
