@@ -23,8 +23,22 @@ void assemble_per_model(const LaunchConst &c, const PtrsP &p, const int *perm, c
     }
 }
 
-// 3D: eight particles per CTA (27 threads each) up to two CTAs per SM, then 32, a
-// whole warp's worth of evaluations
+// 3D: whether one thread per particle (k_assemble) is the faster assembly of n.
+// Residual only: its 27 nodes are too little work to spread (10,648 particles 84 us
+// against 87, 32,768: 91 against 175, 262,144: 546 against 1,290; 8,000: 82 against 65).
+// With an FP64 tangent it takes one wave of 148 x 256 threads (255 registers) after the
+// other, 2.1 ms each, and k_assemble3 59 ns a particle: worth it where the waves are
+// full (110,592 particles 6.29 ms against 6.61, 262,144: 14.7 against 15.5; 175,616,
+// 93% full: 10.35 against 10.40; 64,000: 4.07 against 3.86).  With an FP32 tangent
+// never (110,592: 5.95 against 6.01, 262,144: 13.9 against 13.8).
+bool thread_per_particle3(int n, bool want_K, int prec) {
+    if (!want_K) return n > 10240;
+    constexpr int64_t wave = 148 * 256;
+    return prec == GW_PREC_F64 && 15 * ((n + wave - 1) / wave * wave) < 16 * (int64_t)n;
+}
+
+// k_assemble3: eight particles per CTA (27 threads each) up to two CTAs per SM, then
+// 32, a whole warp's worth of evaluations
 template <bool WANT_K, typename VT>
 int launch_assemble3(const LaunchConst &c, const PtrsP &p, const int *perm, const uint8_t *fm, const double *un,
                      const double *uo, const PtrsA &a, double *R, double *force, cudaStream_t s) {
@@ -56,7 +70,11 @@ int launch_assemble(const LaunchConst &c, const PtrsP &p, const int *perm, const
         ProfScope ps(PC_ASSEMBLE, s, per_p * p.n + grid + mat);
         if constexpr (KIND == GW_KIND_COUPLED3D) {
             int rc;
-            if (!want_K) rc = launch_assemble3<false, double>(c, p, perm, fm, un, uo, a, R, force, s);
+            if (thread_per_particle3(p.n, want_K, prec)) {
+                if (want_K) k_assemble<KIND, true, double><<<gw_count_launch(b), pb, 0, s>>>(c, p, perm, fm, un, uo, a, R, force);
+                else k_assemble<KIND, false, double><<<gw_count_launch(b), pb, 0, s>>>(c, p, perm, fm, un, uo, a, R, force);
+                rc = GW_OK;
+            } else if (!want_K) rc = launch_assemble3<false, double>(c, p, perm, fm, un, uo, a, R, force, s);
             else if (prec == GW_PREC_F64) rc = launch_assemble3<true, double>(c, p, perm, fm, un, uo, a, R, force, s);
             else rc = launch_assemble3<true, float>(c, p, perm, fm, un, uo, a, R, force, s);
             if (rc) return rc;
