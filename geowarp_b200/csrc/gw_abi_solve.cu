@@ -533,18 +533,21 @@ int mg_pattern(MgHier &h, const gw_bsr_t *A0, gw_mg_plan_t *plan, cudaStream_t s
     const int nl_bound = h.nl;
     h.lv[0].L = lat_of(h.lv[0].g);
     h.lv[0].A = *A0;
-    // active nodes and row counts of every level, read once
-    GW_CUDA(cudaMemsetAsync(h.counts, 0, 4 * kMgMaxLevels, s));
-    for (int q = 0; q + 1 < nl_bound; ++q) {
-        MgLevel &f = h.lv[q], &c = h.lv[q + 1];
-        c.L = lat_of(c.g);
-        k_mg_coarse_flags<<<gw_count_launch(nblk(c.g.n_nodes, kThreads)), kThreads, 0, s>>>(
-            f.L, q == 0 ? (const int *)f.A.node2row : nullptr, q == 0 ? nullptr : f.flags, c.L, c.flags, h.counts + q + 1);
-    }
-    GW_LAUNCHED();
+    // active nodes and row counts of the levels that may be needed (none below one whose
+    // whole lattice is small enough for the dense level), read once
+    const int64_t coarse = g_tune[GW_TUNE_MG_COARSE];
     int counts[kMgMaxLevels + 1] = {0};
-    if (A0->n_rows * NF > g_tune[GW_TUNE_MG_COARSE]) {
-        GW_CUDA(cudaMemcpyAsync(counts, h.counts, 4 * nl_bound, cudaMemcpyDeviceToHost, s));
+    if ((int64_t)A0->n_rows * NF > coarse) {
+        GW_CUDA(cudaMemsetAsync(h.counts, 0, 4 * kMgMaxLevels, s));
+        int q = 0;
+        for (; q + 1 < nl_bound && (int64_t)h.lv[q].g.n_nodes * NF > coarse; ++q) {
+            MgLevel &f = h.lv[q], &c = h.lv[q + 1];
+            c.L = lat_of(c.g);
+            k_mg_coarse_flags<<<gw_count_launch(nblk(c.g.n_nodes, kThreads)), kThreads, 0, s>>>(
+                f.L, q == 0 ? (const int *)f.A.node2row : nullptr, q == 0 ? nullptr : f.flags, c.L, c.flags, h.counts + q + 1);
+        }
+        GW_LAUNCHED();
+        GW_CUDA(cudaMemcpyAsync(counts, h.counts, 4 * (q + 1), cudaMemcpyDeviceToHost, s));
         GW_CUDA(cudaStreamSynchronize(s));
     }
     int l = 0;
@@ -606,21 +609,23 @@ int mg_pattern(MgHier &h, const gw_bsr_t *A0, gw_mg_plan_t *plan, cudaStream_t s
                 make_ptrs(v.A), lpr, v.strips, v.scols);
             GW_LAUNCHED();
         }
-    MgTotals tot;
-    memset(&tot, 0, sizeof(tot));
-    tot.n = h.nl;
-    for (int q = 0; q < h.nl; ++q) {
-        tot.row_ptr[q] = h.lv[q].A.row_ptr;
-        tot.n_rows[q] = h.lv[q].A.n_rows;
-    }
-    k_mg_totals<<<gw_count_launch(1), 32, 0, s>>>(tot, h.counts);
-    GW_LAUNCHED();
-    GW_CUDA(cudaMemcpyAsync(counts, h.counts, 4 * (kMgMaxLevels + 1), cudaMemcpyDeviceToHost, s));
-    GW_CUDA(cudaStreamSynchronize(s));
-    for (int q = 1; q < h.nl; ++q) h.lv[q].A.nnzb = counts[q];
-    if (counts[kMgMaxLevels]) {  // an index guard failed
-        const int gc = guard_check(s, "multigrid plan");
-        if (gc) return gc;
+    if (h.nl > 1) {
+        MgTotals tot;
+        memset(&tot, 0, sizeof(tot));
+        tot.n = h.nl;
+        for (int q = 0; q < h.nl; ++q) {
+            tot.row_ptr[q] = h.lv[q].A.row_ptr;
+            tot.n_rows[q] = h.lv[q].A.n_rows;
+        }
+        k_mg_totals<<<gw_count_launch(1), 32, 0, s>>>(tot, h.counts);
+        GW_LAUNCHED();
+        GW_CUDA(cudaMemcpyAsync(counts, h.counts, 4 * (kMgMaxLevels + 1), cudaMemcpyDeviceToHost, s));
+        GW_CUDA(cudaStreamSynchronize(s));
+        for (int q = 1; q < h.nl; ++q) h.lv[q].A.nnzb = counts[q];
+        if (counts[kMgMaxLevels]) {  // an index guard failed
+            const int gc = guard_check(s, "multigrid plan");
+            if (gc) return gc;
+        }
     }
     memset(plan, 0, sizeof(*plan));
     plan->levels = h.nl;
