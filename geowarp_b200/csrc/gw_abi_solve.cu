@@ -1,6 +1,8 @@
 // C ABI, Krylov solvers: BiCGSTAB / CG, restarted GMRES, multigrid-
 // preconditioned flexible GMRES, the workspace-free Krylov entry point and
 // SpMV (declarations and reference citations in include/geowarp_b200.h).
+#include <limits.h>
+
 #include <algorithm>
 #include <memory>
 #include <mutex>
@@ -583,7 +585,9 @@ int mg_pattern(MgHier &h, const gw_bsr_t *A0, gw_mg_plan_t *plan, cudaStream_t s
         if (rc) return rc;
         c.A.n_rows = nrc;
         c.A.nf = NF;
-        c.A.nnzb = N * (D == 2 ? 25 : 125);  // its capacity, until the block counts are read below
+        // its capacity, until the block counts are read below (which are ints: rows of a
+        // lattice of more than 2^31 / 125 nodes need not be)
+        c.A.nnzb = (int)std::min<int64_t>((int64_t)N * (D == 2 ? 25 : 125), INT_MAX);
         c.A.mask_words = mw;
         PtrsA ca = make_ptrs(c.A);
         if (D == 2) k_pattern_fill<2><<<gw_count_launch(nblk(nrc, kThreads)), kThreads, 0, s>>>(c.g, ca, (int *)c.A.cols);
