@@ -410,7 +410,8 @@ struct MgLevel {
     int *tmp, *sws, *blockrow;
     int *child;             // coarse levels: fine rows of the 3^D children of each row (pattern phase)
     int *parent;            // levels with a coarser one: coarse rows of the 2^D parents of each row
-    void *pvals;            // level 0: BF16 copy of the fine Jacobian read by the V-cycle (mixed)
+    void *pvals;            // level 0: BF16 copy of the fine Jacobian read by the V-cycle (mixed);
+                            // in 2D past the FP32 values in svals, which has room for FP64
     uint8_t *flags;
     // 2D: the sliced layout (gw_sell.cuh) of this level's matrix
     int *scols, *strips;
@@ -472,8 +473,12 @@ void mg_carve_hier(Bump &bp, MgHier &h, const gw_grid_t &g0, int64_t n_rows0, in
     l0.fixed = (uint8_t *)bp.take(n_rows0);
     const int CN = D == 2 ? 9 : 27, PN = D == 2 ? 4 : 8;
     l0.parent = (int *)bp.take(4 * n_rows0 * PN);
-    l0.pvals = bp.take(2 * (D == 2 ? sell_elems(n_rows0) : n_rows0 * S) * nf * nf);
-    if (D == 2) mg_carve_sell(bp, l0, n_rows0, nf);
+    if (D == 2) {
+        mg_carve_sell(bp, l0, n_rows0, nf);
+        if (l0.svals) l0.pvals = (float *)l0.svals + sell_elems(n_rows0) * nf * nf;
+    } else {
+        l0.pvals = bp.take(2 * n_rows0 * S * nf * nf);
+    }
     gw_grid_t g = g0;
     int64_t nodes = g0.n_nodes;
     int l = 0;

@@ -31,6 +31,8 @@
 // this layout and dependent launch alone: 26k rows FP64 125 -> 91 us, 267k rows FP32
 // 297 -> 189 us.
 #pragma once
+#include <algorithm>
+
 #include "gw_mg.cuh"
 
 namespace gw {
@@ -48,7 +50,8 @@ __host__ __device__ inline int sell_trips(int lpr) { return (kSellSlots + lpr - 
 // rows: 26k rows FP64 (finest level) 7.79 -> 7.59 ms, 72k and 267k rows FP32 (each with a
 // level of 19k) 14.40 -> 14.59 and 51.3 -> 52.1 ms, so it lies between 19k and 26k.
 // Raising it to 100,000 costs 30 Arnoldi steps of 72k rows FP32 2.63 -> 2.95 ms.
-inline int sell_lpr(int n_rows) { return n_rows >= 24576 ? 1 : 4; }
+constexpr int kSellOneLane = 24576;
+inline int sell_lpr(int n_rows) { return n_rows >= kSellOneLane ? 1 : 4; }
 
 __host__ __device__ inline int sell_chunks(int n_rows, int lpr) { return (n_rows + 32 / lpr - 1) / (32 / lpr); }
 
@@ -69,8 +72,10 @@ struct SellA {
     const int *trips;
 };
 
-inline int64_t sell_elems(int64_t n_rows) {  // upper bound over the lanes per row
-    return ((n_rows + 31) / 32 + 1) * 32 * 28;
+// block slots of a level of at most n_rows rows, whatever its lanes per row
+inline int64_t sell_elems(int64_t n_rows) {
+    const int64_t four = std::min<int64_t>(n_rows, kSellOneLane - 1), one = n_rows >= kSellOneLane ? n_rows : 0;
+    return 32 * std::max((four + 7) / 8 * kSellTrips<4>, (one + 31) / 32 * kSellTrips<1>);
 }
 
 __device__ __forceinline__ void unit_get(float v, double *o) { o[0] = (double)v; }
