@@ -200,12 +200,13 @@ int assemble_sorted(const LaunchConst &c, const PtrsP &p, const int *perm, const
     const double mat = WANT_K ? (double)A->nnzb * NF * NF * sizeof(VT) : 0.0;
     ProfScope ps(PC_ASSEMBLE, s, per_p * p.n + grid + mat);
     GW_CUDA(cudaMemsetAsync(ws, 0, w.box, s));  // cells without particles: start = end = 0
-    k_cell_ranges<<<gw_count_launch(nblk(p.n, kThreads)), kThreads, 0, s>>>(keys, p.n, nc, cstart, cend);
+    k_cell_ranges<<<gw_count_launch(nblk(p.n, kThreads)), kThreads, 0, s>>>(c.g, keys, p.n, fm, a.node2row, a.n_rows, cstart,
+                                                                         cend);
     GW_LAUNCHED();
     launch_particle_q<KIND, WANT_K, VT>(c, p, perm, un, uo, scratch, force, s);
     GW_LAUNCHED();
     k_cell_blocks<KIND, WANT_K, VT><<<gw_count_launch(nblk(nc, kCellGroups)), 16 * kCellGroups, 0, s>>>(
-        c, nc, by_cell, cstart, cend, scratch, fm, a.node2row, a.n_rows, sums, box);
+        c, nc, by_cell, cstart, cend, scratch, sums, box);
     if (A->n_rows > 0)
         k_row_gather<KIND, WANT_K, VT><<<gw_count_launch(nblk(A->n_rows, kGatherRows)), 32 * kGatherRows, 0, s>>>(
             c.g, by_cell, cstart, box, sums, fm, a, R);

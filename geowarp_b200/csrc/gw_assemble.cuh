@@ -66,15 +66,33 @@ struct CellSums {
     static const int ND = (81 * NF * NF + 9 * NF + 1) / 2 * 2;  // doubles, for the largest box
 };
 
-// sorted keys -> [start, end) of every occupied cell (cells without particles keep start = end = 0)
-__global__ void k_cell_ranges(const int *__restrict__ keys, int n, int n_cells, int *__restrict__ cstart,
+// sorted keys -> [start, end) of every occupied cell (cells without particles keep start = end = 0).
+// The cell's first thread also looks up the rows of its nodes that have free DOFs: a
+// contribution to a node that no row gathers (a stale row map) fails the guard.  (Here
+// it costs at most 1% of the assembly; in pass 2, 1-5%.)
+__global__ void k_cell_ranges(gw_grid_t grid, const int *__restrict__ keys, int n, const uint8_t *__restrict__ free_mask,
+                              const int *__restrict__ node2row, int n_rows, int *__restrict__ cstart,
                               int *__restrict__ cend) {
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= n) return;
-    const int k = keys[t];
-    if (!in_range(k, n_cells, GS_ASSEMBLE)) return;
-    if (t == 0 || keys[t - 1] != k) cstart[k] = t;
+    const int k = keys[t], ncx = grid.n_grid[0], ncy = grid.n_grid[1];
+    if (!in_range(k, ncx * ncy, GS_ASSEMBLE)) return;
     if (t == n - 1 || keys[t + 1] != k) cend[k] = t + 1;
+    if (t > 0 && keys[t - 1] == k) return;
+    cstart[k] = t;
+    const int cx = k % ncx, cy = k / ncx;
+    unsigned m[9];
+    int row[9];
+#pragma unroll
+    for (int a = 0; a < 9; ++a) {
+        const int nx = cx + a % 3, ny = cy + a / 3, node = nx + ny * (ncx + 1);
+        const bool in = nx <= ncx && ny <= ncy;
+        m[a] = in ? free_mask[node] : 0u;
+        row[a] = in ? node2row[node] : 0;
+    }
+#pragma unroll
+    for (int a = 0; a < 9; ++a)
+        if (m[a]) in_range(row[a], n_rows, GS_ASSEMBLE);
 }
 
 // Pass 1: one thread per particle in sorted order.
@@ -164,8 +182,6 @@ __global__ void __launch_bounds__(16 * kCellGroups) k_cell_blocks(LaunchConst c,
                                                                   const int *__restrict__ cstart,
                                                                   const int *__restrict__ cend,
                                                                   const unsigned char *__restrict__ scratch,
-                                                                  const uint8_t *__restrict__ free_mask,
-                                                                  const int *__restrict__ node2row, int n_rows,
                                                                   double *__restrict__ sums, int *__restrict__ box) {
     typedef KindTraits<KIND> KT;
     typedef Layout<KIND> L;
@@ -213,11 +229,6 @@ __global__ void __launch_bounds__(16 * kCellGroups) k_cell_blocks(LaunchConst c,
     const bool one = p1 - p0 <= kCellBatch;  // the axes of the only batch are in place
     const float ins = 1.0f / (float)max(ns, 1), ie0 = 1.0f / (float)max(e0, 1);  // exact quotients of small integers below
     double *const out = sums + (size_t)(by_cell ? cell : p0) * CS::ND;
-    if (lane < ns) {  // a node with free DOFs that no row would gather (a stale row map)
-        const int ay = (int)(((float)lane + 0.5f) * ie0), nx = cx + lane - ay * e0, ny = cy + ay;
-        const int node = nx + ny * (ncx + 1);
-        if (nx <= ncx && ny <= c.g.n_grid[1] && free_mask[node]) in_range(node2row[node], n_rows, GS_ASSEMBLE);
-    }
     __syncwarp(gmask);
 
     for (int q0 = 0; q0 < ns * NF; q0 += 16) {  // residual entries (slot a, field f)
