@@ -2,6 +2,8 @@
 // citations in include/geowarp_b200.h): the deterministic cell-sum
 // assembly of the 2D kinds (gw_assemble_sorted) and the atomic one
 // (gw_assemble, used for the 3D kind).
+#include <algorithm>
+
 #include "gw_host.cuh"
 #include "gw_assemble.cuh"
 
@@ -133,14 +135,29 @@ namespace {
 struct AsmParts {
     int64_t cend, box, rec, sums, bytes;
 };
-AsmParts asm_parts(int64_t n_cells, int64_t n, int64_t rec_bytes, int64_t sum_bytes) {
+// Cells whose sums are held at once: all of them in batches of up to half a million
+// (1.4 GB in the solid kind, 3.2 GB in u-p); a larger grid goes in bands of rows of
+// cells, at least 16 rows high, whose last two rows the next band computes again.
+// Where particles are fewer than cells, the sums lie at a cell's first particle, unless
+// they are more than a band and at least a quarter of the cells (each band looks at every
+// row, which a grid of mostly empty cells would not repay).
+constexpr int64_t kSumCells = 1 << 19;
+int64_t sum_cells(const gw_grid_t &g) {
+    const int64_t nc = (int64_t)g.n_grid[0] * g.n_grid[1], most = std::max<int64_t>(kSumCells, 16 * g.n_grid[0]);
+    return nc < most ? nc : most / g.n_grid[0] * g.n_grid[0];
+}
+bool sums_by_cell(const gw_grid_t &g, int64_t n) {
+    const int64_t nc = (int64_t)g.n_grid[0] * g.n_grid[1];
+    return nc <= n || (sum_cells(g) < n && nc <= 4 * n);
+}
+AsmParts asm_parts(const gw_grid_t &g, int64_t n, int64_t rec_bytes, int64_t sum_bytes) {
     AsmParts w;
-    const int64_t c = align256(4 * n_cells);
+    const int64_t n_cells = (int64_t)g.n_grid[0] * g.n_grid[1], c = align256(4 * n_cells);
     w.cend = c;
     w.box = 2 * c;
     w.rec = 3 * c;
     w.sums = w.rec + align256(rec_bytes * n);
-    w.bytes = w.sums + sum_bytes * (n_cells < n ? n_cells : n);
+    w.bytes = w.sums + sum_bytes * (sums_by_cell(g, n) ? sum_cells(g) : n);
     return w;
 }
 
@@ -178,10 +195,10 @@ template <int KIND, bool WANT_K, typename VT>
 int assemble_sorted(const LaunchConst &c, const PtrsP &p, const int *perm, const int *keys, const uint8_t *fm,
                     const double *un, const double *uo, const gw_bsr_t *A, double *R, double *force, const PtrsA &a,
                     char *ws, int64_t ws_bytes, cudaStream_t s) {
-    const int ncx = c.g.n_grid[0], ncy = c.g.n_grid[1], nc = ncx * ncy;
+    const int ncx = c.g.n_grid[0], ncy = c.g.n_grid[1];
     // the records written below must fit the caller's workspace (record size
     // of this instantiation, not of another precision)
-    const AsmParts w = asm_parts(nc, p.n, QRecord<KIND, VT>::BYTES, 8 * CellSums<KIND>::ND);
+    const AsmParts w = asm_parts(c.g, p.n, QRecord<KIND, VT>::BYTES, 8 * CellSums<KIND>::ND);
     if (w.bytes > ws_bytes) {
         snprintf(g_msg, sizeof(g_msg), "gw_assemble_sorted: workspace of %lld bytes, %lld needed",
                  (long long)ws_bytes, (long long)w.bytes);
@@ -190,7 +207,7 @@ int assemble_sorted(const LaunchConst &c, const PtrsP &p, const int *perm, const
     int *cstart = (int *)ws, *cend = (int *)(ws + w.cend), *box = (int *)(ws + w.box);
     unsigned char *scratch = (unsigned char *)(ws + w.rec);
     double *sums = (double *)(ws + w.sums);
-    const int by_cell = nc <= p.n;  // the cells' sums by cell, or by their first particle: whichever is fewer
+    const int by_cell = sums_by_cell(c.g, p.n);
     const int D = KindTraits<KIND>::D, NF = KindTraits<KIND>::NF;
     // algorithmic bytes, each array once: particle state in (x, lp, F_old, b_old,
     // E) and out (F_new, b_new, sigma), the scratch records written and read
@@ -205,11 +222,16 @@ int assemble_sorted(const LaunchConst &c, const PtrsP &p, const int *perm, const
     GW_LAUNCHED();
     launch_particle_q<KIND, WANT_K, VT>(c, p, perm, un, uo, scratch, force, s);
     GW_LAUNCHED();
-    k_cell_blocks<KIND, WANT_K, VT><<<gw_count_launch(nblk(nc, kCellGroups)), 16 * kCellGroups, 0, s>>>(
-        c, nc, by_cell, cstart, cend, scratch, sums, box);
-    if (A->n_rows > 0)
-        k_row_gather<KIND, WANT_K, VT><<<gw_count_launch(nblk(A->n_rows, kGatherRows)), 32 * kGatherRows, 0, s>>>(
-            c.g, by_cell, cstart, box, sums, fm, a, R);
+    const int rows = by_cell ? (int)(sum_cells(c.g) / ncx) : ncy;  // rows of cells at once
+    for (int y0 = 0;; y0 += rows - 2) {
+        const int y1 = std::min(y0 + rows, ncy);
+        k_cell_blocks<KIND, WANT_K, VT><<<gw_count_launch(nblk((int64_t)ncx * (y1 - y0), kCellGroups)), 16 * kCellGroups, 0, s>>>(
+            c, y0 * ncx, y1 * ncx, by_cell, cstart, cend, scratch, sums, box);
+        if (A->n_rows > 0)  // a node's cells start up to two rows below it
+            k_row_gather<KIND, WANT_K, VT><<<gw_count_launch(nblk(A->n_rows, kGatherRows)), 32 * kGatherRows, 0, s>>>(
+                c.g, by_cell, y0 * ncx, y0 ? y0 + 2 : 0, y1 < ncy ? y1 : ncy + 1, cstart, box, sums, fm, a, R);
+        if (y1 == ncy) break;
+    }
     GW_LAUNCHED();
     return GW_OK;
 }
@@ -246,9 +268,8 @@ int assemble_sorted_kind(const LaunchConst &c, const PtrsP &p, const int *perm, 
 extern "C" int64_t gw_assemble_workspace_bytes(const gw_grid_t *grid, int32_t n_particles, int32_t prec) {
     if (!grid || n_particles < 0) return -1;
     if (grid->dim != 2) return 0;  // the 3D kind assembles with atomics and needs no workspace
-    const int64_t nc = (int64_t)grid->n_grid[0] * grid->n_grid[1];
     const int64_t sum = 8 * (grid->kind == GW_KIND_SOLID2D ? CellSums<GW_KIND_SOLID2D>::ND : CellSums<GW_KIND_COUPLED2D>::ND);
-    return asm_parts(nc, n_particles, record_bytes(grid->kind, prec), sum).bytes;
+    return asm_parts(*grid, n_particles, record_bytes(grid->kind, prec), sum).bytes;
 }
 
 extern "C" int gw_assemble_sorted(const gw_grid_t *grid, const gw_material_t *mat, const gw_step_t *st,

@@ -170,7 +170,8 @@ __device__ __forceinline__ void record_row(const double *p, double d[4]) {
 // entries l, l + 16, one at a time over all the cell's particles, so it holds one
 // block in registers and the SM many cells.  (A cell of more than eight particles
 // evaluates its axes again for each round.)  box[cell]: the box's extents, 0 without
-// particles.
+// particles.  Cells cell0 .. cell1 - 1, their sums from the buffer's start (by_cell) or
+// at their first particle.
 constexpr int kCellGroups = 8;   // cells per CTA
 constexpr int kCellBatch = 8;
 struct CellAxis {
@@ -178,7 +179,7 @@ struct CellAxis {
     int off, span;  // corner offset from the cell (a particle clamped at the grid edge), nodes
 };
 template <int KIND, bool WANT_K, typename VT>
-__global__ void __launch_bounds__(16 * kCellGroups) k_cell_blocks(LaunchConst c, int n_cells, int by_cell,
+__global__ void __launch_bounds__(16 * kCellGroups) k_cell_blocks(LaunchConst c, int cell0, int cell1, int by_cell,
                                                                   const int *__restrict__ cstart,
                                                                   const int *__restrict__ cend,
                                                                   const unsigned char *__restrict__ scratch,
@@ -191,9 +192,9 @@ __global__ void __launch_bounds__(16 * kCellGroups) k_cell_blocks(LaunchConst c,
     constexpr int D = 2, NF = KT::NF;
     __shared__ CellAxis axs[kCellGroups][kCellBatch][2];
     const int lane = threadIdx.x & 15, grp = threadIdx.x >> 4;
-    const int cell = blockIdx.x * kCellGroups + grp;
+    const int cell = cell0 + blockIdx.x * kCellGroups + grp;
     const unsigned gmask = 0xffffu << (threadIdx.x & 16);  // this cell's half of the warp
-    if (cell >= n_cells) return;  // whole groups; group-wide syncs below
+    if (cell >= cell1) return;  // whole groups; group-wide syncs below
     const int p0 = cstart[cell], p1 = cend[cell];
     if (p1 <= p0) {
         if (lane == 0) box[cell] = 0;
@@ -228,7 +229,7 @@ __global__ void __launch_bounds__(16 * kCellGroups) k_cell_blocks(LaunchConst c,
     const int ns = e0 * e1, nb = ns * ns;
     const bool one = p1 - p0 <= kCellBatch;  // the axes of the only batch are in place
     const float ins = 1.0f / (float)max(ns, 1), ie0 = 1.0f / (float)max(e0, 1);  // exact quotients of small integers below
-    double *const out = sums + (size_t)(by_cell ? cell : p0) * CS::ND;
+    double *const out = sums + (size_t)(by_cell ? cell - cell0 : p0) * CS::ND;
     __syncwarp(gmask);
 
     for (int q0 = 0; q0 < ns * NF; q0 += 16) {  // residual entries (slot a, field f)
@@ -359,10 +360,12 @@ __device__ __forceinline__ void load_rw_blk(const double *p, double v[N]) {
 }
 
 // Pass 3: a warp per block row.  Lane t < 25 sums the block at stencil bit t, lanes
-// 25 .. 25 + NF - 1 the residual fields, over the cells that reach the node.
+// 25 .. 25 + NF - 1 the residual fields, over the cells that reach the node.  Rows of
+// the nodes with ny0 <= y < ny1; cell0 as in pass 2.
 constexpr int kGatherRows = 8;  // rows per CTA
 template <int KIND, bool WANT_K, typename VT>
 __global__ void __launch_bounds__(32 * kGatherRows) k_row_gather(gw_grid_t grid, int by_cell,
+                                                                 int cell0, int ny0, int ny1,
                                                                  const int *__restrict__ cstart,
                                                                  const int *__restrict__ box,
                                                                  const double *__restrict__ sums,
@@ -377,6 +380,7 @@ __global__ void __launch_bounds__(32 * kGatherRows) k_row_gather(gw_grid_t grid,
     const int node = A.row2node[r];
     if (!in_range(node, grid.n_nodes, GS_ASSEMBLE)) return;
     const int nx = node % (ncx + 1), ny = node / (ncx + 1);
+    if (ny < ny0 || ny >= ny1) return;  // whole warps
     const unsigned fa = free_mask[node];
     // lanes 0-8: the cell of each (cx mod 3, cy mod 3) that reaches this node, in the order of the sums
     int slot = 0, info = 0;  // info: box extents, and this node's slot (ax, ay)
@@ -387,7 +391,7 @@ __global__ void __launch_bounds__(32 * kGatherRows) k_row_gather(gw_grid_t grid,
             const int cell = cx + cy * ncx, b = box[cell], ax = nx - cx, ay = ny - cy;
             if (ax < (b & 3) && ay < (b >> 2)) {
                 info = b | ax << 4 | ay << 6;
-                slot = by_cell ? cell : cstart[cell];
+                slot = by_cell ? cell - cell0 : cstart[cell];
             }
         }
     }

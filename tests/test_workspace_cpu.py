@@ -27,3 +27,16 @@ def test_multigrid_bytes_per_finest_row(lo, hi, slots, nf):
     vectors = 8 * nf * (2 * restart + 2 + 4) + 8 * nf * nf + 4 * 4 + 1
     matrix = slots * (4 + 8 * nf * nf) + 4 / 8
     assert (b - a) / (hi - lo) <= vectors + matrix + 0.5  # every array is rounded to 256 bytes
+
+
+@pytest.mark.parametrize("kind,nf", [(L.KIND_SOLID2D, 2), (L.KIND_COUPLED2D, 3)])
+@pytest.mark.parametrize("nx,ny,n", [(2000, 2000, 16000000), (2000, 2000, 3000000), (100000, 60, 24000000)])
+def test_assembly_bytes_are_bounded(kind, nf, nx, ny, n):
+    """Beside the particle records and three words a cell: the sums (81 blocks and nine
+    nodes' residuals, FP64) of half a million cells, or of 16 rows of cells."""
+    lib = L.load()
+    g = _grid(kind, nx, ny)
+    rec = (lib.gw_assemble_workspace_bytes(C.byref(_grid(kind, 1, 1)), 200000, L.PREC_F64)
+           - lib.gw_assemble_workspace_bytes(C.byref(_grid(kind, 1, 1)), 100000, L.PREC_F64)) / 100000
+    sums = 8 * (81 * nf * nf + 9 * nf + 1) * max(2 ** 19, 16 * nx)
+    assert lib.gw_assemble_workspace_bytes(C.byref(g), n, L.PREC_F64) <= (rec + 0.01) * n + 12 * nx * ny + sums + 4096
