@@ -495,9 +495,11 @@ const char *gw_profile_name(int32_t cls);
  *                           levels' constants and vectors in shared memory
  *                           (bitwise the same V-cycle).  Levels that do not
  *                           fit there stay one launch per phase.
- *                           0..1048576 (default 0: up to 2,048 rows; values
- *                           above 16,384 act as 16,384; 3D hierarchies run
- *                           one launch per phase); recaptures the step graphs
+ *                           0..1048576 (default 0: up to 2,048 rows, the
+ *                           bound that measured fastest; 1: no level is
+ *                           fused, one launch per phase; values above 16,384
+ *                           act as 16,384; 3D hierarchies run one launch per
+ *                           phase); recaptures the step graphs
  *   GW_TUNE_MG_BF16         1: in mixed-precision multigrid solves the V-cycle
  *                           reads a BF16 copy of the fine-level Jacobian (made
  *                           before each solve; GMRES still applies the FP32
