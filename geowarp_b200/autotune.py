@@ -23,7 +23,8 @@ from . import _lib as L
 # 0.8 and above makes the block-Jacobi smoother diverge (GMRES then runs to
 # its iteration cap).  GW_TUNE_MG_TAIL is not searched either: its
 # default bound of 2,048 rows was the fastest, or within 0.3% of it, from 640
-# to 1.0 M particles.
+# to 1.0 M particles.  Of row_warps, 8 and 16 are one launch shape in 2D (its row kernels
+# use at most 8) and two in 3D.
 KNOBS = {
     "row_warps": (L.TUNE_ROW_WARPS, (2, 4, 8, 16)),
     "mg_coarse": (L.TUNE_MG_COARSE, (40, 80, 160)),

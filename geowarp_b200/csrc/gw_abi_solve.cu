@@ -264,8 +264,11 @@ int gmres(const gw_bsr_t *A, int precond, const double *b, double *x, double rto
     k_precond_setup<NF, VT><<<gw_count_launch(nblk(nr, kThreads)), kThreads, 0, s>>>(a, D, precond, G.Minv);
     GW_LAUNCHED();
     const int gr = red_grid_rows(nr), ge = red_grid_elems(nr);
-    // a warp per row where the rows alone do not fill the device and are long
-    // enough for it (below 16 blocks most of its lanes would idle)
+    // A warp per row where the rows alone do not fill the device and are long enough
+    // for it (below 16 blocks most of its lanes would idle).  A solve of 24 columns with
+    // eight lanes per row -> a warp: 1,000 rows of 125 blocks 4 x 4 FP64 987 -> 622 us, 4,096
+    // rows of 27 649 -> 617, 3,600 of 25 2 x 2 522 -> 477, of 9 499 -> 482; FP32 4 x 4 rows of
+    // 27: 4,096 602 -> 591, 8,000 646 -> 690, 13,824 742 -> 861 (FP64 there 982 -> 910).
     const bool wide = nr <= 8192 && (int64_t)A->nnzb >= 16 * (int64_t)nr;
     GScalars h;
     memset(&h, 0, head);
@@ -583,7 +586,7 @@ int mg_pattern(MgHier &h, const gw_bsr_t *A0, gw_mg_plan_t *plan, cudaStream_t s
             k_mg_coarse_stencil2<<<gw_count_launch(nblk((int64_t)nrc * 32, kThreads)), kThreads, 0, s>>>(
                 f.L, fa, c.L, nrc, c.A.row2node, (uint32_t *)c.A.stencil, c.tmp);
         else
-            k_mg_coarse_stencil<3><<<gw_count_launch(nblk(nrc, kThreads)), kThreads, 0, s>>>(
+            k_mg_coarse_stencil<<<gw_count_launch(nblk(nrc, kThreads)), kThreads, 0, s>>>(
                 f.L, fa, c.L, nrc, c.A.row2node, (uint32_t *)c.A.stencil, mw, c.tmp);
         GW_LAUNCHED();
         rc = scan_exclusive(c.tmp, (int *)c.A.row_ptr, nrc + 1, c.sws, s);
@@ -688,7 +691,7 @@ int mg_numeric(MgHier &h, cudaStream_t s) {
         PtrsA fa = make_ptrs(f.A), ca = make_ptrs(c.A);
         const int nb = c.A.nnzb;
         if (D == 2) k_mg_rap2<NF, VT><<<gw_count_launch(nblk((int64_t)nb * 16, kThreads)), kThreads, 0, s>>>(fa, f.fixed, c.child, c.L, ca, c.blockrow);
-        else k_mg_rap<3, NF, VT><<<gw_count_launch(nblk(nb, kThreads)), kThreads, 0, s>>>(f.L, fa, f.fixed, c.L, ca, c.blockrow);
+        else k_mg_rap<NF, VT><<<gw_count_launch(nblk(nb, kThreads)), kThreads, 0, s>>>(f.L, fa, f.fixed, c.L, ca, c.blockrow);
         GW_LAUNCHED();
         const int nrc = c.A.n_rows;
         k_mg_fix_empty_rows<NF, VT><<<gw_count_launch(nblk(nrc, kThreads)), kThreads, 0, s>>>(ca);
@@ -1107,7 +1110,7 @@ double *mg_vcycle(const MgHier &h, const int *skip, cudaStream_t s) {
                                     tune_rows_block(), 0, s>>>(a, v.b, x, v.r, skip);
         }
         ProfScope ps(PC_MG_TRANSFER, s, vs + 8.0 * c.A.n_rows * NF);
-        k_mg_restrict_list<3, NF><<<gw_count_launch(nblk(c.A.n_rows, kThreads)), kThreads, 0, s>>>(
+        k_mg_restrict_list<NF><<<gw_count_launch(nblk(c.A.n_rows, kThreads)), kThreads, 0, s>>>(
                 c.A.n_rows, v.A.n_rows, c.child, v.fixed, v.r, c.b, skip);
         cur[l] = x;
         oth[l] = y;
@@ -1121,7 +1124,7 @@ double *mg_vcycle(const MgHier &h, const int *skip, cudaStream_t s) {
         double *x = cur[l], *y = oth[l];
         {
         ProfScope ps(PC_MG_TRANSFER, s, 16.0 * v.A.n_rows * NF + 8.0 * c.A.n_rows * NF);
-        k_mg_prolong_list<3, NF><<<gw_count_launch(nblk(v.A.n_rows, kThreads)), kThreads, 0, s>>>(
+        k_mg_prolong_list<NF><<<gw_count_launch(nblk(v.A.n_rows, kThreads)), kThreads, 0, s>>>(
                 v.A.n_rows, c.A.n_rows, v.parent, v.fixed, cur[l + 1], x, skip);
         }
         for (int it = 0; it < mg_sweeps(l); ++it) {

@@ -19,7 +19,7 @@
 //     element blocks (slot a, slot b) and residual entries over the cell's
 //     particles in sorted order and leaves them, in FP64, in the cell's buffer.
 //
-//  3. k_row_gather (16 lanes per block row): a row's entries and blocks are the sums
+//  3. k_row_gather (a warp per block row): a row's entries and blocks are the sums
 //     over the up to nine cells that reach its node; it is written once, with its
 //     Dirichlet identity entries.
 //

@@ -217,7 +217,7 @@ static inline int n_cells_of(const gw_grid_t &g) {
     return c;
 }
 
-inline const char *kGuardNames[GS_COUNT] = {"none", "row_mv column", "coarse flags", "coarse stencil", "pattern fill",
+inline const char *kGuardNames[GS_COUNT] = {"none", "row_mv column", "coarse stencil", "pattern fill",
                                      "Galerkin product (coarse block)", "Galerkin product (fine block)",
                                      "smoother setup", "restriction", "prolongation", "dense coarsest level",
                                      "Krylov column counter", "transpose", "assembly scatter", "adjoint scatter",

@@ -31,7 +31,7 @@ constexpr int ST_RANGE = 1, ST_NAN = 2, ST_BREAKDOWN = 4;
 // (gw_guard_read), so a corrupted pattern surfaces as GW_ERANGE on the host
 // instead of as a memory fault.
 enum GuardSite {
-    GS_NONE = 0, GS_ROW_MV, GS_COARSE_FLAGS, GS_COARSE_STENCIL, GS_PATTERN_FILL, GS_RAP_COARSE, GS_RAP_FINE,
+    GS_NONE = 0, GS_ROW_MV, GS_COARSE_STENCIL, GS_PATTERN_FILL, GS_RAP_COARSE, GS_RAP_FINE,
     GS_SMOOTHER, GS_RESTRICT, GS_PROLONG, GS_DENSE, GS_KRYLOV_K, GS_TRANSPOSE, GS_ASSEMBLE, GS_ADJOINT,
     GS_BLOCKROW, GS_FIXED, GS_PRESMOOTH, GS_COUNT
 };

@@ -655,7 +655,7 @@ constexpr int kGmresMaxRestart = 128;
 
 struct GScalars {
     // scalar header first: the host polls only this prefix
-    double beta, bnorm, tol, resid, wnorm;
+    double beta, bnorm, tol, resid;
     double gs_eta2;  // second Gram-Schmidt pass below this fraction of ||w||^2 left
     int k;           // completed Arnoldi columns in the current cycle
     int cycle_done, done, status, iters, max_iter, restart;
@@ -668,7 +668,6 @@ struct GScalars {
     double cs[kGmresMaxRestart], sn[kGmresMaxRestart];
     double g[kGmresMaxRestart + 1];
     double y[kGmresMaxRestart];
-    double h2[kGmresMaxRestart + 1];
 };
 
 struct GmresVecs {
@@ -814,7 +813,10 @@ constexpr int kGsThreads = 256;
 constexpr int kGsBlocks = 296;                    // element blocks: two per SM
 constexpr int kGsItems = kGmresMaxRestart + 1;    // (v_i, w), i <= k < restart, and (w, w)
 constexpr int kGsGroup = 8;                       // items per block of k_gm_dots
-constexpr int kGsSplitMax = 16384;                // unknowns up to which k_gm_update splits the basis over warps
+// Unknowns up to which k_gm_update splits the basis over warps.  A solve of 100 columns,
+// never split -> always: 8,788 unknowns 2,988 -> 2,683 us, 16,384: 3,397 -> 3,148, 23,328:
+// 3,764 -> 3,865, 32,000: 4,136 -> 4,291, 108,000: 9,425 -> 10,478.
+constexpr int kGsSplitMax = 16384;
 // partials: dots item i of element block b at [i * kGsBlocks + b]; ||w||^2 after them
 constexpr int kGsPartials = (kGsItems + 1) * kGsBlocks;
 
@@ -1083,7 +1085,6 @@ __device__ __forceinline__ void gs_close(GScalars *sc, int k, double hn) {
         if (rr > 0.0) { c = a / rr; s = hn / rr; }
         h[k] = rr;
         const double gk = sc->g[k], next = -s * gk;
-        sc->wnorm = hn;
         sc->cs[k] = c;
         sc->sn[k] = s;
         sc->H[k + 1][k] = 0.0;

@@ -36,7 +36,7 @@ namespace {  // internal linkage: each translation unit compiles the kernels it 
 
 constexpr int kMgMaxLevels = GW_MG_MAX_LEVELS;
 // unknowns of the coarsest (dense) level: its n x n FP64 matrix (204,800 bytes
-// at 160) is inverted in one CTA's shared memory
+// at 160) is inverted in one CTA's registers
 constexpr int kMgCoarseMax = 160;
 constexpr int kMgCoarseMin = 8;  // smallest coarsest-level bound a caller may set
 
@@ -130,8 +130,7 @@ __global__ void k_mg_totals(MgTotals t, int *__restrict__ out) {
     if (l == kMgMaxLevels) out[l] = g_guard_site;
 }
 
-// coarse stencil mask of every coarse row and its block count
-template <int D>
+// 3D: coarse stencil mask of every coarse row and its block count
 __global__ void k_mg_coarse_stencil(Lat Lf, PtrsA Af, Lat Lc, int nc_rows, const int *__restrict__ c_row2node,
                                     uint32_t *__restrict__ c_stencil, int mw, int *__restrict__ c_count) {
     const int R = blockIdx.x * blockDim.x + threadIdx.x;
@@ -141,12 +140,12 @@ __global__ void k_mg_coarse_stencil(Lat Lf, PtrsA Af, Lat Lc, int nc_rows, const
     int C[3];
     lat_coords(Lc, I, C);
     uint32_t mask[4] = {0u, 0u, 0u, 0u};
-    for (int oz = (D == 3 ? -1 : 0); oz <= (D == 3 ? 1 : 0); ++oz)
+    for (int oz = -1; oz <= 1; ++oz)
         for (int oy = -1; oy <= 1; ++oy)
             for (int ox = -1; ox <= 1; ++ox) {
                 const int ci[3] = {2 * C[0] + ox, 2 * C[1] + oy, 2 * C[2] + oz};
                 bool in = true;
-                for (int k = 0; k < D; ++k) in = in && ci[k] >= 0 && ci[k] < Lf.n[k];
+                for (int k = 0; k < 3; ++k) in = in && ci[k] >= 0 && ci[k] < Lf.n[k];
                 if (!in) continue;
                 const int i = lat_id(Lf, ci);
                 if (Af.node2row[i] < 0) continue;
@@ -156,7 +155,7 @@ __global__ void k_mg_coarse_stencil(Lat Lf, PtrsA Af, Lat Lc, int nc_rows, const
                         int bit = w * 32 + __ffs(m) - 1;
                         m &= m - 1u;
                         int cj[3] = {ci[0], ci[1], ci[2]};
-                        for (int k = 0; k < D; ++k) {
+                        for (int k = 0; k < 3; ++k) {
                             cj[k] += bit % 5 - 2;
                             bit /= 5;
                         }
@@ -164,16 +163,16 @@ __global__ void k_mg_coarse_stencil(Lat Lf, PtrsA Af, Lat Lc, int nc_rows, const
                         int lo[3], cnt[3];
                         for (int k = 0; k < 3; ++k) {
                             lo[k] = (cj[k] >> 1) - C[k];
-                            cnt[k] = (k < D && (cj[k] & 1)) ? 2 : 1;
+                            cnt[k] = (cj[k] & 1) ? 2 : 1;
                         }
                         for (int a = 0; a < cnt[0]; ++a)
                             for (int b = 0; b < cnt[1]; ++b)
                                 for (int d = 0; d < cnt[2]; ++d) {
                                     const int off[3] = {lo[0] + a, lo[1] + b, lo[2] + d};
                                     bool ok = true;
-                                    for (int k = 0; k < D; ++k) ok = ok && in_range(off[k] + 2, 5, GS_COARSE_STENCIL);
+                                    for (int k = 0; k < 3; ++k) ok = ok && in_range(off[k] + 2, 5, GS_COARSE_STENCIL);
                                     if (!ok) continue;
-                                    const int ob = offset_bit<D>(off);
+                                    const int ob = offset_bit<3>(off);
                                     mask[ob >> 5] |= 1u << (ob & 31);
                                 }
                     }
@@ -236,9 +235,9 @@ __global__ void k_mg_blockrow(const int *__restrict__ row_ptr, int n_rows, int n
 }
 
 // ---------------------------------------------------------------- Galerkin product
-// One thread per coarse block (I, J): sum over children i of I and j of J,
+// 3D: one thread per coarse block (I, J), sum over children i of I and j of J,
 // in lattice order, of w_i w_j A(i, j) restricted to free DOFs.
-template <int D, int NF, typename VT>
+template <int NF, typename VT>
 __global__ void k_mg_rap(Lat Lf, PtrsA Af, const uint8_t *__restrict__ ffixed, Lat Lc, PtrsA Ac,
                          const int *__restrict__ c_blockrow) {
     const int jb = blockIdx.x * blockDim.x + threadIdx.x;
@@ -263,38 +262,38 @@ __global__ void k_mg_rap(Lat Lf, PtrsA Af, const uint8_t *__restrict__ ffixed, L
 #pragma unroll
         for (int g = 0; g < NF; ++g) acc[f][g] = 0.0;
     const VT *vals = (const VT *)Af.vals;
-    for (int iz = (D == 3 ? -1 : 0); iz <= (D == 3 ? 1 : 0); ++iz)
+    for (int iz = -1; iz <= 1; ++iz)
         for (int iy = -1; iy <= 1; ++iy)
             for (int ix = -1; ix <= 1; ++ix) {
                 const int ci[3] = {2 * CI[0] + ix, 2 * CI[1] + iy, 2 * CI[2] + iz};
                 bool in = true;
-                for (int k = 0; k < D; ++k) in = in && ci[k] >= 0 && ci[k] < Lf.n[k];
+                for (int k = 0; k < 3; ++k) in = in && ci[k] >= 0 && ci[k] < Lf.n[k];
                 if (!in) continue;
                 const int i = lat_id(Lf, ci);
                 const int fr = Af.node2row[i];
                 if (fr < 0 || !in_range(fr, Af.n_rows, GS_RAP_FINE)) continue;
                 double wi = 1.0;
-                for (int k = 0; k < D; ++k) wi *= p_weight(ci[k], CI[k]);
+                for (int k = 0; k < 3; ++k) wi *= p_weight(ci[k], CI[k]);
                 const uint8_t fi = ffixed[fr];
-                for (int jz = (D == 3 ? -1 : 0); jz <= (D == 3 ? 1 : 0); ++jz)
+                for (int jz = -1; jz <= 1; ++jz)
                     for (int jy = -1; jy <= 1; ++jy)
                         for (int jx = -1; jx <= 1; ++jx) {
                             const int cj[3] = {2 * CJ[0] + jx, 2 * CJ[1] + jy, 2 * CJ[2] + jz};
                             int off[3] = {0, 0, 0};
                             bool ok = true;
-                            for (int k = 0; k < D; ++k) {
+                            for (int k = 0; k < 3; ++k) {
                                 off[k] = cj[k] - ci[k];
                                 ok = ok && off[k] >= -2 && off[k] <= 2 && cj[k] >= 0 && cj[k] < Lf.n[k];
                             }
                             if (!ok) continue;
-                            const int slot = stencil_slot(Af.stencil, Af.mw, i, offset_bit<D>(off));
+                            const int slot = stencil_slot(Af.stencil, Af.mw, i, offset_bit<3>(off));
                             if (slot < 0) continue;
                             const int fc = Af.node2row[lat_id(Lf, cj)];
                             if (fc < 0 || !in_range(fc, Af.n_rows, GS_RAP_FINE)) continue;
                             const long long fb = (long long)Af.row_ptr[fr] + slot;
                             if (!in_range(fb, Af.nnzb, GS_RAP_FINE)) continue;
                             double wj = 1.0;
-                            for (int k = 0; k < D; ++k) wj *= p_weight(cj[k], CJ[k]);
+                            for (int k = 0; k < 3; ++k) wj *= p_weight(cj[k], CJ[k]);
                             const uint8_t fj = ffixed[fc];
                             const VT *blk = vals + (size_t)fb * NF * NF;
                             const double w = wi * wj;
@@ -654,12 +653,12 @@ __global__ void k_mg_parents(Lat Lf, PtrsA Af, Lat Lc, PtrsA Ac, int *__restrict
             }
 }
 
-// b_c = P^T r_f through the child lists
-template <int D, int NF>
+// 3D: b_c = P^T r_f through the child lists
+template <int NF>
 __global__ void k_mg_restrict_list(int nc, int nf_rows, const int *__restrict__ child,
                                    const uint8_t *__restrict__ ffixed, const double *__restrict__ rf,
                                    double *__restrict__ bc, const int *__restrict__ skip) {
-    constexpr int CN = D == 2 ? 9 : 27;
+    constexpr int CN = 27;
     if (skip && *skip) return;
     const int R = blockIdx.x * blockDim.x + threadIdx.x;
     if (R >= nc) return;
@@ -677,7 +676,7 @@ __global__ void k_mg_restrict_list(int nc, int nf_rows, const int *__restrict__ 
         double w = 1.0;
         w *= ox == 0 ? 1.0 : 0.5;
         w *= oy == 0 ? 1.0 : 0.5;
-        if (D == 3) w *= oz == 0 ? 1.0 : 0.5;
+        w *= oz == 0 ? 1.0 : 0.5;
         const uint8_t fx = ffixed[fr[q]];
 #pragma unroll
         for (int f = 0; f < NF; ++f)
@@ -687,12 +686,12 @@ __global__ void k_mg_restrict_list(int nc, int nf_rows, const int *__restrict__ 
     for (int f = 0; f < NF; ++f) bc[(size_t)R * NF + f] = acc[f];
 }
 
-// x_f += P x_c through the parent lists
-template <int D, int NF>
+// 3D: x_f += P x_c through the parent lists
+template <int NF>
 __global__ void k_mg_prolong_list(int n_rows, int nc, const int *__restrict__ parent,
                                   const uint8_t *__restrict__ ffixed, const double *__restrict__ xc,
                                   double *__restrict__ xf, const int *__restrict__ skip) {
-    constexpr int PN = D == 2 ? 4 : 8;
+    constexpr int PN = 8;
     if (skip && *skip) return;
     const int r = blockIdx.x * blockDim.x + threadIdx.x;
     if (r >= n_rows) return;

@@ -46,10 +46,12 @@ __host__ __device__ inline int sell_trips(int lpr) { return (kSellSlots + lpr - 
 // Lanes per row of a level, by its rows alone (both the separate kernels and
 // the fused tail follow it, so their sums are the same).  Few rows with a lane each
 // are less than 6 warps per SM, and too few loads in flight; above, four lanes load a
-// quarter more (9 blocks in 12 slots).  Solves with the change at 32,768 -> at 16,384
-// rows: 26k rows FP64 (finest level) 7.79 -> 7.59 ms, 72k and 267k rows FP32 (each with a
-// level of 19k) 14.40 -> 14.59 and 51.3 -> 52.1 ms, so it lies between 19k and 26k.
-// Raising it to 100,000 costs 30 Arnoldi steps of 72k rows FP32 2.63 -> 2.95 ms.
+// quarter more (9 blocks in 12 slots).  30 Arnoldi steps with the finest level at four
+// lanes -> one, 2 x 2 blocks FP64 / FP32: 10,000 rows 2.01 -> 2.04 / 2.01 -> 2.01 ms, 15,129:
+// 2.15 -> 2.17 / 2.17 -> 2.16, 19,881: 2.32 -> 2.26 / 2.29 -> 2.20, 24,964: 2.36 -> 2.27 /
+// 2.37 -> 2.24, 40,000: 2.92 -> 2.74 / 2.85 -> 2.64, 90,000: 4.26 -> 3.84 / 4.00 -> 3.54; 3 x 3
+// blocks alike.  Below the finest level, 19k FP32 rows got slower with one lane (solves on
+// 72k and 267k rows 14.40 -> 14.59 and 51.3 -> 52.1 ms), so the line lies above them.
 constexpr int kSellOneLane = 24576;
 inline int sell_lpr(int n_rows) { return n_rows >= kSellOneLane ? 1 : 4; }
 

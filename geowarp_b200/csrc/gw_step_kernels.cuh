@@ -720,7 +720,7 @@ __global__ void k_g2p(LaunchConst c, PtrsP p, const double *__restrict__ u_new, 
 }
 
 // ================================================================ single-point return maps
-// One instantiation per model (MODEL < 0: at run time), so each carries its own code only.
+// One instantiation per model, so each carries its own code only.
 template <int MODEL>
 __global__ void __launch_bounds__(128) k_return_map(MatConst mc, double lam, double mu, int n, const double *__restrict__ etr,
                              const double *__restrict__ evt, const double *__restrict__ pi_old,
